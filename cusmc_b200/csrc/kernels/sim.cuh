@@ -182,15 +182,15 @@ inline size_t batch_smem_bytes(uint32_t n_jobs, uint32_t group_stride, int block
 }
 // Shared memory of one lane group's run state (sim_impl.cuh: RunState): 48
 // bytes of scalars, the variables and one inverse rate per rate program,
-// 16-aligned; then the group's slot masks, component gl*K + k of lane gl at
-// [k * lanes + gl].
+// 16-aligned; then the delay records (8 bytes), the slot masks (u32) and the
+// global location indices (u16) of the components.
 __host__ __device__ inline uint32_t group_vars_bytes(uint32_t n_vars, uint32_t n_rate_prog) {
     return (48u + 4u * (n_vars + n_rate_prog) + 15u) & ~15u;
 }
 __host__ __device__ inline uint32_t group_state_stride(uint32_t n_vars, uint32_t n_rate_prog, uint32_t lanes,
                                                        uint32_t comps_per_lane) {
     // 16-aligned: the next group's scalars hold doubles
-    return (group_vars_bytes(n_vars, n_rate_prog) + 4u * lanes * comps_per_lane + 15u) & ~15u;
+    return (group_vars_bytes(n_vars, n_rate_prog) + 14u * lanes * comps_per_lane + 15u) & ~15u;
 }
 // Bytes of one thread's state in a batch slab (16-bit locations, slot masks).
 inline size_t batch_state_bytes_per_thread(uint32_t max_comps, uint32_t max_vars, uint32_t max_rate_prog) {

@@ -65,6 +65,7 @@ template <int K, bool VERIFY>
 static __device__ __forceinline__ void batch_group_phase(const BatchParams &p, const BatchJob *jobs, uint8_t *smem) {
     const uint32_t lane = threadIdx.x & 31u;
     RunState *s = reinterpret_cast<RunState *>(smem + p.n_jobs * sizeof(BatchJob) + (threadIdx.x >> 5) * p.group_stride);
+    GroupRun<32, K, VERIFY> g(s, lane);
     unsigned long long acc_hits = 0, acc_steps = 0, acc_capped = 0;
     uint32_t jb = 0;
     for (;;) {
@@ -80,8 +81,10 @@ static __device__ __forceinline__ void batch_group_phase(const BatchParams &p, c
         const BatchJob &J = jobs[jb];
         const Net n = net_view(J.blob, J.net);
         const unsigned long long local = r - J.run_begin;
-        group_run<32, K, VERIFY>(n, s, J, J.first_run + local, local, lane, 0u, 0xffffffffu, acc_hits, acc_steps,
-                                 acc_capped);
+        const SeedKeys keys{J.seed};
+        const uint32_t bits = ceil_log2(n.n_comps);
+        g.init(n, J);
+        while (!g.finish(n, J, local, acc_hits, acc_steps, acc_capped)) g.advance(n, J, keys, J.first_run + local, bits);
     }
     if (lane == 0) flush_counters(jobs[jb], acc_hits, acc_steps, acc_capped);
 }

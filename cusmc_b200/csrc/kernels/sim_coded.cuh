@@ -94,7 +94,7 @@ static __device__ __forceinline__ float desc_delay(const Net &n, const CodedView
     const uint64_t dsc = n.loc_desc[li];
     const uint32_t lo = static_cast<uint32_t>(dsc), fl = static_cast<uint32_t>(dsc >> 32);
     if (fl & CSMC_DESC_ZERO) return 0.0f;
-    if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) return bounded_delay(n, rv.vars, rv.rates, li, lo, fl, x);
+    if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) return bounded_delay(n.base, rv.vars, rv.rates, li, lo, fl, x);
     const float inv = (fl & CSMC_DESC_PROG) ? rv.rates[lo] : __uint_as_float(lo);
     return exp_delay(x, inv);
 }

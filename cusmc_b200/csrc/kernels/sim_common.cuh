@@ -14,8 +14,13 @@ constexpr double kEps = 0.00001;                     // DBL_EPSILON, include/com
 constexpr double kDblMax = 1.7976931348623158e+308;  // include/common_macros.h:71
 constexpr double kDblMin = 2.2250738585072014e-308;
 
-// The packed network as seen from shared memory.
+// The packed network as seen from shared memory.  Functions that are not
+// inlined take `base` (and rebuild the view) or single pointers, never a
+// reference to the view: a view whose address escapes lives in local memory,
+// every access reloads its pointer from there, and the compiler no longer
+// knows that the tables lie in shared memory.
 struct Net {
+    const uint8_t *base;  // the blob (its header first)
     const csmc_comp *comp;
     const csmc_loc *loc;
     const csmc_edge *edge;
@@ -36,6 +41,7 @@ struct Net {
 static __device__ __forceinline__ Net net_view(const uint8_t *base) {
     const csmc_net_header *h = reinterpret_cast<const csmc_net_header *>(base);
     Net n;
+    n.base = base;
     n.comp = reinterpret_cast<const csmc_comp *>(base + h->off_comp);
     n.loc = reinterpret_cast<const csmc_loc *>(base + h->off_loc);
     n.edge = reinterpret_cast<const csmc_edge *>(base + h->off_edge);
@@ -63,6 +69,7 @@ static __device__ __forceinline__ Net net_view(const uint8_t *base) {
 // The same view with offsets and counts taken from the kernel parameters.
 static __device__ __forceinline__ Net net_view(const uint8_t *base, const NetLayout &l) {
     Net n;
+    n.base = base;
     n.comp = reinterpret_cast<const csmc_comp *>(base + l.off_comp);
     n.loc = reinterpret_cast<const csmc_loc *>(base + l.off_loc);
     n.edge = reinterpret_cast<const csmc_edge *>(base + l.off_edge);
@@ -143,15 +150,15 @@ static __device__ __forceinline__ double apply_op(uint32_t op, double v1, double
 // General programs: a real stack.  PN operators push without popping
 // (expressions.cu:192-193 pass stack_top by value); SKIP pops one; tree
 // operators pop two.
-static __device__ __noinline__ double eval_stack(const Net &n, VarView vars, uint32_t p) {
+static __device__ __noinline__ double eval_stack(const uint64_t *code, const double *konst, VarView vars, uint32_t p) {
     double st[CSMC_MAX_STACK];
     int top = 0;
     for (uint32_t ip = p + 1;; ++ip) {
-        const uint64_t ins = n.code[ip];
+        const uint64_t ins = code[ip];
         const uint32_t op = CSMC_INS_OP(ins), a = CSMC_INS_A(ins);
         double r;
         if (op == CSMC_OP_END) return top > 0 ? st[top - 1] : 0.0;
-        if (op == CSMC_OP_PUSH_C) r = n.konst[a];
+        if (op == CSMC_OP_PUSH_C) r = konst[a];
         else if (op == CSMC_OP_PUSH_V) r = static_cast<double>(vars[a]);
         else if (op == CSMC_OP_SKIP) {
             --top;
@@ -171,15 +178,15 @@ static __device__ __noinline__ double eval_stack(const Net &n, VarView vars, uin
 
 // Programs that only ever read the two top entries (header flag WINDOW)
 // run on two registers; the rest on the stack machine.
-static __device__ __noinline__ double eval_prog(const Net &n, VarView vars, uint32_t p) {
-    if (!(CSMC_INS_A(n.code[p]) & CSMC_PROG_WINDOW)) return eval_stack(n, vars, p);
+static __device__ __noinline__ double eval_prog(const uint64_t *code, const double *konst, VarView vars, uint32_t p) {
+    if (!(CSMC_INS_A(code[p]) & CSMC_PROG_WINDOW)) return eval_stack(code, konst, vars, p);
     double a = 0.0, b = 0.0;
     for (uint32_t ip = p + 1;; ++ip) {
-        const uint64_t ins = n.code[ip];
+        const uint64_t ins = code[ip];
         const uint32_t op = CSMC_INS_OP(ins), x = CSMC_INS_A(ins);
         double r;
         if (op == CSMC_OP_END) return b;
-        if (op == CSMC_OP_PUSH_C) r = n.konst[x];
+        if (op == CSMC_OP_PUSH_C) r = konst[x];
         else if (op == CSMC_OP_PUSH_V) r = static_cast<double>(vars[x]);
         else r = apply_op(op, a, b);
         a = b;
@@ -215,7 +222,7 @@ static __device__ __forceinline__ double eval(const Net &n, VarView vars, uint32
         if (CSMC_INS_OP(i4) != CSMC_OP_END) r = chain_op(CSMC_INS_OP(n.code[p + 5]), r, chain_operand(n, vars, i4));
         return r;
     }
-    return eval_prog(n, vars, p);
+    return eval_prog(n.code, n.konst, vars, p);
 }
 
 // simulation.cu:184-266

@@ -1,7 +1,30 @@
 // Lane-group simulation kernel (see sim.cuh for the mapping); instantiated
 // per (lanes per run, components per lane) shape in sim_shapes_*.cu.
-// Semantics follow the reference kernel line by line; file:line references
-// are to simulation/simulation.cu of the reference.
+// Semantics follow the reference kernel; file:line references are to
+// simulation/simulation.cu of the reference.
+//
+// What bounds it: a run's steps are a serial chain, so a launch that does not
+// fill the GPU takes (steps of its longest run) x (latency of one step), and
+// one that does is bound by instruction issue.  Both ask for few dependent
+// instructions per step:
+//   * what a component's delay needs is one 8-byte record (1/rate and the
+//     delay's form) in shared memory, read as it is by the component's lane
+//     and written again only when the component has moved or the rate table
+//     has changed (kept in registers, the records of 4 to 16 components cost
+//     more in spills than their 16-byte shared loads);
+//   * the rate table is evaluated again only after a transition (unless a
+//     rate reads a clock), the clocks advance by one float addition each;
+//   * the race is two warp-wide integer minima (delay key, then bit-reversed
+//     index) in a full warp, a butterfly of 32-bit words in a narrower group;
+//   * a winner without edges is done there; else the lanes evaluate the
+//     guards of its edges in parallel and one lane takes the chosen edge.
+// All groups of a warp meet at the head of the step loop, so groups whose
+// runs end at different steps keep advancing together.
+// Measured (B200), against the form with a 64-bit butterfly, per-component
+// location records read every step and every step's rate table evaluated:
+// 100 agents, 32 lanes x 4, 64 runs 9.3 -> 3.0 ms, 65,536 runs 142 -> 49 ms
+// (355 warp instructions a step); 256-process mutex, 32 x 8, 2,000 runs
+// 237 -> 157 ms (1,370 -> 729 instructions a step).
 #pragma once
 #include "sim_common.cuh"
 
@@ -12,256 +35,462 @@ struct RunState {  // per group, in shared memory (group_state_stride bytes)
     RunScalars sc;
     uint32_t pad2[2];
     float vars[1];  // n_vars entries, then n_rate_prog inverse rates, then
-                    // (at group_vars_bytes) the slot masks [k * G + lane]
+                    // (at group_vars_bytes) the delay records, the slot
+                    // masks and the global location indices of the components
+};
+
+// Where a run's Philox round keys come from: the kernel's parameter bank
+// (one network, one seed) or the seed itself (a batch job).
+struct BankKeys {
+    const PhiloxKeys &k;
+    __device__ __forceinline__ u32x4 block(uint32_t step, uint64_t run, uint32_t q) const {
+        return philox_one(k, step, run, q);
+    }
+};
+struct SeedKeys {
+    uint64_t seed;
+    __device__ __forceinline__ u32x4 block(uint32_t step, uint64_t run, uint32_t q) const {
+        return delay_block(seed, run, step, q);
+    }
 };
 
 template <bool VERIFY>
-static __device__ __noinline__ uint32_t group_take(const Net &n, RunState *s, uint64_t seed, int32_t var_id,
+static __device__ __noinline__ uint32_t group_take(const uint8_t *base, RunState *s, uint64_t seed, int32_t var_id,
                                                    uint64_t run, uint32_t step, uint32_t c, uint32_t cur_loc,
                                                    uint32_t en, uint32_t slot_mask, uint32_t which) {
-    return take_edge<VERIFY>(n, VarView{s->vars, 1}, s->sc, seed, var_id, run, step, c, cur_loc, en, slot_mask,
-                             which);
+    return take_edge<VERIFY>(net_view(base), VarView{s->vars, 1}, s->sc, seed, var_id, run, step, c, cur_loc, en,
+                             slot_mask, which);
 }
 
-// The winner's step (simulation.cu:656-667): enabled edges, slot update,
-// transition.  Returns the new local location; *slots is updated.
-template <bool VERIFY>
-static __device__ __noinline__ uint32_t win_step(const Net &n, RunState *s, uint64_t seed, int32_t var_id,
-                                                 uint64_t run, uint32_t step, uint32_t c, uint32_t cur_loc,
-                                                 uint32_t *slots) {
-    const uint32_t en = enabled_edges(n, VarView{s->vars, 1}, n.comp[c].loc_begin + cur_loc);
-    *slots = write_slots(*slots, en);
-    if (en) return group_take<VERIFY>(n, s, seed, var_id, run, step, c, cur_loc, en, *slots, 0);
-    if (VERIFY) mix(s->sc.digest, 0xffffffffu);
-    return cur_loc;
+static __device__ __noinline__ uint32_t recv_mask(const uint8_t *base, RunState *s, uint32_t li, int chan) {
+    return recv_edges(net_view(base), VarView{s->vars, 1}, li, chan);
 }
 
-static __device__ __noinline__ uint32_t recv_mask(const Net &n, RunState *s, uint32_t li, int chan) {
-    return recv_edges(n, VarView{s->vars, 1}, li, chan);
+// Delay of a component outside the cached forms (several invariants, a
+// computed bound, a rate that is evaluated per component).
+static __device__ __noinline__ float group_slow_delay(const uint8_t *base, const float *vars, const float *rates,
+                                                      uint32_t li, uint32_t x) {
+    return comp_delay(net_view(base), VarView{const_cast<float *>(vars), 1}, VarView{const_cast<float *>(rates), 1},
+                      li, x);
 }
 
-// One whole run (stream index `run`, output index `ridx`) simulated by the
-// G lanes of a group: lane gl holds components gl*K .. gl*K+K-1 (C <= G*K)
-// and their locations in registers; the group's scalars, variables, rate
-// table and slot masks live in *s (slot masks are touched only by the
-// step's winner and receivers, so they stay out of the registers).  Q supplies the
-// query (seed, max_steps, threshold, horizon, var_id, loc_mode, is_max) and
-// the per-run output arrays (flags, values, steps, digests, final_state; any
-// may be null): the kernel parameters of one network, or one batch job.
-// Lane 0 of the group writes the outputs and adds the run's hits, steps and
-// capped flag to its accumulators.
-template <int G, int K, bool VERIFY, class Q>
-static __device__ __forceinline__ void group_run(const Net &n, RunState *s, const Q &q, uint64_t run,
-                                                 uint64_t ridx, uint32_t gl,
-                                                 uint32_t gbase, uint32_t gmask, unsigned long long &acc_hits,
-                                                 unsigned long long &acc_steps, unsigned long long &acc_capped) {
-    const uint32_t C = n.n_comps, V = n.n_vars;
-    const uint32_t bits = ceil_log2(C);
-    const bool rate_table = (n.flags & CSMC_NET_RATE_TABLE) && n.n_rate_prog > 0;
-    const VarView vars{s->vars, 1};
-    const VarView rates{s->vars + V, 1};
-    const uint32_t c0 = gl * K;
-    const float T = q.horizon;
-    const uint64_t cap = q.max_steps;
+// Form of a component's delay, the second word of its record: exponential,
+// zero, through comp_delay, or the one-invariant word + kFormInv1.
+constexpr uint32_t kFormExp = 0u, kFormZero = 1u, kFormSlow = 2u, kFormInv1 = 3u;
+
+// Key of a delay for 32-bit comparisons (delay_key): one OR unless the
+// delay is negative or NaN.
+static __device__ __forceinline__ uint32_t group_key(float d) {
+    const uint32_t b = f_bits(d);
+    return b <= 0x7f800000u ? (b | 0x80000000u) : delay_key(d);
+}
+
+// Bit reversal of k over the K (a power of two) components of a lane.
+static __host__ __device__ constexpr int lane_brev(int k, int K) {
+    int r = 0;
+    for (int b = 1; b < K; b <<= 1) {
+        r = (r << 1) | (k & 1);
+        k >>= 1;
+    }
+    return r;
+}
+
+// One run at a time simulated by the G lanes of a group: lane gl holds
+// components gl*K .. gl*K+K-1 (C <= G*K).  The group's scalars, variables,
+// rate table, slot masks and locations live in *s.
+template <int G, int K, bool VERIFY>
+struct GroupRun {
+    RunState *s;
+    uint32_t gl, gbase, gmask;
+    uint2 *rec;        // delay records (rec_of)
+    uint32_t *slotv;   // per component
+    uint16_t *locv;    // per component: global location index
+    float *rates;
+    // this run
+    float time;
+    uint32_t step, chan, goal;
+    bool dirty;        // variables changed since the rate table was evaluated
+    uint32_t pm;       // bit k: this lane's component k has its rate from the table
+
+    __device__ __forceinline__ GroupRun(RunState *state, uint32_t lane) {
+        s = state;
+        gl = lane % G;
+        gbase = lane - gl;
+        gmask = G == 32 ? 0xffffffffu : (((1u << (G & 31)) - 1u) << gbase);
+    }
+
+    // Record of this lane's component k: pairs of components side by side
+    // (one 16-byte load), lanes next to each other.
+    __device__ __forceinline__ uint2 *rec_of(int k) const {
+        return K == 1 ? rec + gl : rec + 2 * ((k >> 1) * G + gl) + (k & 1);
+    }
+
+    // Writes component k's record from its location li.
+    __device__ __forceinline__ void look_up(const Net &n, int k, uint32_t li) {
+        const uint64_t dsc = n.loc_desc[li];
+        const uint32_t lo = static_cast<uint32_t>(dsc), fl = static_cast<uint32_t>(dsc >> 32);
+        uint32_t inv = lo, form = kFormExp;
+        pm &= ~(1u << k);
+        if (fl & CSMC_DESC_ZERO) {
+            form = kFormZero;
+        } else if ((fl & CSMC_DESC_EVAL) || (fl & (CSMC_DESC_INV | CSMC_DESC_INV1)) == CSMC_DESC_INV) {
+            form = kFormSlow;
+        } else {
+            if (fl & CSMC_DESC_INV) {
+                const uint32_t w = n.loc_inv1[li];
+                form = w < 0xffffffffu - kFormInv1 ? w + kFormInv1 : kFormSlow;
+            }
+            if (fl & CSMC_DESC_PROG) {
+                pm |= 1u << k;
+                inv = __float_as_uint(rates[lo]);
+            }
+        }
+        *rec_of(k) = make_uint2(inv, form);
+    }
 
     // run initialisation (simulation.cu:766-831)
-    for (uint32_t v = gl; v < V; v += G) s->vars[v] = n.var[v].init;
-    if (gl == 0) {
-        double q0 = 0.0;
-        if (q.var_id >= 0 && static_cast<uint32_t>(q.var_id) < V && n.var[q.var_id].kind == 0)
-            q0 = static_cast<double>(n.var[q.var_id].init);
-        s->sc.qmin = q0;
-        s->sc.qmax = q0;
-        s->sc.chan = 0;
-        s->sc.sender = -1;
-        s->sc.goal = 0;
-        s->sc.digest = 0xcbf29ce484222325ull;
+    template <class Q>
+    __device__ __forceinline__ void init(const Net &n, const Q &q) {
+        const uint32_t C = n.n_comps, V = n.n_vars;
+        uint8_t *tail = reinterpret_cast<uint8_t *>(s) + group_vars_bytes(V, n.n_rate_prog);
+        rec = reinterpret_cast<uint2 *>(tail);
+        slotv = reinterpret_cast<uint32_t *>(tail + 8u * G * K);
+        locv = reinterpret_cast<uint16_t *>(tail + 12u * G * K);
+        rates = s->vars + V;
+        __syncwarp(gmask);  // the lanes are done with the previous run's state
+        for (uint32_t v = gl; v < V; v += G) s->vars[v] = n.var[v].init;
+        if (gl == 0) {
+            double q0 = 0.0;
+            if (q.var_id >= 0 && static_cast<uint32_t>(q.var_id) < V && n.var[q.var_id].kind == 0)
+                q0 = static_cast<double>(n.var[q.var_id].init);
+            s->sc.qmin = q0;
+            s->sc.qmax = q0;
+            s->sc.chan = 0;
+            s->sc.sender = -1;
+            s->sc.goal = 0;
+            s->sc.digest = 0xcbf29ce484222325ull;
+        }
+        for (uint32_t c = gl; c < C; c += G) {
+            locv[c] = static_cast<uint16_t>(n.comp[c].loc_begin + n.comp[c].init_local);
+            slotv[c] = 0u;
+        }
+        __syncwarp(gmask);
+        time = 0.0f;
+        step = 0;
+        chan = 0;
+        goal = 0;
+        pm = 0;
+        eval_rates(n);
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+            const uint32_t c = gl * K + k;
+            if (c < C) look_up(n, k, locv[c]);
+            else *rec_of(k) = make_uint2(0x7fffffffu, kFormExp);  // no component: a delay of NaN
+        }
+        dirty = false;
     }
-    uint32_t loc[K];
-    uint32_t *const slots =
-        reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(s) + group_vars_bytes(V, n.n_rate_prog)) + gl;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const uint32_t c = c0 + k;
-        loc[k] = c < C ? n.comp[c].loc_begin + n.comp[c].init_local : 0u;  // global location index
-        slots[k * G] = 0u;
-    }
-    __syncwarp(gmask);
 
-    float time = 0.0f;
-    uint32_t step = 0;
-    uint32_t flag = 0, capped = 0;
-    while (time < T) {  // simulation.cu:835
-        if (q.loc_mode && s->sc.goal) {  // simulation.cu:839-849
-            flag = 1;
-            break;
+    // distinct rate programs, spread over the lanes
+    __device__ __forceinline__ void eval_rates(const Net &n) {
+        if (!(n.flags & CSMC_NET_RATE_TABLE) || n.n_rate_prog == 0) return;
+        for (uint32_t j = gl; j < n.n_rate_prog; j += G)
+            rates[j] = inv_rate(eval(n, VarView{s->vars, 1}, n.rate_prog[j]));
+        __syncwarp(gmask);
+    }
+
+    // Broadcast receivers of the previous step's sender (SyncInSerial,
+    // simulation.cu:357-407): every enabled set is taken before any receiver
+    // moves, then the receivers move in component order.
+    template <class Q>
+    __device__ __forceinline__ void receivers(const Net &n, const Q &q, uint64_t run) {
+        const uint32_t C = n.n_comps;
+        const int sender = s->sc.sender;
+        uint32_t *const rmv = reinterpret_cast<uint32_t *>(rec);  // the records are written again below
+        bool any = false;
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+            const uint32_t c = gl * K + k;
+            uint32_t m = 0;
+            if (c < C && static_cast<int>(c) != sender && n.loc[locv[c]].n_recv)
+                m = recv_mask(n.base, s, locv[c], static_cast<int>(chan));
+            any |= m != 0;
+            rmv[gl * K + k] = m;
         }
-        if (step >= cap) {
-            capped = 1;
-            break;
-        }
-        // ---- broadcast receivers (SyncInSerial, simulation.cu:357-407)
-        const int chan = s->sc.chan;
-        if (chan > 0) {
-            const int sender = s->sc.sender;
-            uint32_t rm[K];
-            bool any = false;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                rm[k] = 0;
-                const uint32_t c = c0 + k;
-                if (c < C && static_cast<int>(c) != sender && n.loc[loc[k]].n_recv && has_receivers(n, chan)) {
-                    rm[k] = recv_mask(n, s, loc[k], chan);
-                    any |= rm[k] != 0;
+        uint32_t pending = (__ballot_sync(gmask, any) & gmask) >> gbase;
+        __syncwarp(gmask);
+        if (pending) dirty = true;
+        while (pending) {
+            const uint32_t who = static_cast<uint32_t>(__ffs(pending) - 1);
+            if (gl == who) {
+#pragma unroll 1
+                for (int k = 0; k < K; ++k) {
+                    const uint32_t c = gl * K + k, rm = rmv[c];
+                    if (!rm) continue;
+                    const uint32_t base = n.comp[c].loc_begin;
+                    const uint32_t m = write_slots(slotv[c], rm);
+                    slotv[c] = m;
+                    if (VERIFY) mix(s->sc.digest, c | 0x80000000u);
+                    locv[c] = static_cast<uint16_t>(base + group_take<VERIFY>(n.base, s, q.seed, q.var_id, run, step, c,
+                                                                              locv[c] - base, rm, m, 1));
                 }
             }
-            uint32_t pending = (__ballot_sync(gmask, any) & gmask) >> gbase;
-            __syncwarp(gmask);  // every enabled set is taken before any receiver moves
-            while (pending) {
-                const uint32_t who = static_cast<uint32_t>(__ffs(pending) - 1);
-                if (gl == who) {
+            __syncwarp(gmask);
+            pending &= pending - 1;
+        }
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+            const uint32_t c = gl * K + k;
+            if (c < C) look_up(n, k, locv[c]);
+            else *rec_of(k) = make_uint2(0x7fffffffu, kFormExp);
+        }
+        goal = static_cast<uint32_t>(s->sc.goal);
+    }
+
+    // This lane's delays and their minimum (simulation.cu:409-541): key,
+    // bit-reversed index and the delay itself.
+    template <class KEYS>
+    __device__ __forceinline__ void lane_min(const Net &n, const KEYS &keys, uint64_t run, uint32_t bits,
+                                             uint32_t &bkey, uint32_t &bbr, float &bd) {
+        constexpr int B = K < 4 ? K : 4;  // components per Philox block of this lane
+        const uint32_t C = n.n_comps;
+        bkey = 0xffffffffu;
+        bbr = 0xffffffffu;
+        bd = 0.0f;
+#pragma unroll 1
+        for (int b = 0; b < K; b += B) {
+            const uint32_t c = gl * K + b;
+            if (K > 4 && c >= C) break;  // no components from here on
+            uint32_t iv[B], form[B];
+            if (B == 1) {
+                const uint2 r = rec[gl];
+                iv[0] = r.x;
+                form[0] = r.y;
+            } else {
 #pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        if (!rm[k]) continue;
-                        const uint32_t c = c0 + k;
-                        const uint32_t base = n.comp[c].loc_begin;
-                        const uint32_t sm = write_slots(slots[k * G], rm[k]);
-                        slots[k * G] = sm;
-                        if (VERIFY) mix(s->sc.digest, c | 0x80000000u);
-                        loc[k] = base + group_take<VERIFY>(n, s, q.seed, q.var_id, run, step, c, loc[k] - base,
-                                                           rm[k], sm, 1);
+                for (int h = 0; h < B / 2; ++h) {
+                    const uint4 r = *reinterpret_cast<const uint4 *>(rec_of(b + 2 * h));
+                    iv[2 * h] = r.x;
+                    form[2 * h] = r.y;
+                    iv[2 * h + 1] = r.z;
+                    form[2 * h + 1] = r.w;
+                }
+            }
+            const u32x4 blk = keys.block(step, run, c >> 2);
+            float d[B];
+            uint32_t special = 0;
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                d[i] = exp_delay(B == 4 ? word_of(blk, i) : word_of(blk, (c + i) & 3u), __uint_as_float(iv[i]));
+                special |= form[i];
+            }
+            if (special) {
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    const uint32_t x = B == 4 ? word_of(blk, i) : word_of(blk, (c + i) & 3u);
+                    if (form[i] >= kFormInv1) {
+                        // uniform on (0, bound - clock] while the bound lies
+                        // ahead (comp_delay's arithmetic, inv1_delay)
+                        const uint32_t w = form[i] - kFormInv1;
+                        double ttb = d_sub(n.konst[CSMC_INV1_CONST(w)], static_cast<double>(s->vars[CSMC_INV1_VAR(w)]));
+                        if (CSMC_INV1_STRICT(w)) ttb = d_sub(ttb, 1e-6);
+                        if (ttb >= 0) d[i] = uniform_delay(x, ttb);
+                    } else if (form[i] == kFormZero) {
+                        d[i] = 0.0f;
+                    } else if (form[i] == kFormSlow) {
+                        d[i] = group_slow_delay(n.base, s->vars, rates, locv[c + i], x);
                     }
                 }
-                __syncwarp(gmask);
-                pending &= pending - 1;
             }
+            uint32_t key = 0xffffffffu;
+            int kk = 0;
+            float d0 = 0.0f;
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                // in order of bit-reversed index, so a later equal key loses
+                const int i = lane_brev(j, B);
+                const uint32_t kd = group_key(d[i]);
+                if (kd < key) {
+                    key = kd;
+                    kk = i;
+                    d0 = d[i];
+                }
+            }
+            const uint32_t br = bitrev_bits(c + kk, bits);
+            if (key < bkey || (key == bkey && key != 0xffffffffu && br < bbr)) {
+                bkey = key;
+                bbr = br;
+                bd = d0;
+            }
+        }
+    }
+
+    // The lowest bit-reversed index among this lane's components (a race in
+    // which every delay is NaN).
+    __device__ __forceinline__ uint32_t lowest_brev(uint32_t C, uint32_t bits) const {
+        uint32_t r = 0xffffffffu;
+        for (uint32_t k = 0; k < K; ++k)
+            if (gl * K + k < C) r = min(r, bitrev_bits(gl * K + k, bits));
+        return r;
+    }
+
+    static __device__ __forceinline__ uint32_t group_min(uint32_t v, uint32_t mask) {
+        if (G == 32) return __reduce_min_sync(mask, v);
+#pragma unroll
+        for (int off = G / 2; off > 0; off >>= 1) v = min(v, __shfl_xor_sync(mask, v, off, G));
+        return v;
+    }
+
+    // One step of the run: receivers, rate table, delays, race, clock
+    // advance, the winner's transition, time.
+    template <class Q, class KEYS>
+    __device__ __forceinline__ void advance(const Net &n, const Q &q, const KEYS &keys, uint64_t run, uint32_t bits) {
+        const VarView vars{s->vars, 1};
+        if (chan) {
+            if (has_receivers(n, static_cast<int>(chan))) receivers(n, q, run);
+            __syncwarp(gmask);
             if (gl == 0) {
                 s->sc.chan = 0;
                 s->sc.sender = -1;
             }
+            chan = 0;
             __syncwarp(gmask);
         }
-
-        // ---- distinct rate programs, once per step per run
-        if (rate_table) {
-            for (uint32_t j = gl; j < n.n_rate_prog; j += G) rates[j] = inv_rate(eval(n, vars, n.rate_prog[j]));
-            __syncwarp(gmask);
-        }
-
-        // ---- delays (simulation.cu:409-541)
-        unsigned long long best = ~0ull;
-        float bestd = 0.0f;
-        u32x4 blk{0, 0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint32_t c = c0 + k;
-            if (c < C) {
-                uint32_t x;
-                if (K % 4 == 0) {
-                    if (k % 4 == 0) blk = delay_block(q.seed, run, step, c >> 2);
-                    x = word_of(blk, static_cast<uint32_t>(k & 3));
-                } else {
-                    x = delay_word(q.seed, run, step, c);
-                }
-                const float d = comp_delay(n, vars, rates, loc[k], x);
-                const unsigned long long key =
-                    (static_cast<unsigned long long>(delay_key(d)) << 32) | bitrev_bits(c, bits);
-                if (key < best) {
-                    best = key;
-                    bestd = d;
-                }
+        if (dirty || !(n.flags & CSMC_NET_RATE_NO_CLOCK)) {
+            eval_rates(n);
+            for (uint32_t left = pm; left; left &= left - 1) {
+                const int k = __ffs(left) - 1;
+                rec_of(k)->x = __float_as_uint(rates[static_cast<uint32_t>(n.loc_desc[locv[gl * K + k]])]);
             }
+            dirty = false;
         }
-        // ---- race (simulation.cu:553-628): segmented butterfly min
-#pragma unroll
-        for (int off = G / 2; off > 0; off >>= 1) {
-            const unsigned long long ob = __shfl_xor_sync(gmask, best, off, G);
-            const float od = __shfl_xor_sync(gmask, bestd, off, G);
-            if (ob < best) {
-                best = ob;
-                bestd = od;
-            }
+
+        // ---- delays and the race (simulation.cu:409-628)
+        uint32_t bkey, bbr;
+        float bd;
+        lane_min(n, keys, run, bits, bkey, bbr, bd);
+        const uint32_t m = group_min(bkey, gmask);
+        if (m == 0xffffffffu) {
+            bbr = lowest_brev(n.n_comps, bits);
+            bd = __uint_as_float(0x7fffffffu);
         }
-        const uint32_t win = bitrev_bits(static_cast<uint32_t>(best & 0xffffffffull), bits);
-        const float dmin = bestd;
+        const uint32_t win = bitrev_bits(group_min(bkey == m ? bbr : 0xffffffffu, gmask), bits);
         const uint32_t owner = win / K;
-        if (VERIFY && gl == owner) {
+        const float dmin = G == 1 ? bd : __shfl_sync(gmask, bd, owner, G);
+        if (VERIFY && gl == 0) {
             mix(s->sc.digest, step);
             mix(s->sc.digest, win);
             mix(s->sc.digest, f_bits(dmin));
         }
-        if (static_cast<double>(dmin) < kDblMax) {
+        if (dmin < __uint_as_float(0x7f800000u)) {
             // clocks advance (simulation.cu:632-651)
-            for (uint32_t j = gl; j < n.n_clocks; j += G) {
-                const uint32_t v = n.clock[j];
-                s->vars[v] = d2f(d_add(static_cast<double>(s->vars[v]), static_cast<double>(dmin)));
-            }
-            __syncwarp(gmask);
-            if (gl == owner) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    if (c0 + k != win) continue;
-                    const uint32_t base = n.comp[win].loc_begin;
-                    loc[k] = base + win_step<VERIFY>(n, s, q.seed, q.var_id, run, step, win, loc[k] - base,
-                                                     &slots[k * G]);
+            if (n.n_clocks) {
+                for (uint32_t j = gl; j < n.n_clocks; j += G) {
+                    const uint32_t v = n.clock[j];
+                    s->vars[v] = time_add(s->vars[v], dmin);
                 }
+                __syncwarp(gmask);
             }
-            __syncwarp(gmask);
+            // the winner's enabled edges (simulation.cu:268-305), one lane per edge
+            const uint32_t li = locv[win];
+            const csmc_loc L = n.loc[li];
+            uint32_t en = 0;
+            for (uint32_t e0 = 0; e0 < L.n_edges; e0 += G) {
+                bool ok = false;
+                if (e0 + gl < L.n_edges) {
+                    const csmc_edge e = n.edge[L.edge_begin + e0 + gl];
+                    ok = e.channel >= 0 && guards_ok(n, vars, e);
+                }
+                const uint32_t b = G == 1 ? (ok ? 1u : 0u) : ((__ballot_sync(gmask, ok) & gmask) >> gbase);
+                en |= b << e0;
+            }
+            if (en) {
+                if (gl == 0) {
+                    const uint32_t base = n.comp[win].loc_begin;
+                    const uint32_t slots = write_slots(slotv[win], en);
+                    slotv[win] = slots;
+                    locv[win] = static_cast<uint16_t>(base + take_edge<VERIFY>(n, vars, s->sc, q.seed, q.var_id, run,
+                                                                               step, win, li - base, en, slots, 0));
+                }
+                __syncwarp(gmask);
+                dirty = true;
+                chan = static_cast<uint32_t>(s->sc.chan);
+                goal = static_cast<uint32_t>(s->sc.goal);
+                if (gl == owner) look_up(n, static_cast<int>(win % K), locv[win]);
+            } else if (VERIFY && gl == 0) {
+                mix(s->sc.digest, 0xffffffffu);
+            }
         }
-        time = d2f(d_add(static_cast<double>(time), static_cast<double>(dmin)));  // simulation.cu:876-882
+        time = time_add(time, dmin);  // simulation.cu:876-882
         ++step;
     }
 
-    // per-run outputs (simulation.cu:887-893)
-    if (gl == 0) {
-        const double val = q.is_max ? s->sc.qmax : s->sc.qmin;
-        uint32_t f = flag;
-        if (!q.loc_mode) f = q.is_max ? (val > q.threshold) : (val < q.threshold);
-        if (q.flags) q.flags[ridx] = static_cast<uint8_t>(f);
-        if (q.values) q.values[ridx] = val;
-        if (q.steps) q.steps[ridx] = step;
-        if (VERIFY && q.digests) q.digests[ridx] = s->sc.digest;
-        acc_hits += f;
-        acc_steps += step;
-        acc_capped += capped;
+    // Ended runs (simulation.cu:835-849, 887-893): true when the run is over;
+    // the first lane writes its outputs and adds to its counters.
+    template <class Q>
+    __device__ __forceinline__ bool finish(const Net &n, const Q &q, uint64_t ridx, unsigned long long &acc_hits,
+                                           unsigned long long &acc_steps, unsigned long long &acc_capped) {
+        const bool timeout = !(time < q.horizon);
+        const bool at_goal = q.loc_mode && goal;
+        if (!timeout && !at_goal && step < q.max_steps) return false;
+        if (gl == 0) {
+            const double val = q.is_max ? s->sc.qmax : s->sc.qmin;
+            uint32_t f = (!timeout && at_goal) ? 1u : 0u;
+            if (!q.loc_mode) f = q.is_max ? (val > q.threshold) : (val < q.threshold);
+            if (q.flags) q.flags[ridx] = static_cast<uint8_t>(f);
+            if (q.values) q.values[ridx] = val;
+            if (q.steps) q.steps[ridx] = step;
+            if (VERIFY && q.digests) q.digests[ridx] = s->sc.digest;
+            acc_hits += f;
+            acc_steps += step;
+            acc_capped += (!timeout && !at_goal) ? 1u : 0u;
+        }
+        if (VERIFY && q.final_state) {
+            const uint32_t C = n.n_comps, V = n.n_vars;
+            uint32_t *w = q.final_state + ridx * (C + V);
+            for (uint32_t c = gl; c < C; c += G) w[c] = locv[c] - n.comp[c].loc_begin;
+            for (uint32_t v = gl; v < V; v += G) w[C + v] = f_bits(s->vars[v]);
+        }
+        return true;
     }
-    if (VERIFY && q.final_state) {
-        uint32_t *w = q.final_state + ridx * (C + V);
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (c0 + k < C) w[c0 + k] = loc[k] - n.comp[c0 + k].loc_begin;
-        for (uint32_t v = gl; v < V; v += G) w[C + v] = f_bits(s->vars[v]);
-    }
-    __syncwarp(gmask);
-}
+};
 
 #ifndef CSMC_MIN_CTAS_PER_SM
 #define CSMC_MIN_CTAS_PER_SM 2
 #endif
 
 template <int G, int K, bool VERIFY>
-__global__ void __launch_bounds__(256, CSMC_MIN_CTAS_PER_SM) sim_kernel(const SimParams p) {
+__global__ void __launch_bounds__(256, CSMC_MIN_CTAS_PER_SM) sim_kernel(const __grid_constant__ SimParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     stage_network(smem, p.blob, p.blob_bytes);
     __syncthreads();
-    const Net n = net_view(smem);
-
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t gl = lane % G;  // lane within group
-    const uint32_t gbase = lane - gl;
-    const uint32_t gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << gbase);
-    RunState *s = reinterpret_cast<RunState *>(smem + p.blob_bytes + (threadIdx.x / G) * p.state_stride);
+    const Net n = net_view(smem, p.net);
+    const uint32_t bits = ceil_log2(p.net.n_comps);
+    const BankKeys keys{p.keys};
+    GroupRun<G, K, VERIFY> r(reinterpret_cast<RunState *>(smem + p.blob_bytes + (threadIdx.x / G) * p.state_stride),
+                             threadIdx.x & 31u);
 
     unsigned long long acc_hits = 0, acc_steps = 0, acc_capped = 0;
+    unsigned long long ridx = 0;
+    bool have = false, drained = false;
     for (;;) {
-        unsigned long long ridx = 0;
-        if (gl == 0) ridx = atomicAdd(p.scratch, 1ull);
-        ridx = __shfl_sync(gmask, ridx, 0, G);
-        if (ridx >= p.n_runs) break;
-        group_run<G, K, VERIFY>(n, s, p, p.first_run + ridx, ridx, gl, gbase, gmask, acc_hits, acc_steps,
-                                acc_capped);
+        __syncwarp();
+        if (!have && !drained) {
+            if (r.gl == 0) ridx = atomicAdd(p.scratch, 1ull);
+            ridx = __shfl_sync(r.gmask, ridx, 0, G);
+            if (ridx >= p.n_runs) {
+                drained = true;
+            } else {
+                have = true;
+                r.init(n, p);
+            }
+        }
+        if (__all_sync(0xffffffffu, drained)) break;
+        if (have) {
+            if (r.finish(n, p, ridx, acc_hits, acc_steps, acc_capped)) have = false;
+            else r.advance(n, p, keys, p.first_run + ridx, bits);
+        }
     }
-    if (gl == 0) {
+    if (r.gl == 0) {
         if (acc_hits) atomicAdd(p.scratch + 1, acc_hits);
         if (acc_steps) atomicAdd(p.scratch + 2, acc_steps);
         if (acc_capped) atomicAdd(p.scratch + 3, acc_capped);

@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(CSMC_IS_BLOCK, CSMC_IS_MIN_CTAS_PER_SM) is_war
             }
             __syncwarp();
             stale = __shfl_sync(kFullWarp, took, 0) != 0 || (p.net.n_clocks > 0 && finite);
-            time = d2f(d_add(static_cast<double>(time), static_cast<double>(dmin)));
+            time = time_add(time, dmin);
             ++step;
         }
     }

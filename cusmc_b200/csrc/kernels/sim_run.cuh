@@ -20,8 +20,9 @@ namespace detail {
 // Delay of a component whose descriptor flags INV or EVAL: the one-
 // invariant form inline here, the rest through comp_delay.  One call site
 // per component keeps the race loops' register budget.
-static __device__ __noinline__ float bounded_delay(const Net &n, VarView vars, VarView rates, uint32_t li,
+static __device__ __noinline__ float bounded_delay(const uint8_t *base, VarView vars, VarView rates, uint32_t li,
                                                    uint32_t lo, uint32_t fl, uint32_t x) {
+    const Net n = net_view(base);
     if (fl & CSMC_DESC_INV1) return inv1_delay(n, vars, rates, li, lo, fl, x);
     return comp_delay(n, vars, rates, li, x);
 }
@@ -181,7 +182,7 @@ static __device__ __forceinline__ bool run_commit(const Net &n, uint32_t n_clock
     if (static_cast<double>(dmin) < kDblMax) {
         for (uint32_t j = 0; j < n_clocks; ++j) {
             const uint32_t v = n.clock[j];
-            vars[v] = d2f(d_add(static_cast<double>(vars[v]), static_cast<double>(dmin)));
+            vars[v] = time_add(vars[v], dmin);
         }
         const uint32_t li = rv.loc(n, win);
         const uint32_t en = enabled_edges(n, vars, li);
@@ -199,7 +200,7 @@ static __device__ __forceinline__ bool run_commit(const Net &n, uint32_t n_clock
             mix(sc.digest, 0xffffffffu);
         }
     }
-    time = d2f(d_add(static_cast<double>(time), static_cast<double>(dmin)));
+    time = time_add(time, dmin);
     ++step;
     return took;
 }
@@ -230,7 +231,7 @@ static __device__ __forceinline__ void race_exact(const Net &n, uint32_t C, uint
                 if (fl & CSMC_DESC_PROG) inv = rv.rates[lo];
                 float d = exp_delay(x, inv);
                 if (fl & (CSMC_DESC_ZERO | CSMC_DESC_INV | CSMC_DESC_EVAL))
-                    d = (fl & CSMC_DESC_ZERO) ? 0.0f : bounded_delay(n, rv.vars, rv.rates, li, lo, fl, x);
+                    d = (fl & CSMC_DESC_ZERO) ? 0.0f : bounded_delay(n.base, rv.vars, rv.rates, li, lo, fl, x);
                 const unsigned long long key =
                     (static_cast<unsigned long long>(delay_key(d)) << 32) | bitrev_bits(cc, bits);
                 if (key < best) {
@@ -290,7 +291,7 @@ static __device__ __forceinline__ bool race_classes(const Net &n, uint32_t C, ui
                     if (fl & CSMC_DESC_ZERO) {
                         d = 0.0f;
                     } else if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) {
-                        d = bounded_delay(n, rv.vars, rv.rates, li, lo, fl, x);
+                        d = bounded_delay(n.base, rv.vars, rv.rates, li, lo, fl, x);
                     } else {
                         const float inv = (fl & CSMC_DESC_PROG) ? rv.rates[lo] : __uint_as_float(lo);
                         d = exp_delay(x, inv);

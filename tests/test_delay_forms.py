@@ -1,0 +1,44 @@
+"""The device forms of the exponential delay and of the clock advance give
+the bits of the definitions they replace.
+
+* exp_delay: the integer draw's exponent and mantissa are split before the
+  scaling and the logarithm's quotient is a Markstein division; every one of
+  the 2^24 draws is compared with the host's form (tolerance: none).
+* time_add: one float addition instead of a double sum rounded to float.
+"""
+import numpy as np
+import pytest
+
+import oracle
+
+
+@pytest.mark.gpu
+def test_exp_delay_of_every_draw_equals_the_host():
+    import torch
+    from cusmc_b200 import _native
+    from cusmc_b200._native import check, lib
+    x = np.arange(1 << 24, dtype=np.uint32) << np.uint32(8)
+    inv = np.ones(x.size, dtype=np.float32)
+    got = torch.empty(x.size, dtype=torch.float32, device="cuda")
+    xd, invd = torch.from_numpy(x.view(np.int32)).cuda(), torch.from_numpy(inv).cuda()
+    check(lib().csmc_numeric_eval(_native.NUM_EXP_DELAY, xd.data_ptr(), invd.data_ptr(), x.size, got.data_ptr(), None))
+    torch.cuda.synchronize()
+    want = oracle.numeric(_native.NUM_EXP_DELAY, x, inv)
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+def test_float_sum_equals_the_double_sum_rounded_to_float():
+    """Random floats over all exponents (subnormal results, cancellation,
+    exponent gaps around the 24- and 53-bit limits, overflow)."""
+    rng = np.random.default_rng(5)
+    n = 4_000_000
+    a = rng.integers(0, 2**32, n, dtype=np.uint64).astype(np.uint32).view(np.float32)
+    gap = rng.integers(-60, 61, n)
+    m = (1.0 + rng.integers(0, 2**23, n) * 2.0 ** -23) * rng.choice([-1.0, 1.0], n)
+    with np.errstate(all="ignore"):
+        b = np.where(np.isfinite(a), np.ldexp(m, np.frexp(a)[1] + gap), 1.0).astype(np.float32)
+        ok = np.isfinite(a) & np.isfinite(b)
+        a, b = a[ok], b[ok]
+        once = a + b
+        twice = (a.astype(np.float64) + b.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(once.view(np.uint32), twice.view(np.uint32))
