@@ -107,7 +107,7 @@ bool configure_plan(csmc_net *n, int family, int lanes, int cpl, int block, std:
         }
         const csmc::NetLayout L = csmc::layout_of(h);
         const size_t slab = csmc::coded_slab_bytes(h.n_comps, h.n_vars, h.n_rate_prog, n->slots, block, L.n_classes,
-                                                   (h.recv_chan_lo | h.recv_chan_hi) != 0);
+                                                   (h.recv_chan_lo | h.recv_chan_hi) != 0, CSMC_CODED_KEY_BYTES);
         if (n->bytes + slab > max_smem) {
             why = "network and run state do not fit in shared memory";
             return false;
@@ -471,6 +471,7 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
             }
             n->class_src[g] = (fl & CSMC_DESC_PROG) ? (CSMC_CLASS_SRC_PROG | lo) : lo;
         }
+        n->all_classed = n->all_classed && h->n_comps % 4 == 0;
         // tilt groups of importance sampling one thread per run: the
         // (race class, location class) pairs in order of first appearance,
         // the first CSMC_IS_GROUPS of them; later pairs take the
@@ -504,7 +505,7 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
             bool spill = false;  // a classed location's pair beyond the groups
             for (uint32_t g = 0; g < CSMC_RACE_CLASSES; ++g)
                 for (uint32_t l = 0; l < 4; ++l) spill = spill || id[g][l] == 7;
-            n->is_all_grouped = n->all_classed && !spill && h->n_comps % 4 == 0;
+            n->is_all_grouped = n->all_classed && !spill;
         }
     }
     // default plan: the class-coded thread-per-run kernel when the network

@@ -31,7 +31,7 @@ struct csmc_net {
     bool slots = false;
     bool loc8 = false;     // every automaton has at most 256 locations
     bool classes = false;  // delay descriptors carry race classes
-    bool all_classed = false;  // every location belongs to a race class
+    bool all_classed = false;  // every location belongs to a race class, components a multiple of four
     uint32_t class_src[CSMC_RACE_CLASSES] = {};  // 1/rate source of each class (SimParams::class_src)
     bool state_in_global = false;
     uint8_t *d_state = nullptr;  // thread-per-run state slabs (global-state plans)

@@ -103,17 +103,20 @@ int serial_max_active_ctas(bool verify, bool slots, bool loc8, bool gstate, bool
 // Class-coded thread-per-run kernel (sim_coded.cuh): networks with race
 // classes, at most 256 components and at most 32 locations per automaton,
 // run state in shared memory.
-// all_classed: every location of the network belongs to a race class.
+// all_classed: every location of the network belongs to a race class and the
+// component count is a multiple of four.
 int coded_launch(bool verify, bool slots, bool all_classed, const SimParams &p, int grid, int block, size_t smem,
                  void *stream);
 int coded_max_active_ctas(bool verify, bool slots, bool all_classed, int block, size_t smem, int *ctas);
 // Bytes of a T-thread state slab of the class-coded kernel
 // (carve_coded_view): n_classes race classes, recv: the network has
-// receiving edges (the receiver snapshot is kept).
+// receiving edges (the receiver snapshot is kept), key_bytes: of the keys of
+// one class (four chains).
+#define CSMC_CODED_KEY_BYTES 2048u /* the class-coded kernel: chains of 128 threads whatever the CTA's size */
 inline size_t coded_slab_bytes(uint32_t n_comps, uint32_t n_vars, uint32_t n_rate_prog, bool slots, uint32_t T,
-                               uint32_t n_classes, bool recv) {
+                               uint32_t n_classes, bool recv, uint32_t key_bytes) {
     size_t b = 4u * ((recv ? 2u : 1u) * n_vars + n_rate_prog) * static_cast<size_t>(T);
-    b += 4u * 4u * n_classes * static_cast<size_t>(T);             // class keys: the largest of each chain
+    b += static_cast<size_t>(key_bytes) * n_classes;                 // class keys: the largest of each chain
     b += 4u * ((n_comps + 3u) / 4u) * static_cast<size_t>(T);        // location words
     if (slots) b += 4u * n_comps * static_cast<size_t>(T);          // enabled-edge slot masks
     return (b + 15u) & ~static_cast<size_t>(15);
@@ -251,7 +254,7 @@ size_t is_coded_warp_smem_bytes();
 inline size_t is_coded_slab_bytes(uint32_t n_comps, uint32_t n_vars, uint32_t n_rate_prog, bool slots, uint32_t T,
                                   uint32_t n_groups, bool recv) {
     return 16u * n_groups * static_cast<size_t>(T) + coded_slab_bytes(n_comps, n_vars, n_rate_prog, slots, T,
-                                                                     n_groups, recv);
+                                                                     n_groups, recv, 16u * T);
 }
 
 // tc: theta by warp-level tensor-core MMAs (else the CUDA-core evaluation

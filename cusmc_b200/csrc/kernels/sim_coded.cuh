@@ -8,24 +8,36 @@
 // bytes of components 4q..4q+3 form word q of the thread's state, so one
 // shared load gives the codes of the four components that share Philox
 // block q.  A class member contributes only its key, (24-bit draw) * 256 +
-// (255 - bit-reversed index), to its class's largest key; each class keeps
-// four independent maxima, one per word of the Philox block (chain k), so
-// consecutive members of a class do not wait on each other's shared-memory
-// update.  After the components, the chains of a class are merged and the
-// class takes part in the race with its largest key, as in race_classes
-// (sim_run.cuh).  Where race_classes consults the second largest key (a
-// lower draw that rounds to the same float delay could hide a member with a
-// smaller index), this kernel falls back to race_exact whenever the largest
-// draw of a class whose delay is the race's minimum sits on such a flat
-// spot of the delay function (about 2e-4 .. 4e-3 per step for a class of
-// 1-10 members, far less with many); delays do not increase with the
-// draw, so no flat spot means no tie with a lower draw.
+// (255 - bit-reversed q), to its class's largest key; each class keeps four
+// independent maxima, one per word of the Philox block (chain k).  A block's
+// four key words are loaded together, then stored together (the chains are
+// disjoint; member by member, every load would wait behind the store before
+// it), and the key's address is the thread's own key address plus the code
+// field moved to the class stride: one mask, one shift-and-add.  After the
+// components, the chains of a class are merged (a chain's keys stand for
+// its part of the bit-reversed index) and the class takes part in the race
+// with its largest key, as in race_classes (sim_run.cuh).  Where
+// race_classes consults the second largest key (a lower draw that rounds to
+// the same float delay could hide a member with a smaller index), this
+// kernel falls back to race_exact whenever the largest draw of the winning
+// class sits on such a flat spot of the delay function (about 2e-4 .. 4e-3
+// per step for a class of 1-10 members, far less with many), and whenever
+// two classes tie; delays do not increase with the draw, so no flat spot
+// means no tie with a lower draw.
 //
 // The Philox blocks of a step are computed through philox_step /
 // philox_block (csmc_numeric.h): the counter words the blocks share are
 // folded once per step, and the round keys are kernel parameters.  The
 // per-step rate table is evaluated again only after a step that moved a
 // component, unless a rate program reads a clock.
+//
+// What bounds it: per block of four components and 32 runs, 16 wide multiplies
+// of Philox at 4 cycles each on the FMA-heavy pipe and about 37 two-cycle
+// integer operations on the ALU pipe; the race loop alone runs at 75 cycles a
+// block with four warps per scheduler (both pipes full), the rest of a step
+// (class delays, rate table, transition) is latency.  100-agent epidemic, 1e6
+// runs (B200): 223 ms with one load-update-store per member in turn, 180 ms
+// with a block's four loads first (and one flat-spot check per step).
 //
 // Results are those of serial_kernel: the same draws, the same race
 // outcome, the same transitions.
@@ -40,18 +52,33 @@ namespace detail {
 constexpr uint32_t kCodeGeneral = 7u;  // delay through the location's descriptor
 constexpr uint32_t kCodePad = 6u;      // no component
 #ifndef CSMC_CODED_UNROLL
-#define CSMC_CODED_UNROLL 1
+#define CSMC_CODED_UNROLL 2
 #endif
 constexpr int kCodedUnroll = CSMC_CODED_UNROLL;  // Philox blocks of the race loop in flight per iteration
+// Bytes between the chains of a class and between classes (threads of a CTA
+// next to each other, at most 128).
+constexpr uint32_t kKeyChain = 4u * 128u, kKeyClass = 4u * kKeyChain;
+static_assert(kKeyClass == CSMC_CODED_KEY_BYTES, "coded_slab_bytes");
+
+static __device__ __forceinline__ uint32_t ld_key(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+static __device__ __forceinline__ void st_key(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v));
+}
 
 // Run state of one thread in the class-coded layout: vars[V] | rates[P] |
 // shadow[V] (floats; only for networks with receiving edges, else the
 // snapshot view aliases the variables and is never used) | class keys
-// ([class*4 + chain], NG classes) | location words [ceil(C/4)] | slots[C]
-// (all 4-byte words); element i of thread t at [i * T + t].
+// (kKeyClass bytes per class) | location words [ceil(C/4)] | slots[C]
+// (all 4-byte words); element i of thread t at [i * T + t], the keys at
+// class * kKeyClass + chain * kKeyChain + 4 t.
 struct CodedView {
     VarView vars, rates, shadow;
-    uint32_t *keys;   // this thread's chain 0 of class 0; stride T
+    uint32_t keys;    // shared-memory address of this thread's chain 0 of class 0
+    uint32_t *kp;     // the same as a pointer
     uint32_t *lw;     // this thread's location word 0; stride T
     uint32_t *slotv;  // this thread's element 0; stride T
     uint32_t T;
@@ -70,18 +97,20 @@ struct CodedView {
     }
 };
 
+// key_bytes: of the keys of all classes.
 static __host__ __device__ __forceinline__ uint32_t coded_words(uint32_t C) { return (C + 3u) >> 2; }
 
 static __device__ __forceinline__ CodedView carve_coded_view(uint8_t *st, uint32_t V, uint32_t P, uint32_t C,
-                                                             uint32_t NG, bool recv, uint32_t T, uint32_t t) {
+                                                             uint32_t key_bytes, bool recv, uint32_t T, uint32_t t) {
     float *fb = reinterpret_cast<float *>(st);
     CodedView r;
     r.vars = VarView{fb + t, T};
     r.rates = VarView{fb + V * T + t, T};
     r.shadow = recv ? VarView{fb + (V + P) * T + t, T} : r.vars;
     const uint32_t kb = 4u * ((recv ? 2u : 1u) * V + P) * T;
-    r.keys = reinterpret_cast<uint32_t *>(st + kb) + t;
-    const uint32_t lb = kb + 4u * 4u * NG * T;
+    r.keys = static_cast<uint32_t>(__cvta_generic_to_shared(st + kb)) + 4u * t;
+    r.kp = reinterpret_cast<uint32_t *>(st + kb) + t;
+    const uint32_t lb = kb + key_bytes;
     r.lw = reinterpret_cast<uint32_t *>(st + lb) + t;
     r.slotv = reinterpret_cast<uint32_t *>(st + lb + 4u * coded_words(C) * T) + t;
     r.T = T;
@@ -99,24 +128,44 @@ static __device__ __forceinline__ float desc_delay(const Net &n, const CodedView
     return exp_delay(x, inv);
 }
 
-// One component's part in the race: a class member updates its class's
-// chain-k largest key, any other component (ALLCLS false) races with its own
-// delay.  cb: 255 minus the component's bit-reversed index (bitrev_bits(cc,
-// bits)), the low byte of its class key: (x | 0xff) - br = (x & ~0xff) | cb.
-template <bool ALLCLS, uint32_t k>
-static __device__ __forceinline__ void race_member(const Net &n, uint32_t bits, const CodedView &rv, uint32_t wd,
-                                                   uint32_t cc, uint32_t x, uint32_t cb, unsigned long long &best,
-                                                   float &bestd) {
+// The address of member k's key: chain k of the class in byte k of wd.
+template <uint32_t k>
+static __device__ __forceinline__ uint32_t key_addr(const CodedView &rv, uint32_t wd) {
+    static_assert(kKeyClass == 2048u, "the code field moves from bit 8k + 5 to bit 11");
+    const uint32_t f = wd & (0xe0u << (8u * k));
+    return rv.keys + (k == 0 ? f << 6 : f >> (8u * k - 6u));
+}
+
+// The four members of Philox block q, all of them class members.  cb: 255
+// minus the bit-reversed q, the low byte of their keys.
+static __device__ __forceinline__ void race_block(const CodedView &rv, uint32_t wd, const u32x4 &x, uint32_t cb) {
+    const uint32_t a0 = key_addr<0>(rv, wd), a1 = key_addr<1>(rv, wd), a2 = key_addr<2>(rv, wd),
+                   a3 = key_addr<3>(rv, wd);
+    const uint32_t o0 = ld_key(a0), o1 = ld_key(a1 + kKeyChain), o2 = ld_key(a2 + 2u * kKeyChain),
+                   o3 = ld_key(a3 + 3u * kKeyChain);
+    st_key(a0, max(o0, (x.x & 0xffffff00u) | cb));
+    st_key(a1 + kKeyChain, max(o1, (x.y & 0xffffff00u) | cb));
+    st_key(a2 + 2u * kKeyChain, max(o2, (x.z & 0xffffff00u) | cb));
+    st_key(a3 + 3u * kKeyChain, max(o3, (x.w & 0xffffff00u) | cb));
+}
+
+// One member of a block with members outside the classes: a class member
+// updates its key, a general one races with its own delay, padding is
+// skipped.
+template <uint32_t k>
+static __device__ __forceinline__ void race_member(const Net &n, const CodedView &rv, uint32_t wd, uint32_t cc,
+                                                   uint32_t x, uint32_t cb, uint32_t hi_shift,
+                                                   unsigned long long &best, float &bestd) {
     const uint32_t b = (wd >> (8u * k)) & 0xffu;
     const uint32_t code = b >> 5;
-    const uint32_t T = rv.T;
-    if (ALLCLS || code < CSMC_RACE_CLASSES) {
-        const uint32_t key = (x & 0xffffff00u) | cb;
-        uint32_t *pp = rv.keys + (code * 4u + k) * T;
-        *pp = max(*pp, key);
+    if (code < CSMC_RACE_CLASSES) {
+        const uint32_t a = key_addr<k>(rv, wd) + k * kKeyChain;
+        st_key(a, max(ld_key(a), (x & 0xffffff00u) | cb));
     } else if (code == kCodeGeneral) {
         const float d = desc_delay(n, rv, n.comp[cc].loc_begin + (b & 31u), x);
-        const unsigned long long key = (static_cast<unsigned long long>(delay_key(d)) << 32) | (255u - cb);
+        constexpr uint32_t kr = ((k & 1u) << 1) | (k >> 1);
+        const unsigned long long key =
+            (static_cast<unsigned long long>(delay_key(d)) << 32) | (255u - cb + (kr << hi_shift));
         if (key < best) {
             best = key;
             bestd = d;
@@ -124,59 +173,69 @@ static __device__ __forceinline__ void race_member(const Net &n, uint32_t bits, 
     }
 }
 
+// race_exact out of line: the view of the network is rebuilt, the run state's
+// view passed by value.
+struct RaceOutcome {
+    unsigned long long best;
+    float d;
+};
+static __device__ __noinline__ RaceOutcome coded_race_exact(const uint8_t *base, CodedView rv, uint64_t seed,
+                                                            uint64_t run, uint32_t step) {
+    const Net n = net_view(base);
+    RaceOutcome r;
+    race_exact(n, n.n_comps, ceil_log2(n.n_comps), rv, seed, run, step, r.best, r.d);
+    return r;
+}
+
 // The race decided from the class keys (race_classes' decision over the
 // same keys); false: the caller runs race_exact.  src: each class's 1/rate
 // source (CSMC_CLASS_SRC_PROG | slot, or float bits).  ALLCLS: every
-// location is classed, so no component takes the descriptor path.
+// location is classed and the component count is a multiple of four, so no
+// block has a general member or padding.
 template <bool ALLCLS>
 static __device__ __forceinline__ bool race_coded(const Net &n, uint32_t C, uint32_t bits, uint32_t NG,
                                                   const CodedView &rv, const PhiloxKeys &K, const uint32_t *src,
                                                   uint64_t run, uint32_t step, unsigned long long &best,
                                                   float &bestd) {
     const uint32_t T = rv.T;
-    for (uint32_t w = 0; w < 4u * NG; ++w) rv.keys[w * T] = 0u;
+    for (uint32_t g = 0; g < NG; ++g)
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) st_key(rv.keys + g * kKeyClass + k * kKeyChain, 0u);
     best = ~0ull;
     bestd = 0.0f;
     const PhiloxStep ps = philox_step(K, step, run);
     // bit reversal of component 4q + k over `bits` (>= 2) bits: the two low
     // bits (k) become the top two, q the low bits - 2 reversed
     const uint32_t hi_shift = bits - 2u;  // bits >= 2: the plan needs at least four components
-    const uint32_t Qf = C >> 2;           // words whose four components all exist
+    const uint32_t Q = (C + 3u) >> 2;
 #pragma unroll kCodedUnroll
-    for (uint32_t q = 0; q < Qf; ++q) {
+    for (uint32_t q = 0; q < Q; ++q) {
+        const uint32_t wd = rv.lw[q * T];
         const u32x4 blk = philox_block(K, ps, q);
-        const uint32_t wd = rv.lw[q * T], cc = 4u * q;
-        const uint32_t rq = hi_shift ? (__brev(q) >> (32u - hi_shift)) : 0u;
-        const uint32_t cb = 255u - rq;
-        race_member<ALLCLS, 0>(n, bits, rv, wd, cc, blk.x, cb, best, bestd);
-        race_member<ALLCLS, 1>(n, bits, rv, wd, cc + 1u, blk.y, cb - (2u << hi_shift), best, bestd);
-        race_member<ALLCLS, 2>(n, bits, rv, wd, cc + 2u, blk.z, cb - (1u << hi_shift), best, bestd);
-        race_member<ALLCLS, 3>(n, bits, rv, wd, cc + 3u, blk.w, cb - (3u << hi_shift), best, bestd);
-    }
-    if (C & 3u) {  // the last, partly filled word
-        const u32x4 blk = philox_block(K, ps, Qf);
-        const uint32_t wd = rv.lw[Qf * T], cc = 4u * Qf, rem = C & 3u;
-        const uint32_t rq = hi_shift ? (__brev(Qf) >> (32u - hi_shift)) : 0u;
-        const uint32_t cb = 255u - rq;
-        race_member<ALLCLS, 0>(n, bits, rv, wd, cc, blk.x, cb, best, bestd);
-        if (rem > 1u) race_member<ALLCLS, 1>(n, bits, rv, wd, cc + 1u, blk.y, cb - (2u << hi_shift), best, bestd);
-        if (rem > 2u) race_member<ALLCLS, 2>(n, bits, rv, wd, cc + 2u, blk.z, cb - (1u << hi_shift), best, bestd);
+        const uint32_t cb = 255u - (hi_shift ? (__brev(q) >> (32u - hi_shift)) : 0u);
+        if (ALLCLS || !(wd & 0x80808080u)) {
+            race_block(rv, wd, blk, cb);
+        } else {
+            race_member<0>(n, rv, wd, 4u * q, blk.x, cb, hi_shift, best, bestd);
+            race_member<1>(n, rv, wd, 4u * q + 1u, blk.y, cb, hi_shift, best, bestd);
+            race_member<2>(n, rv, wd, 4u * q + 2u, blk.z, cb, hi_shift, best, bestd);
+            race_member<3>(n, rv, wd, 4u * q + 3u, blk.w, cb, hi_shift, best, bestd);
+        }
     }
     // each class races with its largest key
-    uint32_t inf_classes = 0, ties = 0;
-    uint32_t top[CSMC_RACE_CLASSES];
-    float dcls[CSMC_RACE_CLASSES], icls[CSMC_RACE_CLASSES];
+    uint32_t inf_classes = 0, wtop = 0;
+    float winv = 0.0f;
+    bool tie = false, from_class = false;
 #pragma unroll
     for (uint32_t g = 0; g < CSMC_RACE_CLASSES; ++g) {
-        top[g] = 0u;
-        dcls[g] = 0.0f;
-        icls[g] = 0.0f;
         if (g >= NG) continue;
-        const uint32_t *kg = rv.keys + (4u * g) * T;
-        const uint32_t a = max(max(kg[0], kg[T]), max(kg[2u * T], kg[3u * T]));
-        // key 0 (draw 0 at bit-reversed index 255) is also the "no member"
-        // value; only component 255 of a 256-component network can hold it
-        if (a == 0u && !(C == 256u && (rv.byte_of(255u) >> 5) == g)) continue;
+        const uint32_t kg = rv.keys + g * kKeyClass;
+        const uint32_t o0 = ld_key(kg), o1 = ld_key(kg + kKeyChain), o2 = ld_key(kg + 2u * kKeyChain),
+                       o3 = ld_key(kg + 3u * kKeyChain);
+        // no chain key is 0 (its low byte is 255 minus at most 63)
+        if ((o0 | o1 | o2 | o3) == 0u) continue;
+        const uint32_t a = max(max(o0, o1 ? o1 - (2u << hi_shift) : 0u),
+                               max(o2 ? o2 - (1u << hi_shift) : 0u, o3 ? o3 - (3u << hi_shift) : 0u));
         const uint32_t sg = src[g];
         const float inv = (sg & CSMC_CLASS_SRC_PROG) ? rv.rates[sg & 0xffffu] : __uint_as_float(sg);
         if (!(inv > 0.0f)) return false;  // delays 0, negative or NaN for the whole class
@@ -184,27 +243,25 @@ static __device__ __forceinline__ bool race_coded(const Net &n, uint32_t C, uint
             inf_classes |= 1u << g;
             continue;
         }
-        const uint32_t m1 = a >> 8, br1 = 255u - (a & 255u);
-        const float d1 = exp_delay(m1 << 8, inv);
-        top[g] = a;
-        dcls[g] = d1;
-        icls[g] = inv;
-        ties |= m1 > 0u ? (1u << g) : 0u;
-        const unsigned long long key = (static_cast<unsigned long long>(delay_key(d1)) << 32) | br1;
+        const float d1 = exp_delay(a & 0xffffff00u, inv);
+        const unsigned long long key =
+            (static_cast<unsigned long long>(f_bits(d1) | 0x80000000u) << 32) | (255u - (a & 255u));  // d1 >= 0
+        tie |= static_cast<uint32_t>(key >> 32) == static_cast<uint32_t>(best >> 32);
         if (key < best) {
+            tie = static_cast<uint32_t>(key >> 32) == static_cast<uint32_t>(best >> 32);
             best = key;
             bestd = d1;
+            wtop = a >> 8;
+            winv = inv;
+            from_class = true;
         }
     }
     // a class can hide a tie (a lower draw of a member with a smaller index
     // that rounds to the same delay) only when its delay is the race's
     // minimum and its largest draw sits on a flat spot of the delay; the
-    // exact race decides those steps
-#pragma unroll
-    for (uint32_t g = 0; g < CSMC_RACE_CLASSES; ++g) {
-        if (!((ties >> g) & 1u) || dcls[g] != bestd) continue;
-        if (exp_delay(((top[g] >> 8) - 1u) << 8, icls[g]) == dcls[g]) return false;
-    }
+    // exact race decides those steps, and those in which two delays tie
+    if (tie) return false;
+    if (from_class && wtop > 0u && exp_delay((wtop - 1u) << 8, winv) == bestd) return false;
     if (inf_classes && static_cast<uint32_t>(best >> 32) >= delay_key(__uint_as_float(0x7f800000u))) return false;
     return true;
 }
@@ -220,7 +277,7 @@ __global__ void __launch_bounds__(128, CSMC_CODED_MIN_CTAS_PER_SM) coded_kernel(
     const uint32_t C = p.net.n_comps, V = p.net.n_vars, P = p.net.n_rate_prog;
     const uint32_t T = blockDim.x, t = threadIdx.x;
     const bool recv = (p.net.recv_lo | p.net.recv_hi) != 0;
-    const CodedView rv = carve_coded_view(smem + p.blob_bytes, V, P, C, p.net.n_classes, recv, T, t);
+    const CodedView rv = carve_coded_view(smem + p.blob_bytes, V, P, C, p.net.n_classes * kKeyClass, recv, T, t);
     // padding bytes of the last location word never change
     if (C & 3u) rv.lw[(C >> 2) * T] = kCodePad * 0x20202020u;  // 0xc0 in every byte
     __syncthreads();
@@ -233,7 +290,7 @@ __global__ void __launch_bounds__(128, CSMC_CODED_MIN_CTAS_PER_SM) coded_kernel(
     const uint32_t lane = threadIdx.x & 31u;
     unsigned long long acc_hits = 0, acc_steps = 0, acc_capped = 0;
 
-    bool have = false;
+    bool have = false, drained = false;
     unsigned long long ridx = 0;
     uint64_t run = 0;
     float time = 0.0f;
@@ -242,27 +299,35 @@ __global__ void __launch_bounds__(128, CSMC_CODED_MIN_CTAS_PER_SM) coded_kernel(
     RunScalars sc{0.0, 0.0, 0, 0, -1, 0, 0};
 
     for (;;) {
+        // all lanes meet here, so that a warp's runs advance in one stream
+        // however their branches differed in the last step; the warp goes on
+        // until its last run has ended
+        __syncwarp();
         // ---- refill finished lanes from the work counter
-        const bool need = !have;
-        const unsigned act = __activemask();
-        const unsigned want = __ballot_sync(act, need);
+        const bool need = !have && !drained;
+        const unsigned want = __ballot_sync(0xffffffffu, need);
         if (want) {
             const int leader = __ffs(want) - 1;
             unsigned long long base = 0;
             if (static_cast<int>(lane) == leader)
                 base = atomicAdd(p.scratch, static_cast<unsigned long long>(__popc(want)));
-            base = __shfl_sync(act, base, leader);
+            base = __shfl_sync(0xffffffffu, base, leader);
             if (need) {
                 ridx = base + __popc(want & ((1u << lane) - 1u));
-                if (ridx >= p.n_runs) break;
-                have = true;
-                run = p.first_run + ridx;
-                run_init<SLOTS>(n, C, V, rv, sc, p.var_id);
-                time = 0.0f;
-                step = 0;
-                dirty = true;
+                if (ridx >= p.n_runs) {
+                    drained = true;
+                } else {
+                    have = true;
+                    run = p.first_run + ridx;
+                    run_init<SLOTS>(n, C, V, rv, sc, p.var_id);
+                    time = 0.0f;
+                    step = 0;
+                    dirty = true;
+                }
             }
+            if (__all_sync(0xffffffffu, drained)) break;
         }
+        if (!have) continue;
 
         // ---- end of run (simulation.cu:835-849, 887-893)
         const RunEnd e = run_end(sc, time, p.horizon, step, p.max_steps, p.loc_mode, p.is_max, p.threshold);
@@ -289,8 +354,11 @@ __global__ void __launch_bounds__(128, CSMC_CODED_MIN_CTAS_PER_SM) coded_kernel(
         }
         unsigned long long best;
         float bestd;
-        if (!race_coded<ALLCLS>(n, C, bits, NG, rv, p.keys, p.class_src, run, step, best, bestd))
-            race_exact(n, C, bits, rv, p.seed, run, step, best, bestd);
+        if (!race_coded<ALLCLS>(n, C, bits, NG, rv, p.keys, p.class_src, run, step, best, bestd)) {
+            const RaceOutcome r = coded_race_exact(n.base, rv, p.seed, run, step);
+            best = r.best;
+            bestd = r.d;
+        }
         const uint32_t win = bitrev_bits(static_cast<uint32_t>(best & 0xffffffffull), bits);
         if (run_commit<VERIFY, SLOTS>(n, p.net.n_clocks, rv, sc, p.seed, p.var_id, run, step, time, win, bestd))
             dirty = true;

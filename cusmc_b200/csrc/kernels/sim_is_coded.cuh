@@ -319,7 +319,7 @@ static __device__ __forceinline__ void is_member(const Net &n, const IsCodedView
     const uint32_t T = rv.T;
     if (ALLG || code < NG) {
         const uint32_t key = (x & 0xffffff00u) | cb;
-        uint32_t *pp = rv.keys + (code * 4u + k) * T;
+        uint32_t *pp = rv.kp + (code * 4u + k) * T;
         *pp = max(*pp, key);
         if ((tilt_mask >> code) & 1u) part = d_add(part, gr.diff(code));
     } else if (code == kCodeGeneral) {
@@ -394,7 +394,7 @@ static __device__ __forceinline__ bool is_race_coded(const Net &n, uint32_t C, u
                                                      const float (&mfac)[CSMC_MLP_CLASSES], const PhiloxKeys &K,
                                                      uint64_t run, uint32_t step, IsBest &best, double &sum) {
     const uint32_t T = rv.T;
-    for (uint32_t w = 0; w < 4u * NG; ++w) rv.keys[w * T] = 0u;
+    for (uint32_t w = 0; w < 4u * NG; ++w) rv.kp[w * T] = 0u;
     best.key = ~0ull;
     best.d = best.inv = best.invp = 0.0f;
     best.tilted = false;
@@ -427,7 +427,7 @@ static __device__ __forceinline__ bool is_race_coded(const Net &n, uint32_t C, u
         top[g] = 0u;
         dg[g] = 0.0f;
         if (g >= NG) continue;
-        const uint32_t *kg = rv.keys + (4u * g) * T;
+        const uint32_t *kg = rv.kp + (4u * g) * T;
         const uint32_t a = max(max(kg[0], kg[T]), max(kg[2u * T], kg[3u * T]));
         // key 0 (draw 0 at bit-reversed index 255) is also the "no member"
         // value; only component 255 of a 256-component network can hold it
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
     const GroupRates gr{reinterpret_cast<uint32_t *>(slab) + t, T};
     const bool recv = (p.net.recv_lo | p.net.recv_hi) != 0;
     IsCodedView rv;
-    static_cast<CodedView &>(rv) = carve_coded_view(slab + 16u * NG * T, V, P, C, NG, recv, T, t);
+    static_cast<CodedView &>(rv) = carve_coded_view(slab + 16u * NG * T, V, P, C, 16u * NG * T, recv, T, t);
     rv.map = ip.group_map;
     if (C & 3u) rv.lw[(C >> 2) * T] = kCodePad * 0x20202020u;  // padding bytes never change
     __syncthreads();
