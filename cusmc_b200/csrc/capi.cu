@@ -65,7 +65,8 @@ int max_smem_optin(int device) {
 }
 
 // Fills the launch geometry of a plan; returns false when it cannot run.
-bool configure_plan(csmc_net *n, int family, int lanes, int cpl, int block, std::string &why) {
+bool configure_plan(const csmc_net *n, csmc_launch_plan &p, int family, int lanes, int cpl, int block,
+                    std::string &why) {
     const csmc_net_header &h = n->h;
     const size_t max_smem = static_cast<size_t>(max_smem_optin(n->device));
     if (family == 0) {
@@ -86,13 +87,13 @@ bool configure_plan(csmc_net *n, int family, int lanes, int cpl, int block, std:
             why = "network and run state do not fit in shared memory";
             return false;
         }
-        n->family = 0;
-        n->lanes = lanes;
-        n->comps_per_lane = cpl;
-        n->block = block;
-        n->state_stride = stride;
-        n->smem = smem;
-        n->state_in_global = false;
+        p.family = 0;
+        p.lanes = lanes;
+        p.comps_per_lane = cpl;
+        p.block = block;
+        p.state_stride = stride;
+        p.smem = smem;
+        p.state_in_global = false;
         return true;
     }
     if (block <= 0 || block % 32 || block > 128) {
@@ -112,13 +113,13 @@ bool configure_plan(csmc_net *n, int family, int lanes, int cpl, int block, std:
             why = "network and run state do not fit in shared memory";
             return false;
         }
-        n->family = 4;
-        n->lanes = 1;
-        n->comps_per_lane = static_cast<int>(h.n_comps);
-        n->block = block;
-        n->state_stride = static_cast<uint32_t>(slab);
-        n->state_in_global = false;
-        n->smem = n->bytes + slab;
+        p.family = 4;
+        p.lanes = 1;
+        p.comps_per_lane = static_cast<int>(h.n_comps);
+        p.block = block;
+        p.state_stride = static_cast<uint32_t>(slab);
+        p.state_in_global = false;
+        p.smem = n->bytes + slab;
         return true;
     }
     if (family == 2) {  // network and run state in global memory
@@ -127,13 +128,13 @@ bool configure_plan(csmc_net *n, int family, int lanes, int cpl, int block, std:
             return false;
         }
         const size_t per = csmc::batch_state_bytes_per_thread(h.n_comps, h.n_vars, h.n_rate_prog);
-        n->family = 2;
-        n->lanes = 1;
-        n->comps_per_lane = static_cast<int>(h.n_comps);
-        n->block = block;
-        n->state_stride = static_cast<uint32_t>((per * block + 15) & ~static_cast<size_t>(15));
-        n->state_in_global = true;
-        n->smem = csmc::batch_smem_bytes(1);
+        p.family = 2;
+        p.lanes = 1;
+        p.comps_per_lane = static_cast<int>(h.n_comps);
+        p.block = block;
+        p.state_stride = static_cast<uint32_t>((per * block + 15) & ~static_cast<size_t>(15));
+        p.state_in_global = true;
+        p.smem = csmc::batch_smem_bytes(1);
         return true;
     }
     if (family != 1) {
@@ -146,19 +147,124 @@ bool configure_plan(csmc_net *n, int family, int lanes, int cpl, int block, std:
     }
     const size_t per_thread = csmc::serial_state_bytes_per_thread(h.n_comps, h.n_vars, h.n_rate_prog, n->slots, n->loc8);
     const size_t slab = (per_thread * block + 15) & ~static_cast<size_t>(15);
-    n->family = 1;
-    n->lanes = 1;
-    n->comps_per_lane = static_cast<int>(h.n_comps);
-    n->block = block;
-    n->state_stride = static_cast<uint32_t>(slab);
+    p.family = 1;
+    p.lanes = 1;
+    p.comps_per_lane = static_cast<int>(h.n_comps);
+    p.block = block;
+    p.state_stride = static_cast<uint32_t>(slab);
     if (n->bytes + slab <= max_smem) {
-        n->state_in_global = false;
-        n->smem = n->bytes + slab;
+        p.state_in_global = false;
+        p.smem = n->bytes + slab;
     } else {
-        n->state_in_global = true;
-        n->smem = n->bytes;
+        p.state_in_global = true;
+        p.smem = n->bytes;
     }
     return true;
+}
+
+// ---- lane-group shapes and the choice by launch size ------------------------
+
+// The shapes (lanes per run, components per lane) a network can run with,
+// widest first: every power of two from one component per lane down to four
+// components per lane, then the lane's share doubled to 16.
+void find_shapes(csmc_net *n) {
+    const csmc_net_header &h = n->h;
+    const size_t cta_smem = static_cast<size_t>(max_smem_optin(n->device));
+    int sm_smem = 0;
+    cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, n->device);
+    n->n_shapes = 0;
+    int G = 0, K = 0;
+    choose_shape(h.n_comps, G, K);
+    for (; G >= 2 && K <= 16 && n->n_shapes < 6;) {
+        if (csmc::sim_supported(G, K)) {
+            csmc_group_shape s;
+            s.lanes = G;
+            s.comps_per_lane = K;
+            s.stride = csmc::group_state_stride(h.n_vars, h.n_rate_prog, G, K);
+            // 16 warps per SM (128 registers a thread) in the largest CTA that
+            // fits: its warps share one copy of the network
+            for (int block : {512, 256, 128, 64, 32}) {
+                const size_t smem = n->bytes + static_cast<size_t>(block / G) * s.stride;
+                if (smem > cta_smem) continue;
+                const int ctas = std::min(512 / block, static_cast<int>(static_cast<size_t>(sm_smem) / (smem + 1024)));
+                const int warps = ctas * (block / 32);
+                if (warps > s.warps) {
+                    s.warps = warps;
+                    s.block = block;
+                }
+            }
+            if (s.warps > 0) n->shapes[n->n_shapes++] = s;
+        }
+        if (h.n_comps <= 4) break;
+        if (K < 4) {  // one Philox block per lane: the lanes of K = 1, 2 draw it and use a part
+            G = static_cast<int>(std::max(2u, csmc::ceil_pow2((h.n_comps + 3) / 4)));
+            K = 4;
+            if (n->n_shapes && n->shapes[n->n_shapes - 1].lanes <= G) G /= 2, K *= 2;
+        } else {
+            G /= 2;
+            K *= 2;
+        }
+    }
+}
+
+// The plan of a launch of n_runs runs.  A run's steps are a serial chain, so
+// a launch that does not fill the GPU takes its longest run's steps times
+// the latency of a step, which falls with the lanes a run has; one that
+// fills it takes the issue slots of all steps, which are fewest with many
+// runs per warp.  In units of one component of a lane, a warp's step has the
+// latency 4.4 L and takes I issue slots:
+//   groups:     L = 3 + K + 0.1 (32 / G - 1), I = 2 + K + 0.45 (32 / G - 1)
+//               (the groups of a warp branch apart)
+//   one thread: L = 12 + 0.22 C (every location classed), 4 + 1.1 C (classes
+//               and descriptors) or 1 + 1.85 C (no classes), latency 5 L (a
+//               warp waits for the longest of 32 runs), I = 1.2 L (1 L)
+// and a launch takes max(latency, (waves + 1) I), a wave being one warp per
+// scheduler; I is scaled by 13.2 (10) / (resident warps per SM) where those
+// are too few to hide the latency.  Fitted to the epidemic (12 to 200
+// agents), the mutex (8 to 256) and random networks (4 to 64 components) at
+// 100 to 131,072 runs on B200.  One thread per run / the best group: 100
+// agents 100 runs 14.3 / 3.0 ms, 16,384 runs 16.2 / 13.8, 32,768 runs 19.6 /
+// 23.5; mutex 32, 100 runs 28.4 / 2.9, 32,768 runs 30.8 / 20.4, 65,536 runs
+// 39.7 / 39.6; random 8, 100 runs 2.2 / 0.7, 131,072 runs 6.3 / 6.0; random
+// 24, 65,536 runs 19.7 / 24.0; random 64, 131,072 runs 288 / 90.
+csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
+    if (n->plan_forced || n->plan.family == 2 || n->n_shapes == 0) return n->plan;
+    const double C = n->h.n_comps, unit = 128.0 * n->sms, runs = static_cast<double>(n_runs);
+    double best = 0.0;
+    const csmc_group_shape *pick = nullptr;
+    for (int i = 0; i < n->n_shapes; ++i) {
+        const csmc_group_shape &s = n->shapes[i];
+        const double K = s.comps_per_lane, apart = 32.0 / s.lanes - 1.0;
+        const double I = (2.0 + K + 0.45 * apart) * std::max(1.0, 13.2 / s.warps);
+        const double t = std::max(4.4 * (3.0 + K + 0.1 * apart), (runs * s.lanes / unit + 1.0) * I);
+        if (!pick || t < best) {
+            best = t;
+            pick = &s;
+        }
+    }
+    if (n->thread_warps > 0) {
+        const bool classes = n->plan.family == 4;
+        const double L = classes ? (n->only_classes ? 12.0 + 0.22 * C : 4.0 + 1.1 * C) : 1.0 + 1.85 * C;
+        const double I = (classes ? 1.2 : 1.0) * L * std::max(1.0, 10.0 / n->thread_warps);
+        const double t = std::max(5.0 * L, (runs / unit + 1.0) * I);
+        // (where both fill the GPU a group is taken only when it is clearly the better one)
+        if (t < best * (runs > 1.75 * unit ? 1.25 : 1.0)) return n->plan;
+    }
+    csmc_launch_plan p;
+    p.family = 0;
+    p.lanes = pick->lanes;
+    p.comps_per_lane = pick->comps_per_lane;
+    p.state_stride = pick->stride;
+    // a launch of few warps: CTAs of one to four warps, to spread them over the SMs
+    p.block = pick->block;
+    const uint64_t warps = (n_runs * pick->lanes + 31) / 32;
+    for (int block : {32, 64, 128})
+        if (block < p.block && warps * 32 <= static_cast<uint64_t>(block) * n->sms) {
+            p.block = block;
+            break;
+        }
+    p.smem = n->bytes + static_cast<size_t>(p.block / p.lanes) * p.state_stride;
+    return p;
 }
 
 const csmc_net_header *header_of(const void *blob, size_t bytes) {
@@ -196,12 +302,13 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
         return fail(CSMC_ERR_ARG, "query variable id " + std::to_string(q->var_id) + " out of range");
     if (first_run + n_runs < first_run || first_run + n_runs > (1ull << 62))
         return fail(CSMC_ERR_ARG, "run range out of bounds");
+    const csmc_launch_plan pl = launch_plan(n, n_runs);
     std::memset(out, 0, sizeof *out);
     out->runs = n_runs;
-    out->lanes_per_run = n->lanes;
-    out->comps_per_lane = n->comps_per_lane;
-    out->runs_per_cta = n->block / n->lanes;
-    out->family = n->family;
+    out->lanes_per_run = pl.lanes;
+    out->comps_per_lane = pl.comps_per_lane;
+    out->runs_per_cta = pl.block / pl.lanes;
+    out->family = pl.family;
     if (n_runs == 0) return CSMC_OK;
     CK(cudaSetDevice(n->device), "cudaSetDevice");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -216,7 +323,7 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
     p.net = csmc::layout_of(n->h);
     p.blob = n->d_blob;
     p.blob_bytes = n->bytes;
-    p.state_stride = n->state_stride;
+    p.state_stride = pl.state_stride;
     p.loc_mode = q->kind == CSMC_QUERY_LOCATION;
     p.var_id = q->var_id;
     p.is_max = q->is_max;
@@ -235,23 +342,20 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
     int ctas = 0;
     p.keys = csmc::philox_keys(seed);
     for (int g = 0; g < CSMC_RACE_CLASSES; ++g) p.class_src[g] = n->class_src[g];
-    int rc = n->family == 0 ? csmc::sim_max_active_ctas(n->lanes, n->comps_per_lane, verify, n->block, n->smem, &ctas)
-             : n->family == 2 ? csmc::batch_max_active_ctas(verify, 0, n->block, n->smem, &ctas)
-             : n->family == 4 ? csmc::coded_max_active_ctas(verify, n->slots, n->all_classed, n->block, n->smem, &ctas)
-                              : csmc::serial_max_active_ctas(verify, n->slots, n->loc8, n->state_in_global, n->classes,
-                                                             n->block, n->smem, &ctas);
+    int rc = pl.family == 0 ? csmc::sim_max_active_ctas(pl.lanes, pl.comps_per_lane, verify, pl.block, pl.smem, &ctas)
+             : pl.family == 2 ? csmc::batch_max_active_ctas(verify, 0, pl.block, pl.smem, &ctas)
+             : pl.family == 4 ? csmc::coded_max_active_ctas(verify, n->slots, n->all_classed, pl.block, pl.smem, &ctas)
+                              : csmc::serial_max_active_ctas(verify, n->slots, n->loc8, pl.state_in_global, n->classes,
+                                                             pl.block, pl.smem, &ctas);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "occupancy query");
     if (ctas < 1) return fail(CSMC_ERR_LIMIT, "kernel cannot be resident with this network (shared memory)");
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device), "cudaDeviceGetAttribute");
-    const uint64_t runs_per_cta = static_cast<uint64_t>(n->block / n->lanes);
-    uint64_t grid = static_cast<uint64_t>(sms) * static_cast<uint64_t>(ctas);
+    const uint64_t runs_per_cta = static_cast<uint64_t>(pl.block / pl.lanes);
+    uint64_t grid = static_cast<uint64_t>(n->sms) * static_cast<uint64_t>(ctas);
     const uint64_t needed = (n_runs + runs_per_cta - 1) / runs_per_cta;
     if (grid > needed) grid = needed;
-    n->grid = static_cast<int>(grid);
     p.state_global = nullptr;
-    if ((n->family == 1 || n->family == 2) && n->state_in_global) {
-        const size_t need = grid * static_cast<size_t>(n->state_stride);
+    if ((pl.family == 1 || pl.family == 2) && pl.state_in_global) {
+        const size_t need = grid * static_cast<size_t>(pl.state_stride);
         if (need > n->state_bytes) {
             cudaFree(n->d_state);
             n->d_state = nullptr;
@@ -261,9 +365,9 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
         }
         p.state_global = n->d_state;
     }
-    p.state_stride = n->state_stride;
+    p.state_stride = pl.state_stride;
     csmc::BatchParams bp{};
-    if (n->family == 2) {  // the batch kernel with a one-job table
+    if (pl.family == 2) {  // the batch kernel with a one-job table
         if (!n->d_job) CK(cudaMalloc(&n->d_job, sizeof(csmc::BatchJob)), "cudaMalloc(job table)");
         csmc::BatchJob job{};
         job.net = p.net;
@@ -287,7 +391,7 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
         CK(cudaMemcpyAsync(n->d_job, &job, sizeof job, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(job table)");
         bp.jobs = n->d_job;
         bp.n_jobs = 1;
-        bp.state_stride = n->state_stride;
+        bp.state_stride = pl.state_stride;
         bp.total_runs = n_runs;
         bp.queue = n->d_scratch;
         bp.state = n->d_state;
@@ -296,13 +400,13 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
         bp.max_comps = n->h.n_comps;
     }
     CK(cudaEventRecord(n->ev0, st), "cudaEventRecord");
-    rc = n->family == 0   ? csmc::sim_launch(n->lanes, n->comps_per_lane, verify, p, static_cast<int>(grid), n->block,
-                                             n->smem, st)
-         : n->family == 2 ? csmc::batch_launch(verify, bp, static_cast<int>(grid), n->block, st)
-         : n->family == 4 ? csmc::coded_launch(verify, n->slots, n->all_classed, p, static_cast<int>(grid), n->block,
-                                               n->smem, st)
-                          : csmc::serial_launch(verify, n->slots, n->loc8, n->state_in_global, n->classes, p,
-                                                static_cast<int>(grid), n->block, n->smem, st);
+    rc = pl.family == 0   ? csmc::sim_launch(pl.lanes, pl.comps_per_lane, verify, p, static_cast<int>(grid), pl.block,
+                                             pl.smem, st)
+         : pl.family == 2 ? csmc::batch_launch(verify, bp, static_cast<int>(grid), pl.block, st)
+         : pl.family == 4 ? csmc::coded_launch(verify, n->slots, n->all_classed, p, static_cast<int>(grid), pl.block,
+                                               pl.smem, st)
+                          : csmc::serial_launch(verify, n->slots, n->loc8, pl.state_in_global, n->classes, p,
+                                                static_cast<int>(grid), pl.block, pl.smem, st);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "simulation kernel launch");
     CK(cudaEventRecord(n->ev1, st), "cudaEventRecord");
     if (need_values) reduce_values<<<kReduceBlocks, 256, 0, st>>>(values, n_runs, n->d_partials);
@@ -471,6 +575,7 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
             }
             n->class_src[g] = (fl & CSMC_DESC_PROG) ? (CSMC_CLASS_SRC_PROG | lo) : lo;
         }
+        n->only_classes = n->all_classed;
         n->all_classed = n->all_classed && h->n_comps % 4 == 0;
         // tilt groups of importance sampling one thread per run: the
         // (race class, location class) pairs in order of first appearance,
@@ -517,12 +622,22 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
     choose_shape(h->n_comps, G, K);
     const size_t per_thread = csmc::serial_state_bytes_per_thread(h->n_comps, h->n_vars, h->n_rate_prog, n->slots, n->loc8);
     const bool serial_fits = n->bytes + 128 * per_thread <= static_cast<size_t>(max_smem_optin(n->device));
-    bool ok = configure_plan(n.get(), 4, 1, static_cast<int>(h->n_comps), 128, why);
-    if (!ok && serial_fits) ok = configure_plan(n.get(), 1, 1, static_cast<int>(h->n_comps), 128, why);
-    if (!ok) ok = configure_plan(n.get(), 0, G, K, 256, why);
-    if (!ok) ok = configure_plan(n.get(), 1, 1, static_cast<int>(h->n_comps), 128, why);
-    if (!ok) ok = configure_plan(n.get(), 2, 1, static_cast<int>(h->n_comps), 128, why);
+    csmc_launch_plan &pl = n->plan;
+    bool ok = configure_plan(n.get(), pl, 4, 1, static_cast<int>(h->n_comps), 128, why);
+    if (!ok && serial_fits) ok = configure_plan(n.get(), pl, 1, 1, static_cast<int>(h->n_comps), 128, why);
+    if (!ok) ok = configure_plan(n.get(), pl, 0, G, K, 256, why);
+    if (!ok) ok = configure_plan(n.get(), pl, 1, 1, static_cast<int>(h->n_comps), 128, why);
+    if (!ok) ok = configure_plan(n.get(), pl, 2, 1, static_cast<int>(h->n_comps), 128, why);
     if (!ok) return fail(CSMC_ERR_LIMIT, "no launch plan for this network: " + why);
+    CK(cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, n->device), "cudaDeviceGetAttribute");
+    find_shapes(n.get());
+    if ((pl.family == 1 && !pl.state_in_global) || pl.family == 4) {
+        int sm_smem = 0;
+        CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, n->device),
+           "cudaDeviceGetAttribute");
+        n->thread_warps = 4 * std::max(1, std::min(4, static_cast<int>(sm_smem / (pl.smem + 1024))));
+    }
+    if (pl.state_in_global) n->n_shapes = 0;
     CK(cudaMalloc(&n->d_blob, n->bytes), "cudaMalloc(network)");
     CK(cudaMemset(n->d_blob, 0, n->bytes), "cudaMemset");
     CK(cudaMemcpy(n->d_blob, blob, h->total_bytes, cudaMemcpyHostToDevice), "cudaMemcpy(network)");
@@ -555,26 +670,20 @@ void csmc_net_free(csmc_net *n) {
 int csmc_set_plan(csmc_net *n, int32_t family, int32_t lanes_per_run, int32_t comps_per_lane,
                   int32_t threads_per_cta) {
     if (!n) return fail(CSMC_ERR_ARG, "null argument");
-    const csmc_net saved = *n;
     std::string why;
-    if (!configure_plan(n, family, lanes_per_run, comps_per_lane, threads_per_cta, why)) {
-        n->family = saved.family;
-        n->lanes = saved.lanes;
-        n->comps_per_lane = saved.comps_per_lane;
-        n->block = saved.block;
-        n->smem = saved.smem;
-        n->state_stride = saved.state_stride;
-        n->state_in_global = saved.state_in_global;
+    csmc_launch_plan p;
+    if (!configure_plan(n, p, family, lanes_per_run, comps_per_lane, threads_per_cta, why))
         return fail(CSMC_ERR_ARG, "plan rejected: " + why);
-    }
+    n->plan = p;
+    n->plan_forced = true;
     return CSMC_OK;
 }
 
 int csmc_plan(const csmc_net *n, int32_t *lanes, int32_t *cpl, int32_t *rpc) {
     if (!n) return fail(CSMC_ERR_ARG, "null argument");
-    if (lanes) *lanes = n->lanes;
-    if (cpl) *cpl = n->comps_per_lane;
-    if (rpc) *rpc = n->block / n->lanes;
+    if (lanes) *lanes = n->plan.lanes;
+    if (cpl) *cpl = n->plan.comps_per_lane;
+    if (rpc) *rpc = n->plan.block / n->plan.lanes;
     return CSMC_OK;
 }
 

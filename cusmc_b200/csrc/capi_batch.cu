@@ -574,7 +574,8 @@ void csmc_batch_free(csmc_batch *b) {
 int csmc_autotune(csmc_net *n, const csmc_query *q, uint64_t seed, uint64_t probe_runs, csmc_result *best) {
     if (!n || !q || !best) return fail(CSMC_ERR_ARG, "null argument");
     if (probe_runs == 0) return fail(CSMC_ERR_ARG, "probe_runs must be positive");
-    int32_t saved[4] = {n->family, n->lanes, n->comps_per_lane, n->block};
+    const csmc_launch_plan saved = n->plan;
+    const bool saved_forced = n->plan_forced;
     struct Cand {
         int family, lanes, cpl, block;
     };
@@ -594,7 +595,7 @@ int csmc_autotune(csmc_net *n, const csmc_query *q, uint64_t seed, uint64_t prob
     for (int block : {64, 128}) cands.push_back({2, 1, C, block});
     csmc_result r{}, top{};
     bool have = false;
-    int32_t pick[4] = {saved[0], saved[1], saved[2], saved[3]};
+    int32_t pick[4] = {saved.family, saved.lanes, saved.comps_per_lane, saved.block};
     for (const Cand &c : cands) {
         if (csmc_set_plan(n, c.family, c.lanes, c.cpl, c.block) != CSMC_OK) continue;
         if (csmc_run(n, q, seed, 0, probe_runs, nullptr, nullptr, nullptr, &r, nullptr) != CSMC_OK) continue;
@@ -608,7 +609,8 @@ int csmc_autotune(csmc_net *n, const csmc_query *q, uint64_t seed, uint64_t prob
         }
     }
     if (!have) {
-        csmc_set_plan(n, saved[0], saved[1], saved[2], saved[3]);
+        n->plan = saved;
+        n->plan_forced = saved_forced;
         return fail(CSMC_ERR_LIMIT, "no plan could run this network");
     }
     int rc = csmc_set_plan(n, pick[0], pick[1], pick[2], pick[3]);

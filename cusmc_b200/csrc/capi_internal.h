@@ -9,6 +9,23 @@
 
 #include <string>
 
+// The geometry of one launch of the simulation kernels.
+struct csmc_launch_plan {
+    int family = 1;  // 0 = lane groups (lanes, comps_per_lane), 1 = one thread per run, 2 = one thread per run with
+                     // the network read from global memory (the batch kernel with one job), 4 = class-coded
+    int lanes = 0, comps_per_lane = 0, block = 256;
+    size_t smem = 0;
+    uint32_t state_stride = 0;
+    bool state_in_global = false;
+};
+
+// A lane-group shape that fits the network, as launches choose among them.
+struct csmc_group_shape {
+    int lanes = 0, comps_per_lane = 0, block = 0;  // block: threads per CTA of a launch that fills the GPU
+    uint32_t stride = 0;                           // shared memory of one group's run state
+    int warps = 0;                                 // resident warps per SM at that block
+};
+
 struct csmc_net {
     int device = 0;
     uint8_t *d_blob = nullptr;
@@ -21,19 +38,18 @@ struct csmc_net {
     uint64_t cap_runs = 0;
     double *d_partials = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // launch plan: family 0 = lane groups (lanes, comps_per_lane), 1 = one
-    // thread per run, 2 = one thread per run with the network read from
-    // global memory (the batch kernel with one job)
-    int family = 1;
-    int lanes = 0, comps_per_lane = 0, block = 256, grid = 0;
-    size_t smem = 0;
-    uint32_t state_stride = 0;
+    csmc_launch_plan plan;     // the plan set by csmc_set_plan, else the default of launches that fill the GPU
+    bool plan_forced = false;  // csmc_set_plan: every launch uses `plan`
+    csmc_group_shape shapes[6];  // lane-group shapes for launches that do not fill the GPU one thread per run
+    int n_shapes = 0;
+    int sms = 0;               // SMs of the device
+    int thread_warps = 0;      // resident warps per SM of the default plan when it runs one thread per run (0: it does not)
     bool slots = false;
     bool loc8 = false;     // every automaton has at most 256 locations
     bool classes = false;  // delay descriptors carry race classes
+    bool only_classes = false; // every location belongs to a race class
     bool all_classed = false;  // every location belongs to a race class, components a multiple of four
     uint32_t class_src[CSMC_RACE_CLASSES] = {};  // 1/rate source of each class (SimParams::class_src)
-    bool state_in_global = false;
     uint8_t *d_state = nullptr;  // thread-per-run state slabs (global-state plans)
     size_t state_bytes = 0;
     csmc::BatchJob *d_job = nullptr;  // family 2: the one-job table

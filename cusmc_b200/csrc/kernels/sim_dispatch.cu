@@ -64,7 +64,9 @@ int serial_max_active_ctas(bool verify, bool slots, bool loc8, bool gstate, bool
                  : serial_occ_l<false, false>(loc8, gstate, classes, block, smem, ctas);
 }
 
-#define CSMC_SHAPES(X) X(1, 1) X(2, 1) X(4, 1) X(8, 1) X(16, 1) X(32, 1) X(32, 2) X(32, 4) X(32, 8) X(32, 16) X(32, 32)
+#define CSMC_SHAPES(X) \
+    X(1, 1) X(2, 1) X(4, 1) X(8, 1) X(16, 1) X(32, 1) X(32, 2) X(32, 4) X(32, 8) X(32, 16) X(32, 32) \
+    X(2, 4) X(4, 4) X(8, 4) X(16, 4) X(4, 8) X(8, 8) X(16, 8) X(8, 16) X(16, 16)
 
 bool sim_supported(int g, int k) {
 #define X(GG, KK) \

@@ -454,12 +454,9 @@ struct GroupRun {
     }
 };
 
-#ifndef CSMC_MIN_CTAS_PER_SM
-#define CSMC_MIN_CTAS_PER_SM 2
-#endif
-
+// At most 512 threads per CTA, 128 registers a thread (16 warps per SM).
 template <int G, int K, bool VERIFY>
-__global__ void __launch_bounds__(256, CSMC_MIN_CTAS_PER_SM) sim_kernel(const __grid_constant__ SimParams p) {
+__global__ void __launch_bounds__(512, 1) sim_kernel(const __grid_constant__ SimParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     stage_network(smem, p.blob, p.blob_bytes);
     __syncthreads();
