@@ -559,6 +559,15 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
     n->classes = (h->flags & CSMC_NET_RACE_CLASSES) != 0 && h->n_comps <= 256;
     if (n->classes && h->off_loc_desc + 8ull * h->n_locs > h->total_bytes)
         return fail(CSMC_ERR_ARG, "not a network blob (descriptor table out of range)");
+    if (h->off_loc_desc && h->off_loc_desc + 8ull * h->n_locs <= h->total_bytes && h->n_locs <= 0xffffu) {
+        n->is_plain = true;
+        for (uint32_t i = 0; i < h->n_locs; ++i) {
+            uint64_t d;
+            std::memcpy(&d, static_cast<const uint8_t *>(blob) + h->off_loc_desc + 8ull * i, 8);
+            const uint32_t fl = static_cast<uint32_t>(d >> 32);
+            if (!(fl & CSMC_DESC_ZERO) && (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL))) n->is_plain = false;
+        }
+    }
     if (n->classes) {
         // each class's 1/rate source, and whether every location is classed
         // (the class-coded kernel's launch parameters)

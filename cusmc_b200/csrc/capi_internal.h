@@ -54,6 +54,7 @@ struct csmc_net {
     size_t state_bytes = 0;
     csmc::BatchJob *d_job = nullptr;  // family 2: the one-job table
     // importance sampling
+    bool is_plain = false;  // every location is exponential (a literal or a rate program) or zero-delay
     csmc::MlpParams *d_mlp = nullptr;  // the proposal network
     double *d_wvals = nullptr;         // per run: flag * likelihood ratio
     uint8_t *d_is_flags = nullptr;

@@ -60,6 +60,7 @@ struct Launch {
     size_t smem = 0;
     uint32_t slab = 0;  // shared-memory bytes per warp (one run)
     bool slots = false, loc8 = false;
+    bool plain = false;  // the kernel of networks without invariants
 };
 
 // One run per warp: the network and the proposal network once per CTA, then
@@ -69,19 +70,26 @@ int plan_is(const csmc_net *n, bool trace, uint64_t n_runs, Launch &L) {
     L.slots = h.max_edges_per_loc >= 2;
     L.loc8 = h.max_locs_per_comp <= 256;
     const size_t per = csmc::serial_state_bytes_per_thread(h.n_comps, h.n_vars, h.n_rate_prog, L.slots, L.loc8);
-    L.slab = static_cast<uint32_t>(csmc::is_warp_slab_bytes(per, n->is_tc));
+    const bool recv = (h.recv_chan_lo | h.recv_chan_hi) != 0;
+    L.plain = n->is_plain;
+    L.slab = static_cast<uint32_t>(L.plain ? csmc::is_plain_slab_bytes(h.n_comps, h.n_vars, h.n_rate_prog, recv, n->is_tc)
+                                           : csmc::is_warp_slab_bytes(per, n->is_tc));
     const size_t base = n->bytes + csmc::is_mlp_smem_bytes();
     int max_smem = 0, sms = 0, ctas = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, n->device), "device attribute");
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device), "device attribute");
     int warps = CSMC_IS_BLOCK / 32;
+    // few runs: CTAs of fewer warps, spread over the SMs (a run's steps are a
+    // serial chain: it gains from a scheduler of its own)
+    while (warps > 1 && n_runs <= static_cast<uint64_t>(warps / 2) * sms) warps /= 2;
     while (warps > 1 && base + static_cast<size_t>(warps) * L.slab > static_cast<size_t>(max_smem)) warps /= 2;
     L.block = 32 * warps;
     L.smem = base + static_cast<size_t>(warps) * L.slab;
     if (L.smem > static_cast<size_t>(max_smem))
         return fail(CSMC_ERR_LIMIT, "importance sampling needs the network, the proposal network and one run's "
                                     "state in shared memory (" + std::to_string(L.smem) + " bytes)");
-    int rc = csmc::is_max_active_ctas(n->is_tc, trace, L.slots, L.loc8, L.block, L.smem, &ctas);
+    int rc = L.plain ? csmc::is_plain_max_active_ctas(n->is_tc, trace, L.block, L.smem, &ctas)
+                     : csmc::is_max_active_ctas(n->is_tc, trace, L.slots, L.loc8, L.block, L.smem, &ctas);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "occupancy query");
     if (ctas < 1) return fail(CSMC_ERR_LIMIT, "importance-sampling kernel cannot be resident");
     uint64_t grid = static_cast<uint64_t>(sms) * ctas;
@@ -305,7 +313,8 @@ int csmc_is_run(csmc_net *n, const csmc_query *q, const void *params, uint64_t s
     }
     CK(cudaEventRecord(n->ev0, st), "cudaEventRecord");
     rc = coded ? csmc::is_coded_launch(L.slots, n->is_all_grouped, ip, L.grid, L.block, L.smem, st)
-               : csmc::is_launch(n->is_tc, false, L.slots, L.loc8, ip, L.grid, L.block, L.smem, st);
+         : L.plain ? csmc::is_plain_launch(n->is_tc, false, ip, L.grid, L.block, L.smem, st)
+                   : csmc::is_launch(n->is_tc, false, L.slots, L.loc8, ip, L.grid, L.block, L.smem, st);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "importance-sampling kernel launch");
     CK(cudaEventRecord(n->ev1, st), "cudaEventRecord");
     reduce_weights<<<csmc::kReduceBlocks, 256, 0, st>>>(n->d_wvals, n_runs, n->d_partials);
@@ -352,7 +361,8 @@ int csmc_is_trace(csmc_net *n, const csmc_query *q, const void *params, uint64_t
     ip.row_offset = row_offset;
     ip.rows = static_cast<csmc::MlpRow *>(rows);
     ip.rows_cap = rows_cap;
-    rc = csmc::is_launch(n->is_tc, true, L.slots, L.loc8, ip, L.grid, L.block, L.smem, st);
+    rc = L.plain ? csmc::is_plain_launch(n->is_tc, true, ip, L.grid, L.block, L.smem, st)
+                 : csmc::is_launch(n->is_tc, true, L.slots, L.loc8, ip, L.grid, L.block, L.smem, st);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "replay kernel launch");
     unsigned long long sc[CSMC_SCRATCH_WORDS];
     CK(cudaMemcpyAsync(sc, n->d_scratch, sizeof sc, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");

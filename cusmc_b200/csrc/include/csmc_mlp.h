@@ -96,8 +96,8 @@ CSMC_HD float exp2_f(float t) {
     return f_mul(p, bits_f(static_cast<uint32_t>(e + 127) << 23));
 }
 
-/* sigmoid(s) = 1 / (1 + 2^(-s log2 e)) */
-CSMC_HD float sigmoid_f(float s) { return f_div(1.0f, f_add(1.0f, exp2_f(f_mul(s, -1.44269502f)))); }
+/* sigmoid(s) = 1 / (1 + 2^(-s log2 e)); the exponential is at most 2^126 */
+CSMC_HD float sigmoid_f(float s) { return rcp_from_one(f_add(1.0f, exp2_f(f_mul(s, -1.44269502f)))); }
 
 /* GELU, tanh form, and its derivative. */
 CSMC_HD float gelu_arg(float x) {
@@ -149,7 +149,7 @@ CSMC_HD MlpFeatures mlp_default_features(uint32_t n_vars, uint32_t C) {
  * the truncation is the floor; the multiples up to 1 are exact in BF16). */
 CSMC_HD float mlp_time_feature(float t, float T) {
     const float steps = static_cast<float>(static_cast<int>(f_mul(f_div(t, T), CSMC_MLP_TIME_STEPS)));
-    return bf16_round(f_div(steps, CSMC_MLP_TIME_STEPS));
+    return bf16_round(f_mul(steps, 1.0f / CSMC_MLP_TIME_STEPS));  /* exact: a power of two */
 }
 
 /* Features of location class l (local index modulo 4): v[i] the value of
@@ -227,7 +227,7 @@ CSMC_HD bool tiltable(float inv) { return inv > 0.0f && inv < bits_f(0x7f800000u
 
 /* 1/inv' - 1/inv: the change of one component's rate (log2 units). */
 CSMC_HD double rate_change(float inv, float invp) {
-    return d_sub(d_div(1.0, static_cast<double>(invp)), d_div(1.0, static_cast<double>(inv)));
+    return d_sub(d_rcp(static_cast<double>(invp)), d_rcp(static_cast<double>(inv)));
 }
 
 /* Log-likelihood ratio (nominal over proposal) of one race step that took

@@ -257,6 +257,18 @@ inline size_t is_coded_slab_bytes(uint32_t n_comps, uint32_t n_vars, uint32_t n_
                                                                      n_groups, recv, 16u * T);
 }
 
+// The one-warp-per-run kernel of networks whose locations are all
+// exponential or zero-delay (sim_is_plain.cuh), and the shared memory of one
+// of its warps.
+int is_plain_launch(bool tc, bool trace, const IsParams &p, int grid, int block, size_t smem, void *stream);
+int is_plain_max_active_ctas(bool tc, bool trace, int block, size_t smem, int *ctas);
+inline size_t is_plain_slab_bytes(uint32_t n_comps, uint32_t n_vars, uint32_t n_rate_prog, bool recv, bool tc) {
+    const size_t nb = (n_comps + 3u) / 4u;
+    const size_t b = (tc ? 0u : 4u * CSMC_MLP_HID * CSMC_MLP_CLASSES) + 4u * 16u + nb * (32u + 16u) + 4u * n_comps +
+                     4u * ((recv ? 2u : 1u) * n_vars + n_rate_prog) + 2u * n_comps;
+    return (b + 15u) & ~static_cast<size_t>(15);
+}
+
 // tc: theta by warp-level tensor-core MMAs (else the CUDA-core evaluation
 // that is bit-identical to the CPU oracle).
 int is_launch(bool tc, bool trace, bool slots, bool loc8, const IsParams &p, int grid, int block, size_t smem,

@@ -110,6 +110,13 @@ struct VarView {
     __device__ __forceinline__ float &operator[](uint32_t i) const { return base[i * stride]; }
 };
 
+// Key of a delay for 32-bit comparisons (delay_key): one OR unless the
+// delay is negative or NaN.
+static __device__ __forceinline__ uint32_t group_key(float d) {
+    const uint32_t b = f_bits(d);
+    return b <= 0x7f800000u ? (b | 0x80000000u) : delay_key(d);
+}
+
 static __device__ __forceinline__ void mix(unsigned long long &h, uint32_t w) { h = (h ^ w) * 0x100000001b3ull; }
 
 // One operator of the expression language on the two top stack entries

@@ -78,13 +78,6 @@ static __device__ __noinline__ float group_slow_delay(const uint8_t *base, const
 // zero, through comp_delay, or the one-invariant word + kFormInv1.
 constexpr uint32_t kFormExp = 0u, kFormZero = 1u, kFormSlow = 2u, kFormInv1 = 3u;
 
-// Key of a delay for 32-bit comparisons (delay_key): one OR unless the
-// delay is negative or NaN.
-static __device__ __forceinline__ uint32_t group_key(float d) {
-    const uint32_t b = f_bits(d);
-    return b <= 0x7f800000u ? (b | 0x80000000u) : delay_key(d);
-}
-
 // Bit reversal of k over the K (a power of two) components of a lane.
 static __host__ __device__ constexpr int lane_brev(int k, int K) {
     int r = 0;

@@ -46,11 +46,14 @@ constexpr unsigned kFullWarp = 0xffffffffu;
 
 struct MlpSmem {  // the proposal network in shared memory
     float w1t[CSMC_MLP_IN][CSMC_MLP_HID];   // FP32 copies of the BF16 weights, [input][unit]
-    float w2t[CSMC_MLP_HID][CSMC_MLP_HID];  // [input unit][output unit]
+    float2 w2t[CSMC_MLP_HID][CSMC_MLP_HID / 2];  // [input unit][lane]: output units lane and lane + 32
     float b1[CSMC_MLP_HID], b2[CSMC_MLP_HID], w3[CSMC_MLP_HID];
     float b3, pad[3];
     uint16_t w1h[CSMC_MLP_HID][CSMC_MLP_IN];  // BF16, [unit][input]: MMA B fragments
     uint16_t w2h[CSMC_MLP_HID][CSMC_MLP_HID];
+    __device__ __forceinline__ void set_w2(uint32_t in, uint32_t out, float w) {
+        (out < 32u ? w2t[in][out].x : w2t[in][out - 32u].y) = w;
+    }
 };
 static_assert(sizeof(MlpSmem) % 16 == 0, "warp slabs follow the proposal network 16-byte aligned");
 
@@ -63,7 +66,7 @@ static __device__ __forceinline__ void stage_mlp(MlpSmem *m, const MlpParams *P)
     for (uint32_t i = threadIdx.x; i < CSMC_MLP_HID * CSMC_MLP_HID; i += blockDim.x) {
         const uint16_t w = (&P->w2[0][0])[i];
         (&m->w2h[0][0])[i] = w;
-        m->w2t[i % CSMC_MLP_HID][i / CSMC_MLP_HID] = bf16_to_f(w);
+        m->set_w2(i % CSMC_MLP_HID, i / CSMC_MLP_HID, bf16_to_f(w));
     }
     for (uint32_t i = threadIdx.x; i < CSMC_MLP_HID; i += blockDim.x) {
         m->b1[i] = P->b1[i];
@@ -116,7 +119,8 @@ static __device__ __forceinline__ void theta_exact(const MlpSmem *m, float *h1s,
 #pragma unroll 8
     for (int j = 0; j < CSMC_MLP_HID; ++j) {
         const float4 h = h4[j];
-        const float wa = m->w2t[j][lane], wb = m->w2t[j][lane + 32];
+        const float2 w = m->w2t[j][lane];
+        const float wa = w.x, wb = w.y;
         ya[0] = f_fma(h.x, wa, ya[0]);
         ya[1] = f_fma(h.y, wa, ya[1]);
         ya[2] = f_fma(h.z, wa, ya[2]);
@@ -204,15 +208,22 @@ static __device__ __forceinline__ void theta_tc(const MlpSmem *m, const float *x
 // ---- the race under the proposal ------------------------------------------
 
 // Delay of a component on the general path under the proposal.
-static __device__ __noinline__ float is_slow_delay(const Net &n, VarView vars, VarView rates, uint32_t li, uint32_t x,
-                                                   float mfac, bool *tilted, float *inv_o, float *invp_o) {
-    *tilted = false;
-    *inv_o = *invp_o = 0.0f;
+struct SlowDelay {
+    float d, inv, invp;
+    bool tilted;
+};
+static __device__ __noinline__ SlowDelay is_slow_delay(const uint8_t *base, VarView vars, VarView rates, uint32_t li,
+                                                       uint32_t x, float mfac) {
+    const Net n = net_view(base);
+    SlowDelay o{0.0f, 0.0f, 0.0f, false};
     const csmc_loc L = n.loc[li];
-    if (L.type > 1) return 0.0f;
+    if (L.type > 1) return o;
     if (L.n_inv) {
         double max_delay;
-        if (delay_bound(n, vars, L, max_delay)) return uniform_delay(x, max_delay);
+        if (delay_bound(n, vars, L, max_delay)) {
+            o.d = uniform_delay(x, max_delay);
+            return o;
+        }
     }
     float inv;
     if (n.flags & CSMC_NET_RATE_TABLE) {
@@ -224,11 +235,12 @@ static __device__ __noinline__ float is_slow_delay(const Net &n, VarView vars, V
     float invp = inv;
     if (tiltable(inv)) {
         invp = f_mul(inv, mfac);
-        *tilted = true;
+        o.tilted = true;
     }
-    *inv_o = inv;
-    *invp_o = invp;
-    return exp_delay(x, invp);
+    o.inv = inv;
+    o.invp = invp;
+    o.d = exp_delay(x, invp);
+    return o;
 }
 
 struct LaneRace {  // one lane's share of a step's race
@@ -273,8 +285,14 @@ static __device__ __forceinline__ void lane_race(const Net &n, uint32_t C, uint3
                 float d, inv = 0.0f, invp = 0.0f;
                 bool tilted = false;
                 if (fl & (CSMC_DESC_ZERO | CSMC_DESC_INV | CSMC_DESC_EVAL)) {
-                    if (fl & CSMC_DESC_ZERO) d = 0.0f;
-                    else d = is_slow_delay(n, rv.vars, rv.rates, li, x, m, &tilted, &inv, &invp);
+                    d = 0.0f;
+                    if (!(fl & CSMC_DESC_ZERO)) {
+                        const SlowDelay o = is_slow_delay(n.base, rv.vars, rv.rates, li, x, m);
+                        d = o.d;
+                        inv = o.inv;
+                        invp = o.invp;
+                        tilted = o.tilted;
+                    }
                 } else {
                     inv = __uint_as_float(lo);
                     if (fl & CSMC_DESC_PROG) inv = rv.rates[lo];
@@ -293,7 +311,7 @@ static __device__ __forceinline__ void lane_race(const Net &n, uint32_t C, uint3
                         if (TRACE) r = l == 0 ? k_rec[0] : (l == 1 ? k_rec[1] : (l == 2 ? k_rec[2] : k_rec[3]));
                     } else {
                         diff = rate_change(inv, invp);
-                        if (TRACE) r = d_div(1.0, static_cast<double>(inv));
+                        if (TRACE) r = d_rcp(static_cast<double>(inv));
 #pragma unroll
                         for (int j = 0; j < CSMC_MLP_CLASSES; ++j)
                             if (static_cast<uint32_t>(j) == l) {

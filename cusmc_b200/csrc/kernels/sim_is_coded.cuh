@@ -64,7 +64,7 @@ static __device__ __forceinline__ void stage_mlp_exact(MlpSmem *m, const MlpPara
     for (uint32_t i = threadIdx.x; i < CSMC_MLP_HID * CSMC_MLP_IN; i += blockDim.x)
         m->w1t[i % CSMC_MLP_IN][i / CSMC_MLP_IN] = bf16_to_f((&P->w1[0][0])[i]);
     for (uint32_t i = threadIdx.x; i < CSMC_MLP_HID * CSMC_MLP_HID; i += blockDim.x)
-        m->w2t[i % CSMC_MLP_HID][i / CSMC_MLP_HID] = bf16_to_f((&P->w2[0][0])[i]);
+        m->set_w2(i % CSMC_MLP_HID, i / CSMC_MLP_HID, bf16_to_f((&P->w2[0][0])[i]));
     for (uint32_t i = threadIdx.x; i < CSMC_MLP_HID; i += blockDim.x) {
         m->b1[i] = P->b1[i];
         m->b2[i] = P->b2[i];
@@ -206,7 +206,8 @@ static __device__ __forceinline__ void theta_exact_n(const MlpSmem *m, float *h1
         }
 #pragma unroll 4
     for (int j = 0; j < CSMC_MLP_HID; ++j) {
-        const float wa = m->w2t[j][lane], wb = m->w2t[j][lane + 32];
+        const float2 w = m->w2t[j][lane];
+        const float wa = w.x, wb = w.y;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             const float4 h = reinterpret_cast<const float4 *>(h1s + v * (CSMC_MLP_HID * 4))[j];
@@ -273,7 +274,13 @@ static __device__ __forceinline__ float is_desc_delay(const Net &n, VarView vars
     tilted = false;
     inv = invp = 0.0f;
     if (fl & CSMC_DESC_ZERO) return 0.0f;
-    if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) return is_slow_delay(n, vars, rates, li, x, m, &tilted, &inv, &invp);
+    if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) {
+        const SlowDelay o = is_slow_delay(n.base, vars, rates, li, x, m);
+        inv = o.inv;
+        invp = o.invp;
+        tilted = o.tilted;
+        return o.d;
+    }
     inv = (fl & CSMC_DESC_PROG) ? rates[lo] : __uint_as_float(lo);
     invp = inv;
     if (tiltable(inv)) {

@@ -4,6 +4,9 @@ the bits of the definitions they replace.
 * exp_delay: the integer draw's exponent and mantissa are split before the
   scaling and the logarithm's quotient is a Markstein division; every one of
   the 2^24 draws is compared with the host's form (tolerance: none).
+* GELU: its sigmoid's reciprocal is an approximation and a Newton step; a
+  grid of 2^24 floats over the exponents where the sigmoid is neither 0 nor
+  1, and the clamped ends, are compared with the host's form (none).
 * time_add: one float addition instead of a double sum rounded to float.
 """
 import numpy as np
@@ -25,6 +28,26 @@ def test_exp_delay_of_every_draw_equals_the_host():
     torch.cuda.synchronize()
     want = oracle.numeric(_native.NUM_EXP_DELAY, x, inv)
     assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.gpu
+def test_gelu_over_a_dense_grid_equals_the_host():
+    import torch
+    from cusmc_b200 import _native
+    from cusmc_b200._native import check, lib
+    step = np.arange(1 << 22, dtype=np.uint32) * np.uint32(37)
+    x = np.concatenate([(np.uint32(0x3c000000) + step % np.uint32(0x05000000)).view(np.float32),
+                        -(np.uint32(0x3c000000) + step % np.uint32(0x05000000)).view(np.float32),
+                        np.linspace(-12.0, 12.0, 1 << 23, dtype=np.float32),
+                        np.array([0.0, -0.0, 50.0, -50.0, 1e9, -1e9, 3e38, -3e38], np.float32)])
+    for fn in (_native.NUM_GELU_F32, _native.NUM_GELU_GRAD_F32):
+        got = torch.empty(x.size, dtype=torch.float32, device="cuda")
+        xd = torch.from_numpy(x).cuda()
+        check(lib().csmc_numeric_eval(fn, xd.data_ptr(), None, x.size, got.data_ptr(), None))
+        torch.cuda.synchronize()
+        want = oracle.numeric(fn, x)
+        same = got.cpu().numpy().view(np.uint32) == want.view(np.uint32)
+        assert np.all(same | (np.isnan(want) & np.isnan(got.cpu().numpy())))
 
 
 def test_float_sum_equals_the_double_sum_rounded_to_float():
