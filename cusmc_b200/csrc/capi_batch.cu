@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <memory>
 #include <numeric>
@@ -33,6 +34,7 @@ struct csmc_batch {
     std::vector<char> group;           // per job: simulated one warp per run
     int n_group = 0;                   // warp-per-run jobs
     uint32_t group_min_comps = kDefaultGroupMinComps;  // networks this large run one warp per run (0: none do)
+    bool group_auto = true;            // no threshold was chosen: smaller networks may run one warp per run too
     int group_k = 0;                   // components per lane of the warp-per-run jobs
     uint32_t group_stride = 0;         // shared memory of one warp-per-run run state
     std::vector<uint64_t> out_off;     // per job: first run's index in the output buffers
@@ -99,15 +101,53 @@ void drop_graph(csmc_batch *b) {
 // CSMC_BATCH_GROUP_MAX_COMPS components), the job-table order (those jobs
 // first, each part by falling cost), the lanes' component count and the
 // state sizes of both parts.
+//
+// Until the caller chooses a threshold (csmc_batch_set_group_comps, the
+// autotuner), networks below group_min_comps run one warp per run too where
+// the batch is estimated to end earlier so: with few runs the thread-per-run
+// part lasts as long as its longest run at one thread's speed.  The estimate,
+// per threshold m (all networks of m components and more one warp per run):
+// a run of a C-component network makes about 0.57 C T race steps (random
+// networks); a warp's step takes 2 + 4 ceil(C / 128) issue slots and 4.4 (3 +
+// 4 ceil(C / 128)) of latency, 32 threads' step 1 + 1.85 C (latency 5 times
+// that); each part lasts max(longest run, work / schedulers).  In units of
+// launch_plan (capi.cu).
+uint32_t auto_min_comps(const csmc_batch *b) {
+    double best = -1.0;
+    uint32_t pick = b->group_min_comps;
+    for (uint32_t m : {b->group_min_comps, 64u, 32u, 16u, 8u, 4u}) {
+        double warp_work = 0, warp_long = 0, thread_work = 0, thread_long = 0;
+        for (int j = 0; j < b->n_jobs; ++j) {
+            const double C = b->nets[j]->h.n_comps, runs = static_cast<double>(b->n_runs[j]);
+            if (runs == 0) continue;
+            const double steps = C * std::max(1.0, b->qs[j].horizon), its = std::ceil(C / 128.0);
+            if (C >= m && C <= CSMC_BATCH_GROUP_MAX_COMPS) {
+                warp_work += runs * steps * (2.0 + 4.0 * its);
+                warp_long = std::max(warp_long, steps * 4.4 * (3.0 + 4.0 * its));
+            } else {
+                thread_work += runs / 32.0 * steps * (1.0 + 1.85 * C);
+                thread_long = std::max(thread_long, steps * 5.0 * (1.0 + 1.85 * C));
+            }
+        }
+        const double schedulers = 4.0 * std::max(1, b->nets[0]->sms);
+        const double t = std::max(warp_long, warp_work / schedulers) + std::max(thread_long, thread_work / schedulers);
+        if (best < 0.0 || t < 0.9 * best) {
+            best = t;
+            pick = m;
+        }
+    }
+    return pick;
+}
+
 void assign_modes(csmc_batch *b) {
     b->group.assign(b->n_jobs, 0);
     b->n_group = 0;
     b->max_v = b->max_p = b->max_c = 0;
     uint32_t gmax_c = 0, gmax_vp = 0;
+    const uint32_t min_comps = b->group_auto ? auto_min_comps(b) : b->group_min_comps;
     for (int j = 0; j < b->n_jobs; ++j) {
         const csmc_net_header &h = b->nets[j]->h;
-        const bool g = b->group_min_comps > 0 && h.n_comps >= b->group_min_comps &&
-                       h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS;
+        const bool g = min_comps > 0 && h.n_comps >= min_comps && h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS;
         b->group[j] = g;
         if (g) {
             ++b->n_group;
@@ -393,6 +433,7 @@ int csmc_batch_set_group_comps(csmc_batch *b, int32_t min_comps) {
     if (min_comps < 0) return fail(CSMC_ERR_ARG, "negative component threshold");
     CK(cudaSetDevice(b->device), "cudaSetDevice");
     b->group_min_comps = static_cast<uint32_t>(min_comps);
+    b->group_auto = false;
     assign_modes(b);
     int rc = configure(b);
     if (rc) return rc;
@@ -402,7 +443,12 @@ int csmc_batch_set_group_comps(csmc_batch *b, int32_t min_comps) {
 int csmc_batch_group_comps(const csmc_batch *b, int32_t *min_comps, int32_t *group_jobs) {
     if (!b) return fail(CSMC_ERR_ARG, "null argument");
     if (min_comps) *min_comps = static_cast<int32_t>(b->group_min_comps);
-    if (group_jobs) *group_jobs = b->n_group;
+    if (group_jobs) {  // the jobs the threshold selects
+        *group_jobs = 0;
+        for (const csmc_net *n : b->nets)
+            *group_jobs += b->group_min_comps > 0 && n->h.n_comps >= b->group_min_comps &&
+                           n->h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS;
+    }
     return CSMC_OK;
 }
 
@@ -492,10 +538,14 @@ int csmc_batch_autotune(csmc_batch *b, double probe_fraction, int32_t *threads_p
     for (int j = 0; j < b->n_jobs; ++j)
         runs[j] = b->n_runs[j] ? std::max<uint64_t>(1, static_cast<uint64_t>(b->n_runs[j] * probe_fraction)) : 0;
     const int save_block = b->block, save_ctas = b->ctas_per_sm;
+    b->group_auto = false;  // the probes choose the threshold
+    assign_modes(b);
+    int rc = configure(b);
+    if (rc) return rc;
     // 1. measure the cost per run of every job at the current geometry
     std::vector<uint64_t> steps;
     float ms = 0.0f;
-    int rc = probe(b, runs, &ms, &steps);
+    rc = probe(b, runs, &ms, &steps);
     if (rc) return rc;
     for (int j = 0; j < b->n_jobs; ++j)  // measured cost per run where no probe run was capped
         if (runs[j] && steps[j])

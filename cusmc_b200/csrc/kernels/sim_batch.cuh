@@ -2,7 +2,8 @@
 // query) jobs.  Runs of small networks are simulated by one thread each
 // with the step of sim_run.cuh; runs of large networks (the jobs the host
 // marks, at most CSMC_BATCH_GROUP_MAX_COMPS components) by one warp each,
-// 32 lanes x K components, with the lane-group run of sim_impl.cuh, so that
+// with the lane-group run of sim_impl.cuh (a step takes one Philox block per
+// lane and 128 components, whatever the batch's largest network), so that
 // the long runs of a large network do not leave one thread working alone
 // at the end of the batch.
 //
@@ -58,14 +59,13 @@ static __device__ __forceinline__ void flush_counters(const BatchJob &J, unsigne
     hits = steps = capped = 0;
 }
 
-// Warp-per-run jobs (K components per lane): whole warps take runs from
-// p.group_queue until it passes p.group_runs.  Not inlined, so that its
-// registers are allocated apart from the thread-per-run phase's.
-template <int K, bool VERIFY>
+// Warp-per-run jobs: whole warps take runs from p.group_queue until it
+// passes p.group_runs.
+template <bool VERIFY>
 static __device__ __forceinline__ void batch_group_phase(const BatchParams &p, const BatchJob *jobs, uint8_t *smem) {
     const uint32_t lane = threadIdx.x & 31u;
     RunState *s = reinterpret_cast<RunState *>(smem + p.n_jobs * sizeof(BatchJob) + (threadIdx.x >> 5) * p.group_stride);
-    GroupRun<32, K, VERIFY> g(s, lane);
+    GroupRun<32, 4, 0, VERIFY> g(s, lane, 32u * p.group_k);
     unsigned long long acc_hits = 0, acc_steps = 0, acc_capped = 0;
     uint32_t jb = 0;
     for (;;) {
@@ -89,8 +89,8 @@ static __device__ __forceinline__ void batch_group_phase(const BatchParams &p, c
     if (lane == 0) flush_counters(jobs[jb], acc_hits, acc_steps, acc_capped);
 }
 
-template <bool VERIFY, int K>
-__global__ void __launch_bounds__(128, K > 0 ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM : CSMC_BATCH_MIN_CTAS_PER_SM) batch_kernel(const __grid_constant__ BatchParams p) {
+template <bool VERIFY, bool GROUPS>
+__global__ void __launch_bounds__(128, GROUPS ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM : CSMC_BATCH_MIN_CTAS_PER_SM) batch_kernel(const __grid_constant__ BatchParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     {  // stage the job table
         const uint4 *src = reinterpret_cast<const uint4 *>(p.jobs);
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(128, K > 0 ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM 
         for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
     }
     __syncthreads();
-    if constexpr (K > 0) {
-        if (p.n_group_jobs > 0) batch_group_phase<K, VERIFY>(p, reinterpret_cast<const BatchJob *>(smem), smem);
+    if constexpr (GROUPS) {
+        if (p.n_group_jobs > 0) batch_group_phase<VERIFY>(p, reinterpret_cast<const BatchJob *>(smem), smem);
     }
     if (p.n_jobs == p.n_group_jobs) return;
     const BatchJob *jobs = reinterpret_cast<const BatchJob *>(smem) + p.n_group_jobs;
@@ -180,9 +180,9 @@ __global__ void __launch_bounds__(128, K > 0 ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM 
 
 }  // namespace detail
 
-template <bool VERIFY, int K>
+template <bool VERIFY, bool GROUPS>
 int batch_launch_one(const BatchParams &p, int grid, int block, void *stream) {
-    auto fn = detail::batch_kernel<VERIFY, K>;
+    auto fn = detail::batch_kernel<VERIFY, GROUPS>;
     const size_t smem = batch_smem_bytes(p.n_jobs, p.n_group_jobs ? p.group_stride : 0u, block);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -190,9 +190,9 @@ int batch_launch_one(const BatchParams &p, int grid, int block, void *stream) {
     return static_cast<int>(cudaGetLastError());
 }
 
-template <bool VERIFY, int K>
+template <bool VERIFY, bool GROUPS>
 int batch_occupancy_one(int block, size_t smem, int *ctas) {
-    auto fn = detail::batch_kernel<VERIFY, K>;
+    auto fn = detail::batch_kernel<VERIFY, GROUPS>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return static_cast<int>(e);
     return static_cast<int>(cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, fn, block, smem));

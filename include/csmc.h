@@ -165,6 +165,9 @@ int csmc_query_parse(const char *xml_path, const char *formula, csmc_query *q, c
 
 /* Sizes a launch would use for this network: lanes per run, components per
  * lane, runs per CTA. */
+/* (the plan csmc_set_plan or csmc_autotune set; else the default of launches
+ * that fill the GPU: launches of fewer runs take lane groups chosen by the
+ * number of runs, reported in csmc_result) */
 int csmc_plan(const csmc_net *net, int32_t *lanes_per_run, int32_t *comps_per_lane, int32_t *runs_per_cta);
 
 /* Overrides the launch plan of a network handle (used by the autotuner):
@@ -213,9 +216,12 @@ int csmc_batch_plan(const csmc_batch *b, int32_t *threads_per_cta, int32_t *ctas
 /* Jobs whose networks have min_comps .. 512 components are simulated one
  * warp per run (32 lanes, up to 16 components each) instead of one thread
  * per run; every warp takes those runs first, then joins the one-thread-per-
- * run queue.  0: every job runs one thread per run.  Default 128.  The
- * per-run results do not depend on it.  csmc_batch_group_comps reports the
- * threshold and how many jobs it selects. */
+ * run queue.  0: every job runs one thread per run.  Default 128; until the
+ * threshold is set (here or by csmc_batch_autotune), smaller networks run one
+ * warp per run too where the batch is estimated to end earlier so (reported
+ * per job in csmc_result.lanes_per_run).  The per-run results do not depend
+ * on it.  csmc_batch_group_comps reports the threshold and how many jobs it
+ * selects. */
 int csmc_batch_set_group_comps(csmc_batch *b, int32_t min_comps);
 int csmc_batch_group_comps(const csmc_batch *b, int32_t *min_comps, int32_t *group_jobs);
 
