@@ -165,90 +165,94 @@ bool configure_plan(const csmc_net *n, csmc_launch_plan &p, int family, int lane
 // ---- lane-group shapes and the choice by launch size ------------------------
 
 // The shapes (lanes per run, components per lane) a network can run with,
-// widest first: every power of two from one component per lane down to four
-// components per lane, then the lane's share doubled to 16.
+// widest first: one component per lane in groups of 32 lanes down to the
+// network's size (a warp with one group has no other group to branch apart
+// from), two, four components per lane, then the lane's share doubled to 16.
 void find_shapes(csmc_net *n) {
     const csmc_net_header &h = n->h;
     const size_t cta_smem = static_cast<size_t>(max_smem_optin(n->device));
     int sm_smem = 0;
     cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, n->device);
     n->n_shapes = 0;
-    int G = 0, K = 0;
-    choose_shape(h.n_comps, G, K);
-    for (; G >= 2 && K <= 16 && n->n_shapes < 6;) {
-        if (csmc::sim_supported(G, K)) {
-            csmc_group_shape s;
-            s.lanes = G;
-            s.comps_per_lane = K;
-            s.stride = csmc::group_state_stride(h.n_vars, h.n_rate_prog, G, K);
-            // 16 warps per SM (128 registers a thread) in the largest CTA that
-            // fits: its warps share one copy of the network
-            for (int block : {512, 256, 128, 64, 32}) {
-                const size_t smem = n->bytes + static_cast<size_t>(block / G) * s.stride;
-                if (smem > cta_smem) continue;
-                const int ctas = std::min(512 / block, static_cast<int>(static_cast<size_t>(sm_smem) / (smem + 1024)));
-                const int warps = ctas * (block / 32);
-                if (warps > s.warps) {
-                    s.warps = warps;
-                    s.block = block;
-                }
+    auto add = [&](int G, int K) {
+        if (n->n_shapes >= 6 || !csmc::sim_supported(G, K)) return;
+        csmc_group_shape s;
+        s.lanes = G;
+        s.comps_per_lane = K;
+        s.stride = csmc::group_state_stride(h.n_vars, h.n_rate_prog, G, K);
+        // 16 warps per SM (128 registers a thread) in the largest CTA that
+        // fits: its warps share one copy of the network
+        for (int block : {512, 256, 128, 64, 32}) {
+            const size_t smem = n->bytes + static_cast<size_t>(block / G) * s.stride;
+            if (smem > cta_smem) continue;
+            const int ctas = std::min(512 / block, static_cast<int>(static_cast<size_t>(sm_smem) / (smem + 1024)));
+            const int warps = ctas * (block / 32);
+            if (warps > s.warps) {
+                s.warps = warps;
+                s.block = block;
             }
-            if (s.warps > 0) n->shapes[n->n_shapes++] = s;
         }
-        if (h.n_comps <= 4) break;
-        if (K < 4) {  // one Philox block per lane: the lanes of K = 1, 2 draw it and use a part
-            G = static_cast<int>(std::max(2u, csmc::ceil_pow2((h.n_comps + 3) / 4)));
-            K = 4;
-            if (n->n_shapes && n->shapes[n->n_shapes - 1].lanes <= G) G /= 2, K *= 2;
-        } else {
-            G /= 2;
-            K *= 2;
-        }
-    }
+        if (s.warps > 0) n->shapes[n->n_shapes++] = s;
+    };
+    const uint32_t C = h.n_comps, lanes = csmc::ceil_pow2(C), blocks = csmc::ceil_pow2((C + 3) / 4);
+    for (uint32_t G = 32; G >= lanes && G >= 2; G /= 2) add(static_cast<int>(G), 1);
+    if (lanes == 32) add(16, 2);
+    if (lanes == 64) add(32, 2);
+    if (C <= 4) return;
+    uint32_t G = std::min(32u, blocks), K = 4;
+    while (G * K < C) K *= 2;
+    for (; G >= 2 && K <= 16; G /= 2, K *= 2) add(static_cast<int>(G), static_cast<int>(K));
 }
 
 // The plan of a launch of n_runs runs.  A run's steps are a serial chain, so
 // a launch that does not fill the GPU takes its longest run's steps times
 // the latency of a step, which falls with the lanes a run has; one that
 // fills it takes the issue slots of all steps, which are fewest with many
-// runs per warp.  In units of one component of a lane, a warp's step has the
-// latency 4.4 L and takes I issue slots:
-//   groups:     L = 3 + K + 0.1 (32 / G - 1), I = 2 + K + 0.45 (32 / G - 1)
-//               (the groups of a warp branch apart)
-//   one thread: L = 12 + 0.22 C (every location classed), 4 + 1.1 C (classes
-//               and descriptors) or 1 + 1.85 C (no classes), latency 5 L (a
-//               warp waits for the longest of 32 runs), I = 1.2 L (1 L)
-// and a launch takes max(latency, (waves + 1) I), a wave being one warp per
-// scheduler; I is scaled by 13.2 (10) / (resident warps per SM) where those
-// are too few to hide the latency.  Fitted to the epidemic (12 to 200
-// agents), the mutex (8 to 256) and random networks (4 to 64 components) at
+// runs per warp.  A warp's step of a shape costs S:
+//   groups:     S = (12 + K) (1 + d log2(32 / G)), the groups of a warp
+//               branching apart (d = 0.33; 0.5 in networks without race
+//               classes, whose steps differ more)
+//   one thread: S = 48 + 0.7 C (every location classed), 42 + 4.5 C (classes
+//               and descriptors), 30 + 7.5 C (no classes)
+// and a launch takes S times the larger of its latency, 3.9 (2.8 one thread),
+// and its waves + 1, a wave being one warp per scheduler (waves count for more
+// where too few warps are resident to hide the latency).  Runs of networks
+// with clocks are about equally long: what does not fit on the SMs at once
+// waits for a whole latency.  Without clocks they differ, and the longest
+// makes the latency 1.7 times that.  Fitted to the epidemic (12 to 200
+// agents), the mutex (8 to 256) and random networks (2 to 64 components) at
 // 100 to 131,072 runs on B200.  One thread per run / the best group: 100
 // agents 100 runs 14.3 / 3.0 ms, 16,384 runs 16.2 / 13.8, 32,768 runs 19.6 /
-// 23.5; mutex 32, 100 runs 28.4 / 2.9, 32,768 runs 30.8 / 20.4, 65,536 runs
-// 39.7 / 39.6; random 8, 100 runs 2.2 / 0.7, 131,072 runs 6.3 / 6.0; random
-// 24, 65,536 runs 19.7 / 24.0; random 64, 131,072 runs 288 / 90.
+// 23.5; mutex 32, 100 runs 28.4 / 2.8, 32,768 runs 30.8 / 20.4, 65,536 runs
+// 39.7 / 39.6; random 8, 100 runs 2.2 / 0.43 (0.70 with groups of 8 lanes),
+// 131,072 runs 6.3 / 6.0; random 24, 65,536 runs 19.7 / 24.0; random 64,
+// 131,072 runs 288 / 90.
 csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
     if (n->plan_forced || n->plan.family == 2 || n->n_shapes == 0) return n->plan;
     const double C = n->h.n_comps, unit = 128.0 * n->sms, runs = static_cast<double>(n_runs);
+    const bool even = n->h.n_clocks > 0;
+    auto launch_time = [&](double S, double warps, double latency, int resident, double hide) {
+        const double waves = warps * 32.0 / unit;
+        const double rounds = even ? std::ceil(warps / (static_cast<double>(resident) * n->sms)) : 1.7;
+        return S * std::max(latency * rounds, waves * std::max(1.0, hide / resident) + 1.0);
+    };
+    const double apart = n->classes ? 0.33 : 0.5;
     double best = 0.0;
     const csmc_group_shape *pick = nullptr;
     for (int i = 0; i < n->n_shapes; ++i) {
         const csmc_group_shape &s = n->shapes[i];
-        const double K = s.comps_per_lane, apart = 32.0 / s.lanes - 1.0;
-        const double I = (2.0 + K + 0.45 * apart) * std::max(1.0, 13.2 / s.warps);
-        const double t = std::max(4.4 * (3.0 + K + 0.1 * apart), (runs * s.lanes / unit + 1.0) * I);
+        const double S = (12.0 + s.comps_per_lane) * (1.0 + apart * csmc::ceil_log2(32u / s.lanes));
+        const double t = launch_time(S, std::ceil(runs * s.lanes / 32.0), 3.9, s.warps, 13.2);
         if (!pick || t < best) {
             best = t;
             pick = &s;
         }
     }
     if (n->thread_warps > 0) {
-        const bool classes = n->plan.family == 4;
-        const double L = classes ? (n->only_classes ? 12.0 + 0.22 * C : 4.0 + 1.1 * C) : 1.0 + 1.85 * C;
-        const double I = (classes ? 1.2 : 1.0) * L * std::max(1.0, 10.0 / n->thread_warps);
-        const double t = std::max(5.0 * L, (runs / unit + 1.0) * I);
+        const double S = n->plan.family != 4 ? 30.0 + 7.5 * C : n->only_classes ? 48.0 + 0.7 * C : 42.0 + 4.5 * C;
+        const double t = launch_time(S, std::ceil(runs / 32.0), 2.8, n->thread_warps, 10.0);
         // (where both fill the GPU a group is taken only when it is clearly the better one)
-        if (t < best * (runs > 1.75 * unit ? 1.25 : 1.0)) return n->plan;
+        if (t < best * (runs > 1.75 * unit ? 1.3 : 1.0)) return n->plan;
     }
     csmc_launch_plan p;
     p.family = 0;

@@ -66,7 +66,7 @@ int serial_max_active_ctas(bool verify, bool slots, bool loc8, bool gstate, bool
 
 #define CSMC_SHAPES(X) \
     X(1, 1) X(2, 1) X(4, 1) X(8, 1) X(16, 1) X(32, 1) X(32, 2) X(32, 4) X(32, 8) X(32, 16) X(32, 32) \
-    X(2, 4) X(4, 4) X(8, 4) X(16, 4) X(4, 8) X(8, 8) X(16, 8) X(8, 16) X(16, 16)
+    X(16, 2) X(2, 4) X(4, 4) X(8, 4) X(16, 4) X(4, 8) X(8, 8) X(16, 8) X(8, 16) X(16, 16)
 
 bool sim_supported(int g, int k) {
 #define X(GG, KK) \

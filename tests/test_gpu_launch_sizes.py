@@ -80,7 +80,7 @@ def test_location_query_at_small_and_large_launches():
 
 
 @pytest.mark.parametrize("g,k,net", [
-    (2, 4, "random5"), (4, 4, "mutex13"), (8, 4, "mutex32"), (16, 4, "epidemic63"), (4, 8, "mutex32"),
+    (32, 1, "random2"), (16, 2, "mutex32"), (2, 4, "random5"), (4, 4, "mutex13"), (8, 4, "mutex32"), (16, 4, "epidemic63"), (4, 8, "mutex32"),
     (8, 8, "epidemic63"), (16, 8, "epidemic100"), (8, 16, "epidemic100"), (16, 16, "mutex130"), (32, 16, "random300"),
 ])
 def test_lane_group_shapes_give_the_oracle_traces(g, k, net):
