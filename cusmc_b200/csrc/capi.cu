@@ -218,7 +218,8 @@ void find_shapes(csmc_net *n) {
 // and its waves + 1, a wave being one warp per scheduler (waves count for more
 // where too few warps are resident to hide the latency).  Runs of networks
 // with clocks are about equally long: what does not fit on the SMs at once
-// waits for a whole latency.  Without clocks they differ, and the longest
+// waits for most of another latency (random 8, groups of 8 lanes: 9,472 runs
+// fit; 10,000 take 1.4 times the latency of 8,192, 16,384 1.8 times).  Without clocks they differ, and the longest
 // makes the latency 1.7 times that.  Fitted to the epidemic (12 to 200
 // agents), the mutex (8 to 256) and random networks (2 to 64 components) at
 // 100 to 131,072 runs on B200.  One thread per run / the best group: 100
@@ -233,7 +234,9 @@ csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
     const bool even = n->h.n_clocks > 0;
     auto launch_time = [&](double S, double warps, double latency, int resident, double hide) {
         const double waves = warps * 32.0 / unit;
-        const double rounds = even ? std::ceil(warps / (static_cast<double>(resident) * n->sms)) : 1.7;
+        const double full = warps / (static_cast<double>(resident) * n->sms), part = full - std::floor(full);
+        const double rounds =
+            !even ? 1.7 : std::max(1.0, std::floor(full) + (part > 0.0 ? std::min(1.0, 0.6 + 0.55 * part) : 0.0));
         return S * std::max(latency * rounds, waves * std::max(1.0, hide / resident) + 1.0);
     };
     const double apart = n->classes ? 0.33 : 0.5;
