@@ -216,6 +216,23 @@ csmc::IsParams base_params(const csmc_net *n, const csmc_query *q, uint64_t seed
     return ip;
 }
 
+// The time feature's edges for horizon T (IsParams::time_edge): the feature
+// does not fall with the time (a division, an exact product and a truncation),
+// so each edge is found by bisection over the floats' bits.
+void time_edges(float T, float *edge) {
+    uint32_t lo = 0;
+    for (int k = 0; k <= 64; ++k) {
+        uint32_t hi = 0x7f800000u;  // +inf
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            const float q = csmc::f_mul(csmc::f_div(csmc::bits_f(mid), T), CSMC_MLP_TIME_STEPS);
+            if (csmc::f2i_sat(q) > k) hi = mid;
+            else lo = mid + 1;
+        }
+        edge[k] = csmc::bits_f(lo);
+    }
+}
+
 int check_query(const csmc_net *n, const csmc_query *q) {
     if (q->kind != CSMC_QUERY_LOCATION && q->kind != CSMC_QUERY_VARIABLE) return fail(CSMC_ERR_ARG, "bad query kind");
     if (q->kind == CSMC_QUERY_VARIABLE && (q->var_id < 0 || static_cast<uint32_t>(q->var_id) >= n->h.n_vars))
@@ -310,6 +327,7 @@ int csmc_is_run(csmc_net *n, const csmc_query *q, const void *params, uint64_t s
         ip.theta_cache = n->d_theta_cache;
         ip.cache_mask = kThetaCacheEntries - 1;
         ip.cache_gen = n->theta_gen;
+        time_edges(ip.s.horizon, ip.time_edge);
     }
     CK(cudaEventRecord(n->ev0, st), "cudaEventRecord");
     rc = coded ? csmc::is_coded_launch(L.slots, n->is_all_grouped, ip, L.grid, L.block, L.smem, st)

@@ -230,6 +230,9 @@ struct IsParams {
     uint32_t *theta_cache;
     uint32_t cache_mask;
     uint32_t cache_gen;                     // the parameter block's generation (bit 31 clear, not 0)
+    // thread-per-run kernel: [k] the smallest time whose feature is beyond
+    // k / CSMC_MLP_TIME_STEPS (+inf: none)
+    float time_edge[65];
 };
 // Theta cache entry: [0] state (generation, or generation | 1 << 31 while
 // being written), [1..3] the feature key, [4..7] the four class factors.

@@ -19,13 +19,21 @@
 // over tilted components) must carry the bits of the one-warp-per-run
 // kernel, whose lane L sums the components of Philox blocks L, L + 32, ...
 // in component order and whose lanes meet in a butterfly (csmc_mlp.h:
-// warp_lane_of, warp_tree_d).  The butterfly over offsets 16, 8, 4, 2, 1 is
-// the balanced binary tree over the lanes taken in 5-bit bit-reversed order,
-// so the thread walks the lanes in that order (the race does not depend on
-// the order of the blocks), sums each lane's blocks into its partial, and
-// merges the partials with a five-level stack (a binary counter): the same
-// additions in the same order.  A group member adds its group's rate
-// change, computed once per step from the group's 1/rate and factor.
+// warp_lane_of, warp_tree_d).  The sum changes only when the run moves a
+// component or its groups' rates change.  Where every component is in a
+// group, the warp evaluates it for the lanes that need it, one after another,
+// in exactly that form (group_rate_sum), and the race is sim_coded.cuh's.
+// Else (a descriptor path's terms depend on the step) each thread sums on
+// every step: the butterfly over offsets 16, 8, 4, 2, 1 is the balanced
+// binary tree over the lanes taken in 5-bit bit-reversed order, so the thread
+// walks the lanes in that order (the race does not depend on the order of the
+// blocks), sums each lane's blocks into its partial, and merges the partials
+// with a five-level stack (a binary counter): the same additions in the same
+// order.  A group member adds its group's rate change, computed when the
+// group's 1/rate or factor changes.  Measured (B200), 100-agent epidemic under
+// a proposal, 100,000 runs: 98 ms with the sum in the race, 64 ms without (and
+// with the features looked at only when a variable or the time feature
+// changes).
 //
 // Theta.  theta depends only on the run's features (the class one-hot
 // aside) and the parameter block; a thread keeps its last features and
@@ -102,11 +110,15 @@ static __device__ __forceinline__ uint32_t theta_hash(uint32_t k0, uint32_t k1, 
     return h;
 }
 
-// true: mfac holds the cached factors of the features.  *slot: an entry the
+// hit: m holds the cached factors of the features; else slot is an entry the
 // caller may claim for them after computing the factors (~0u: none).
-static __device__ __noinline__ bool theta_lookup(const IsParams &ip, uint32_t k0, uint32_t k1, uint32_t k2,
-                                                 float (&mfac)[CSMC_MLP_CLASSES], uint32_t &slot) {
-    slot = ~0u;
+struct ThetaEntry {
+    float4 m;
+    uint32_t slot;
+    bool hit;
+};
+static __device__ __noinline__ ThetaEntry theta_lookup(const IsParams &ip, uint32_t k0, uint32_t k1, uint32_t k2) {
+    ThetaEntry r{make_float4(0.0f, 0.0f, 0.0f, 0.0f), ~0u, false};
     const uint32_t gen = ip.cache_gen;
     uint32_t i = theta_hash(k0, k1, k2) & ip.cache_mask;
     for (uint32_t probe = 0; probe < kThetaProbes; ++probe, i = (i + 1u) & ip.cache_mask) {
@@ -115,24 +127,21 @@ static __device__ __noinline__ bool theta_lookup(const IsParams &ip, uint32_t k0
         if (st == gen) {
             const uint4 a = *reinterpret_cast<const uint4 *>(e);
             if (a.y == k0 && a.z == k1 && a.w == k2) {
-                const uint4 m = *reinterpret_cast<const uint4 *>(e + 4);
-                mfac[0] = __uint_as_float(m.x);
-                mfac[1] = __uint_as_float(m.y);
-                mfac[2] = __uint_as_float(m.z);
-                mfac[3] = __uint_as_float(m.w);
-                return true;
+                r.m = *reinterpret_cast<const float4 *>(e + 4);
+                r.hit = true;
+                return r;
             }
             continue;
         }
         if (st == (gen | kThetaBusy)) continue;  // being written (its key unknown yet)
-        slot = i;                                // free for this generation
-        return false;
+        r.slot = i;                              // free for this generation
+        return r;
     }
-    return false;
+    return r;
 }
 
 static __device__ __noinline__ void theta_insert(const IsParams &ip, uint32_t slot, uint32_t k0, uint32_t k1,
-                                                 uint32_t k2, const float (&mfac)[CSMC_MLP_CLASSES]) {
+                                                 uint32_t k2, float4 m) {
     const uint32_t gen = ip.cache_gen;
     uint32_t *e = ip.theta_cache + static_cast<size_t>(slot) * CSMC_THETA_CACHE_WORDS;
     const uint32_t old = ld_acquire_u32(e);
@@ -141,9 +150,7 @@ static __device__ __noinline__ void theta_insert(const IsParams &ip, uint32_t sl
     e[1] = k0;
     e[2] = k1;
     e[3] = k2;
-    *reinterpret_cast<uint4 *>(e + 4) =
-        make_uint4(__float_as_uint(mfac[0]), __float_as_uint(mfac[1]), __float_as_uint(mfac[2]),
-                   __float_as_uint(mfac[3]));
+    *reinterpret_cast<float4 *>(e + 4) = m;
     st_release_u32(e, gen);
 }
 
@@ -248,20 +255,18 @@ struct IsCodedView : CodedView {
 };
 
 // Per thread and group: the step's 1/rate and 1/rate' bits and the rate
-// change 1/inv' - 1/inv (FP64, as two words); element i at [i * T].
+// change 1/inv' - 1/inv (FP64); 16 bytes.
 struct GroupRates {
-    uint32_t *w;  // this thread's group 0 word 0; group gi word j at [(4 gi + j) * T]
+    uint32_t *w;  // this thread's group 0; group gi: 1/rate at [2 gi T], 1/rate' at [(2 gi + 1) T]
+    double *d;    // this thread's group 0 rate change; group gi at [gi T]
     uint32_t T;
-    __device__ __forceinline__ float inv(uint32_t gi) const { return __uint_as_float(w[(4u * gi) * T]); }
-    __device__ __forceinline__ float invp(uint32_t gi) const { return __uint_as_float(w[(4u * gi + 1u) * T]); }
-    __device__ __forceinline__ double diff(uint32_t gi) const {
-        return __hiloint2double(static_cast<int>(w[(4u * gi + 3u) * T]), static_cast<int>(w[(4u * gi + 2u) * T]));
-    }
+    __device__ __forceinline__ float inv(uint32_t gi) const { return __uint_as_float(w[(2u * gi) * T]); }
+    __device__ __forceinline__ float invp(uint32_t gi) const { return __uint_as_float(w[(2u * gi + 1u) * T]); }
+    __device__ __forceinline__ double diff(uint32_t gi) const { return d[gi * T]; }
     __device__ __forceinline__ void set(uint32_t gi, float inv, float invp, double diff) const {
-        w[(4u * gi) * T] = __float_as_uint(inv);
-        w[(4u * gi + 1u) * T] = __float_as_uint(invp);
-        w[(4u * gi + 2u) * T] = static_cast<uint32_t>(__double2loint(diff));
-        w[(4u * gi + 3u) * T] = static_cast<uint32_t>(__double2hiint(diff));
+        w[(2u * gi) * T] = __float_as_uint(inv);
+        w[(2u * gi + 1u) * T] = __float_as_uint(invp);
+        d[gi * T] = diff;
     }
 };
 
@@ -314,9 +319,8 @@ static __device__ __forceinline__ void is_take(IsBest &b, unsigned long long key
 
 // One component's part in the race and in its lane's partial sum.  cb:
 // 255 minus the component's bit-reversed index, the low byte of its group
-// key.  ALLG: every component is a group member (no descriptor path, no
-// padding).
-template <bool ALLG, uint32_t k>
+// key.
+template <uint32_t k>
 static __device__ __forceinline__ void is_member(const Net &n, const IsCodedView &rv, const GroupRates &gr,
                                                  uint32_t NG, uint32_t tilt_mask, const float (&mfac)[CSMC_MLP_CLASSES],
                                                  uint32_t wd, uint32_t cc, uint32_t x, uint32_t cb, IsBest &best,
@@ -324,7 +328,7 @@ static __device__ __forceinline__ void is_member(const Net &n, const IsCodedView
     const uint32_t b = (wd >> (8u * k)) & 0xffu;
     const uint32_t code = b >> 5;
     const uint32_t T = rv.T;
-    if (ALLG || code < NG) {
+    if (code < NG) {
         const uint32_t key = (x & 0xffffff00u) | cb;
         uint32_t *pp = rv.kp + (code * 4u + k) * T;
         *pp = max(*pp, key);
@@ -342,10 +346,12 @@ static __device__ __forceinline__ void is_member(const Net &n, const IsCodedView
 
 // The full race under the tilt, one delay per component (the decision of
 // lane_race); used where the groups' largest keys do not decide the step.
-static __device__ __noinline__ void is_race_exact(const Net &n, uint32_t C, uint32_t bits, const IsCodedView &rv,
-                                                  const GroupRates &gr, uint32_t NG,
-                                                  const float (&mfac)[CSMC_MLP_CLASSES], uint64_t seed, uint64_t run,
-                                                  uint32_t step, IsBest &best) {
+static __device__ __noinline__ IsBest is_race_exact(const uint8_t *base, IsCodedView rv, GroupRates gr, uint32_t NG,
+                                                    float4 m, uint64_t seed, uint64_t run, uint32_t step) {
+    const Net n = net_view(base);
+    const uint32_t C = n.n_comps, bits = ceil_log2(C);
+    const float mfac[CSMC_MLP_CLASSES] = {m.x, m.y, m.z, m.w};
+    IsBest best;
     best.key = ~0ull;
     best.d = best.inv = best.invp = 0.0f;
     best.tilted = false;
@@ -374,6 +380,7 @@ static __device__ __noinline__ void is_race_exact(const Net &n, uint32_t C, uint
                     tl);
         }
     }
+    return best;
 }
 
 // One merge step of the butterfly stack: leaf i (0..31, lanes in 5-bit
@@ -395,7 +402,6 @@ static __device__ __forceinline__ void tree_push(uint32_t i, double v, double (&
 // The step's race and sum of rate changes.  Returns false when the groups'
 // keys do not decide the race (the caller runs is_race_exact); `sum` is
 // valid either way.
-template <bool ALLG>
 static __device__ __forceinline__ bool is_race_coded(const Net &n, uint32_t C, uint32_t bits, uint32_t NG,
                                                      uint32_t tilt_mask, const IsCodedView &rv, const GroupRates &gr,
                                                      const float (&mfac)[CSMC_MLP_CLASSES], const PhiloxKeys &K,
@@ -418,10 +424,10 @@ static __device__ __forceinline__ bool is_race_coded(const Net &n, uint32_t C, u
             const uint32_t wd = rv.lw[q * T], cc = 4u * q;
             const uint32_t rq = hi_shift ? (__brev(q) >> (32u - hi_shift)) : 0u;
             const uint32_t cb = 255u - rq;
-            is_member<ALLG, 0>(n, rv, gr, NG, tilt_mask, mfac, wd, cc, blk.x, cb, best, part);
-            is_member<ALLG, 1>(n, rv, gr, NG, tilt_mask, mfac, wd, cc + 1u, blk.y, cb - (2u << hi_shift), best, part);
-            is_member<ALLG, 2>(n, rv, gr, NG, tilt_mask, mfac, wd, cc + 2u, blk.z, cb - (1u << hi_shift), best, part);
-            is_member<ALLG, 3>(n, rv, gr, NG, tilt_mask, mfac, wd, cc + 3u, blk.w, cb - (3u << hi_shift), best, part);
+            is_member<0>(n, rv, gr, NG, tilt_mask, mfac, wd, cc, blk.x, cb, best, part);
+            is_member<1>(n, rv, gr, NG, tilt_mask, mfac, wd, cc + 1u, blk.y, cb - (2u << hi_shift), best, part);
+            is_member<2>(n, rv, gr, NG, tilt_mask, mfac, wd, cc + 2u, blk.z, cb - (1u << hi_shift), best, part);
+            is_member<3>(n, rv, gr, NG, tilt_mask, mfac, wd, cc + 3u, blk.w, cb - (3u << hi_shift), best, part);
         }
         tree_push(i, part, stack, sum);
     }
@@ -464,6 +470,99 @@ static __device__ __forceinline__ bool is_race_coded(const Net &n, uint32_t C, u
     return true;
 }
 
+// The race where every component is a group member (no descriptor path, no
+// padding): a block's four key words are loaded before any is stored (as in
+// race_block), the sum of rate changes is group_rate_sum's, and one flat-spot
+// check covers the winner.  Returns false when is_race_exact has to decide.
+static __device__ __forceinline__ bool is_race_grouped(uint32_t C, uint32_t bits, uint32_t NG, const IsCodedView &rv,
+                                                       const GroupRates &gr, const PhiloxKeys &K, uint64_t run,
+                                                       uint32_t step, IsBest &best) {
+    const uint32_t T = rv.T, chain = 4u * T, group = 16u * T;
+    for (uint32_t w = 0; w < 4u * NG; ++w) st_key(rv.keys + w * chain, 0u);
+    best.key = ~0ull;
+    best.d = best.inv = best.invp = 0.0f;
+    best.tilted = false;
+    const PhiloxStep ps = philox_step(K, step, run);
+    const uint32_t hi_shift = bits - 2u;  // bits >= 2: at least four components
+    const uint32_t Q = C >> 2;
+#pragma unroll kCodedUnroll
+    for (uint32_t q = 0; q < Q; ++q) {
+        const uint32_t wd = rv.lw[q * T];
+        const u32x4 x = philox_block(K, ps, q);
+        const uint32_t cb = 255u - (hi_shift ? (__brev(q) >> (32u - hi_shift)) : 0u);
+        const uint32_t a0 = rv.keys + ((wd >> 5) & 7u) * group, a1 = rv.keys + ((wd >> 13) & 7u) * group + chain,
+                       a2 = rv.keys + ((wd >> 21) & 7u) * group + 2u * chain,
+                       a3 = rv.keys + (wd >> 29) * group + 3u * chain;
+        const uint32_t o0 = ld_key(a0), o1 = ld_key(a1), o2 = ld_key(a2), o3 = ld_key(a3);
+        st_key(a0, max(o0, (x.x & 0xffffff00u) | cb));
+        st_key(a1, max(o1, (x.y & 0xffffff00u) | cb));
+        st_key(a2, max(o2, (x.z & 0xffffff00u) | cb));
+        st_key(a3, max(o3, (x.w & 0xffffff00u) | cb));
+    }
+    // each group races with its largest key under its tilted 1/rate
+    uint32_t inf_groups = 0, wtop = 0, wg = 0;
+    bool tie = false, from_group = false;
+#pragma unroll
+    for (uint32_t g = 0; g < CSMC_IS_GROUPS; ++g) {
+        if (g >= NG) continue;
+        const uint32_t kg = rv.keys + g * group;
+        const uint32_t o0 = ld_key(kg), o1 = ld_key(kg + chain), o2 = ld_key(kg + 2u * chain), o3 = ld_key(kg + 3u * chain);
+        // no chain key is 0 (its low byte is 255 minus at most 63)
+        if ((o0 | o1 | o2 | o3) == 0u) continue;
+        const uint32_t a = max(max(o0, o1 ? o1 - (2u << hi_shift) : 0u),
+                               max(o2 ? o2 - (1u << hi_shift) : 0u, o3 ? o3 - (3u << hi_shift) : 0u));
+        const float invp = gr.invp(g);
+        if (!(invp > 0.0f)) return false;  // delays 0, negative or NaN for the whole group
+        if (!(invp <= 3.40282347e38f)) {    // +inf: the group's delays are +inf (NaN at u = 1)
+            inf_groups |= 1u << g;
+            continue;
+        }
+        const float d1 = exp_delay(a & 0xffffff00u, invp);
+        const uint32_t hi = f_bits(d1) | 0x80000000u;  // delay_key of d1 >= 0
+        const unsigned long long key = (static_cast<unsigned long long>(hi) << 32) | (255u - (a & 255u));
+        const bool eq = hi == static_cast<uint32_t>(best.key >> 32);
+        tie |= eq;
+        if (key < best.key) {
+            tie = eq;
+            best.key = key;
+            best.d = d1;
+            best.invp = invp;
+            wtop = a >> 8;
+            wg = g;
+            from_group = true;
+        }
+    }
+    if (tie) return false;
+    if (from_group && wtop > 0u && exp_delay((wtop - 1u) << 8, best.invp) == best.d) return false;
+    if (inf_groups && static_cast<uint32_t>(best.key >> 32) >= delay_key(__uint_as_float(0x7f800000u))) return false;
+    best.inv = gr.inv(wg);
+    best.tilted = tiltable(best.inv);
+    return true;
+}
+
+// The sum of rate changes of lane j's run by the whole warp, in the
+// one-warp-per-run kernel's own order: lane L sums the members of blocks L,
+// L + 32, .. (words of lane j's state), then the butterfly.  A run's sum
+// changes only when it moves a component or its groups' rates change (about
+// one step in six of an epidemic), so the warp evaluates it for the lanes
+// that need it instead of every lane adding its components on every step.
+// ds: byte distance from this lane's state to lane j's, per 4-byte word.
+static __device__ __forceinline__ double group_rate_sum(uint32_t C, const IsCodedView &rv, const GroupRates &gr,
+                                                        uint32_t tilt_mask, int ds) {
+    const uint32_t lane = threadIdx.x & 31u, T = rv.T;
+    double part = 0.0;
+    for (uint32_t q = lane; 4u * q < C; q += 32u) {
+        const uint32_t wd = rv.lw[static_cast<int>(q * T) + ds];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t code = (wd >> (8u * k + 5u)) & 7u;
+            const double v = gr.d[static_cast<int>(code * T) + ds];
+            if ((tilt_mask >> code) & 1u) part = d_add(part, v);
+        }
+    }
+    return warp_sum_d(part);
+}
+
 template <bool SLOTS, bool ALLG>
 __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_CTAS_PER_SM)
     is_coded_kernel(const __grid_constant__ IsParams ip) {
@@ -478,7 +577,7 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
     uint8_t *h1_base = smem + p.blob_bytes + kMlpExactBytes;
     float *h1s = reinterpret_cast<float *>(h1_base) + (t >> 5) * (kThetaBatch * CSMC_MLP_HID * CSMC_MLP_CLASSES);
     uint8_t *slab = h1_base + (T >> 5) * (4u * kThetaBatch * CSMC_MLP_HID * CSMC_MLP_CLASSES);
-    const GroupRates gr{reinterpret_cast<uint32_t *>(slab) + t, T};
+    const GroupRates gr{reinterpret_cast<uint32_t *>(slab + 8u * NG * T) + t, reinterpret_cast<double *>(slab) + t, T};
     const bool recv = (p.net.recv_lo | p.net.recv_hi) != 0;
     IsCodedView rv;
     static_cast<CodedView &>(rv) = carve_coded_view(slab + 16u * NG * T, V, P, C, 16u * NG * T, recv, T, t);
@@ -502,9 +601,15 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
     // the last evaluated features (BF16 bits of x[4..9], packed in pairs)
     // and their class factors, kept across steps and runs
     uint32_t lk0 = 0, lk1 = 0, lk2 = 0;
+    uint32_t fk0 = 0, fk1 = 0, fk2 = 0;  // this step's
     bool theta_valid = false;
     float mfac[CSMC_MLP_CLASSES] = {1.0f, 1.0f, 1.0f, 1.0f};
     bool rates_changed = true;  // the groups' rates need a new look
+    uint32_t tilt_mask = 0;     // groups whose members are tilted
+    bool new_feat = true;       // a variable that feeds the features may have changed
+    float t_next = 0.0f;        // first time whose time feature differs
+    bool sum_stale = true;      // ALLG: the sum of rate changes below is out of date
+    double rate_sum = 0.0;
     uint32_t gvalid = 0;        // groups whose GroupRates entry has been written
     // the last tilted winner's 1/rate and 1/rate' bits and its log term
     uint32_t w_inv = 0xffffffffu, w_invp = 0xffffffffu;
@@ -532,6 +637,8 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
                     step = 0;
                     logw = 0.0;
                     stale = true;
+                    new_feat = true;
+                    sum_stale = true;
                 }
             }
         }
@@ -553,37 +660,50 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
             }
         }
 
-        // ---- receivers and the rate table (this thread's run)
-        uint32_t fk0 = 0, fk1 = 0, fk2 = 0;
+        // ---- receivers and the rate table (this thread's run), then the
+        // features: the variables' only after a step that can have changed
+        // one, time's when it passes the next of its 64 edges
         bool need_theta = false;
         if (have) {
-            if (run_receivers<false, SLOTS>(n, C, V, rv, sc, p.seed, p.var_id, run, step)) stale = true;
+            if (run_receivers<false, SLOTS>(n, C, V, rv, sc, p.seed, p.var_id, run, step)) {
+                stale = true;
+                sum_stale = true;
+            }
             if (rate_table && stale) {
                 for (uint32_t j = 0; j < P; ++j) rv.rates[j] = inv_rate(eval(n, rv.vars, n.rate_prog[j]));
                 rates_changed = true;
             }
+            new_feat |= stale;
             stale = false;
-            float v4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (new_feat || time >= t_next) {
+                float v4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (F.var[i] >= 0) v4[i] = rv.vars[F.var[i]];
-            const float clk = F.clock_var >= 0 ? rv.vars[F.clock_var] : 0.0f;
-            float x[CSMC_MLP_IN];
-            mlp_features(0, F, v4, clk, time, p.horizon, x);
-            fk0 = (f_bits(x[4]) >> 16) | (f_bits(x[5]) & 0xffff0000u);
-            fk1 = (f_bits(x[6]) >> 16) | (f_bits(x[7]) & 0xffff0000u);
-            fk2 = (f_bits(x[8]) >> 16) | (f_bits(x[9]) & 0xffff0000u);
-            need_theta = !theta_valid || fk0 != lk0 || fk1 != lk1 || fk2 != lk2;
+                for (int i = 0; i < 4; ++i)
+                    if (F.var[i] >= 0) v4[i] = rv.vars[F.var[i]];
+                const float clk = F.clock_var >= 0 ? rv.vars[F.clock_var] : 0.0f;
+                float x[CSMC_MLP_IN];
+                mlp_features(0, F, v4, clk, time, p.horizon, x);
+                fk0 = (f_bits(x[4]) >> 16) | (f_bits(x[5]) & 0xffff0000u);
+                fk1 = (f_bits(x[6]) >> 16) | (f_bits(x[7]) & 0xffff0000u);
+                fk2 = (f_bits(x[8]) >> 16) | (f_bits(x[9]) & 0xffff0000u);
+                const uint32_t k = static_cast<uint32_t>(f_mul(x[9], CSMC_MLP_TIME_STEPS));  // exact: x[9] = k / 64
+                t_next = ip.time_edge[min(k, 64u)];
+                new_feat = false;
+                need_theta = !theta_valid || fk0 != lk0 || fk1 != lk1 || fk2 != lk2;
+            }
         }
 
         // ---- theta for the lanes whose features changed: the cache, then
         // one distinct feature vector at a time evaluated by the whole warp
         uint32_t slot = ~0u;
         if (need_theta && ip.theta_cache) {
-            float mc[CSMC_MLP_CLASSES];
-            if (theta_lookup(ip, fk0, fk1, fk2, mc, slot)) {
-#pragma unroll
-                for (uint32_t l = 0; l < CSMC_MLP_CLASSES; ++l) mfac[l] = mc[l];
+            const ThetaEntry te = theta_lookup(ip, fk0, fk1, fk2);
+            slot = te.slot;
+            if (te.hit) {
+                mfac[0] = te.m.x;
+                mfac[1] = te.m.y;
+                mfac[2] = te.m.z;
+                mfac[3] = te.m.w;
                 lk0 = fk0;
                 lk1 = fk1;
                 lk2 = fk2;
@@ -609,35 +729,53 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
                 theta_valid = true;
                 need_theta = false;
                 rates_changed = true;
-                if (static_cast<int>(lane) == j && slot != ~0u) theta_insert(ip, slot, fk0, fk1, fk2, mfac);
+                if (static_cast<int>(lane) == j && slot != ~0u) 
+                    theta_insert(ip, slot, fk0, fk1, fk2, make_float4(mfac[0], mfac[1], mfac[2], mfac[3]));
             }
             pend &= ~__ballot_sync(kFullWarp, mine);
         }
-        if (!have) continue;
 
         // ---- the groups' tilted rates and rate changes
-        uint32_t tilt_mask = 0;
-        for (uint32_t g = 0; g < NG; ++g) {
-            const uint32_t sg = ip.group_src[g];
-            const float inv = (sg & CSMC_CLASS_SRC_PROG) ? rv.rates[sg & 0xffffu] : __uint_as_float(sg);
-            const bool tl = tiltable(inv);
-            tilt_mask |= tl ? (1u << g) : 0u;
-            if (rates_changed) {
+        if (have && rates_changed) {
+            tilt_mask = 0;
+            for (uint32_t g = 0; g < NG; ++g) {
+                const uint32_t sg = ip.group_src[g];
+                const float inv = (sg & CSMC_CLASS_SRC_PROG) ? rv.rates[sg & 0xffffu] : __uint_as_float(sg);
+                const bool tl = tiltable(inv);
+                tilt_mask |= tl ? (1u << g) : 0u;
                 const float invp = tl ? f_mul(inv, mfac_of(mfac, (ip.group_l >> (2u * g)) & 3u)) : inv;
                 if (!((gvalid >> g) & 1u) || __float_as_uint(inv) != __float_as_uint(gr.inv(g)) ||
                     __float_as_uint(invp) != __float_as_uint(gr.invp(g))) {
                     gr.set(g, inv, invp, tl ? rate_change(inv, invp) : 0.0);
                     gvalid |= 1u << g;
+                    sum_stale = true;
                 }
             }
+            rates_changed = false;
         }
-        rates_changed = false;
+        if constexpr (ALLG) {
+            __syncwarp();  // the states' words and rates are read across the warp
+            unsigned todo = __ballot_sync(kFullWarp, have && sum_stale);
+            while (todo) {
+                const int j = __ffs(todo) - 1;
+                const double v = group_rate_sum(C, rv, gr, __shfl_sync(kFullWarp, tilt_mask, j), j - static_cast<int>(lane));
+                if (static_cast<int>(lane) == j) {
+                    rate_sum = v;
+                    sum_stale = false;
+                }
+                todo &= todo - 1;
+            }
+        }
+        if (!have) continue;
 
         // ---- the race, the log-likelihood ratio, the winner's transition
         IsBest best;
-        double rsum;
-        if (!is_race_coded<ALLG>(n, C, bits, NG, tilt_mask, rv, gr, mfac, p.keys, run, step, best, rsum))
-            is_race_exact(n, C, bits, rv, gr, NG, mfac, p.seed, run, step, best);
+        double rsum = rate_sum;
+        bool decided;
+        if constexpr (ALLG) decided = is_race_grouped(C, bits, NG, rv, gr, p.keys, run, step, best);
+        else decided = is_race_coded(n, C, bits, NG, tilt_mask, rv, gr, mfac, p.keys, run, step, best, rsum);
+        if (!decided)
+            best = is_race_exact(n.base, rv, gr, NG, make_float4(mfac[0], mfac[1], mfac[2], mfac[3]), p.seed, run, step);
         const uint32_t win = bitrev_bits(static_cast<uint32_t>(best.key & 0xffffffffull), bits);
         const float dmin = best.d;
         const bool finite = static_cast<double>(dmin) < kDblMax;
@@ -658,6 +796,7 @@ __global__ void __launch_bounds__(CSMC_IS_CODED_MAX_THREADS, CSMC_IS_CODED_MIN_C
         const bool took = run_commit<false, SLOTS>(n, p.net.n_clocks, rv, sc, p.seed, p.var_id, run, step, time, win,
                                                    dmin);
         stale = took || (p.net.n_clocks > 0 && finite);
+        sum_stale |= took;
     }
     if (acc_hits) atomicAdd(p.scratch + 1, acc_hits);
     if (acc_steps) atomicAdd(p.scratch + 2, acc_steps);
