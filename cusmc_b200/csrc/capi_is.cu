@@ -396,64 +396,87 @@ namespace {
 constexpr int kGradFloats = CSMC_MLP_HID * CSMC_MLP_IN + CSMC_MLP_HID * CSMC_MLP_HID + 3 * CSMC_MLP_HID + 1;
 static_assert(kGradFloats == CSMC_MLP_GRAD_FLOATS, "gradient layout of include/csmc.h");
 
-// Sums the per-CTA gradient partials of mlp_tc_kernel<1> into the gradient
-// (layout w1[64][16], b1[64], w2[64][64], b2[64], w3[64], b3; one thread per
-// entry, CTAs in order, FP64) and the per-CTA objectives into J.  A CTA's
-// partial block holds D4 = [dZ2 | dZ1]^T . [H1 | X | 1] (128 rows of 96:
-// row k < 64 is output unit k of layer 2, row 64 + j is unit j of layer 1;
-// columns 0..63 H1, 64..79 X, 80 the bias input), then dw3[64] and db3.
-__global__ void reduce_mlp_partials(const float *partials, const double *objective, int grid, int pf, float *grad,
-                                    double *J) {
+// Where entry k of the gradient (layout w1[64][16], b1[64], w2[64][64],
+// b2[64], w3[64], b3) lies in a CTA's partial block: D4 = [dZ2 | dZ1]^T .
+// [H1 | X | 1] (128 rows of 96: row k < 64 is output unit k of layer 2, row
+// 64 + j is unit j of layer 1; columns 0..63 H1, 64..79 X, 80 the bias input),
+// then dw3[64] and db3.
+__device__ __forceinline__ int partial_of(int k) {
     constexpr int H = CSMC_MLP_HID, I = CSMC_MLP_IN, N4 = 96;
-    const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (k < kGradFloats) {
-        int src;
-        if (k < H * I) src = (64 + k / I) * N4 + 64 + k % I;                       // dW1[j][i]
-        else if (k < H * I + H) src = (64 + (k - H * I)) * N4 + 80;               // db1[j]
-        else if (k < H * I + H + H * H) src = ((k - H * I - H) / H) * N4 + (k - H * I - H) % H;  // dW2[k][j]
-        else if (k < H * I + 2 * H + H * H) src = (k - H * I - H - H * H) * N4 + 80;             // db2[k]
-        else if (k < H * I + 3 * H + H * H) src = 128 * N4 + (k - H * I - 2 * H - H * H);        // dw3[k]
-        else src = 128 * N4 + 64;                                                                // db3
-        double acc = 0.0;
-        for (int c = 0; c < grid; ++c) acc = csmc::d_add(acc, static_cast<double>(partials[c * pf + src]));
-        grad[k] = static_cast<float>(acc);
-    }
-    if (k == 0) {
-        double s = 0.0;
-        for (int c = 0; c < grid; ++c) s = csmc::d_add(s, objective[c]);
-        *J = s;
-    }
+    if (k < H * I) return (64 + k / I) * N4 + 64 + k % I;                                    // dW1[j][i]
+    if (k < H * I + H) return (64 + (k - H * I)) * N4 + 80;                                  // db1[j]
+    if (k < H * I + H + H * H) return ((k - H * I - H) / H) * N4 + (k - H * I - H) % H;      // dW2[k][j]
+    if (k < H * I + 2 * H + H * H) return (k - H * I - H - H * H) * N4 + 80;                 // db2[k]
+    if (k < H * I + 3 * H + H * H) return 128 * N4 + (k - H * I - 2 * H - H * H);            // dw3[k]
+    return 128 * N4 + 64;                                                                    // db3
 }
 
-// FP32 master vector -> the BF16 parameter block, the host packing's layout
-// (w1 and w2 rounded to BF16, biases and the output layer FP32, padding
-// zero); one thread per entry.
-__global__ void mlp_pack_params(const float *x, csmc::MlpParams *P) {
-    constexpr int H = CSMC_MLP_HID, I = CSMC_MLP_IN;
+// Entry k of the gradient: the CTAs' partials in order, FP64.  The loads are
+// independent of the sum: 37 in flight (148 CTAs in four rounds).
+__device__ __forceinline__ float partial_sum(const float *partials, int grid, int pf, int k) {
+    const float *p = partials + partial_of(k);
+    double acc = 0.0;
+#pragma unroll 37
+    for (int c = 0; c < grid; ++c) acc = csmc::d_add(acc, static_cast<double>(p[static_cast<size_t>(c) * pf]));
+    return static_cast<float>(acc);
+}
+
+__device__ __forceinline__ double objective_sum(const double *objective, int grid) {
+    double s = 0.0;
+#pragma unroll 37
+    for (int c = 0; c < grid; ++c) s = csmc::d_add(s, objective[c]);
+    return s;
+}
+
+constexpr int kEntryThreads = 64;  // threads per CTA of the per-entry kernels: 84 CTAs, so the loads come from many SMs
+constexpr int kEntryBlocks = (kGradFloats + 3 + kEntryThreads - 1) / kEntryThreads;
+
+// The gradient (one thread per entry) and the objective J.
+__global__ void reduce_mlp_partials(const float *partials, const double *objective, int grid, int pf, float *grad,
+                                    double *J) {
     const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (k < H * I) (&P->w1[0][0])[k] = csmc::f_to_bf16(x[k]);
-    else if (k < H * I + H) P->b1[k - H * I] = x[k];
-    else if (k < H * I + H + H * H) (&P->w2[0][0])[k - H * I - H] = csmc::f_to_bf16(x[k]);
-    else if (k < H * I + 2 * H + H * H) P->b2[k - H * I - H - H * H] = x[k];
-    else if (k < H * I + 3 * H + H * H) P->w3[k - H * I - 2 * H - H * H] = x[k];
-    else if (k < kGradFloats) P->b3 = x[k];
+    if (k < kGradFloats) grad[k] = partial_sum(partials, grid, pf, k);
+    if (k == kGradFloats) *J = objective_sum(objective, grid);
+}
+
+// Entry k of the FP32 master vector into the BF16 parameter block, the host
+// packing's layout (w1 and w2 rounded to BF16, biases and the output layer
+// FP32, padding zero).
+__device__ __forceinline__ void pack_entry(int k, float x, csmc::MlpParams *P) {
+    constexpr int H = CSMC_MLP_HID, I = CSMC_MLP_IN;
+    if (k < H * I) (&P->w1[0][0])[k] = csmc::f_to_bf16(x);
+    else if (k < H * I + H) P->b1[k - H * I] = x;
+    else if (k < H * I + H + H * H) (&P->w2[0][0])[k - H * I - H] = csmc::f_to_bf16(x);
+    else if (k < H * I + 2 * H + H * H) P->b2[k - H * I - H - H * H] = x;
+    else if (k < H * I + 3 * H + H * H) P->w3[k - H * I - 2 * H - H * H] = x;
+    else if (k < kGradFloats) P->b3 = x;
     else if (k < kGradFloats + 3) P->pad[k - kGradFloats] = 0.0f;
+}
+__global__ void mlp_pack_params(const float *x, csmc::MlpParams *P) {
+    const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    pack_entry(k, k < kGradFloats ? x[k] : 0.0f, P);
 }
 
 // One Adam ascent step per entry (csmc_mlp_adam's formulas, every operation
-// an IEEE double operation rounded to nearest, x rounded to FP32).
-__global__ void mlp_adam_ascend(float *x, double *m, double *v, const float *g, double lr, double c1, double c2) {
+// an IEEE double operation rounded to nearest, x rounded to FP32) from the
+// gradient kernel's partials, and the parameter block of the next step: one
+// launch between two gradients.
+__global__ void mlp_adam_ascend(const float *partials, const double *objective, int grid, int pf, float *x, double *m,
+                                double *v, double lr, double c1, double c2, csmc::MlpParams *P, double *J) {
     constexpr double b1 = 0.9, b2 = 0.999, eps = 1e-8;
     const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k == kGradFloats) *J = objective_sum(objective, grid);
     if (k >= kGradFloats) return;
-    const double gi = static_cast<double>(g[k]);
+    const double gi = static_cast<double>(partial_sum(partials, grid, pf, k));
     const double mk = csmc::d_add(csmc::d_mul(b1, m[k]), csmc::d_mul(1.0 - b1, gi));
     const double vk = csmc::d_add(csmc::d_mul(b2, v[k]), csmc::d_mul(csmc::d_mul(1.0 - b2, gi), gi));
     m[k] = mk;
     v[k] = vk;
     const double mh = csmc::d_div(mk, c1), vh = csmc::d_div(vk, c2);
     const double up = csmc::d_div(csmc::d_mul(lr, mh), csmc::d_add(csmc::d_sqrt(vh), eps));
-    x[k] = static_cast<float>(csmc::d_add(static_cast<double>(x[k]), up));
+    const float xk = static_cast<float>(csmc::d_add(static_cast<double>(x[k]), up));
+    x[k] = xk;
+    pack_entry(k, xk, P);
 }
 
 // Device buffers of the proposal-network kernels, one set per device, kept
@@ -537,8 +560,7 @@ int mlp_common(int mode, const void *params, const void *rows, uint64_t n_rows, 
     double J = 0.0;
     CK(cudaMemcpyAsync(&err, m.error, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
     if (mode == 1) {
-        reduce_mlp_partials<<<(kGradFloats + 255) / 256, 256, 0, st>>>(m.partials, m.objective, grid, pf, m.grad,
-                                                                        m.J);
+        reduce_mlp_partials<<<kEntryBlocks, kEntryThreads, 0, st>>>(m.partials, m.objective, grid, pf, m.grad, m.J);
         CK(cudaGetLastError(), "gradient reduction launch");
         CK(cudaMemcpyAsync(grad, m.grad, kGradFloats * sizeof(float), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         CK(cudaMemcpyAsync(&J, m.J, sizeof(double), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
@@ -569,21 +591,19 @@ int mlp_adam(const void *rows, uint64_t n_rows, int32_t steps, double lr, float 
     CK(cudaMemcpyAsync(m.x, x, xb, cudaMemcpyHostToDevice, st), "upload master vector");
     CK(cudaMemcpyAsync(m.moments, mom1, mb, cudaMemcpyHostToDevice, st), "upload moments");
     CK(cudaMemcpyAsync(m.moments + kGradFloats, mom2, mb, cudaMemcpyHostToDevice, st), "upload moments");
-    constexpr int kThreads = 256, kBlocks = (kGradFloats + 3 + kThreads - 1) / kThreads;
     int32_t tt = *t;
+    mlp_pack_params<<<kEntryBlocks, kEntryThreads, 0, st>>>(m.x, m.P);
+    CK(cudaGetLastError(), "parameter packing launch");
     for (int32_t s = 0; s < steps; ++s) {
-        mlp_pack_params<<<kBlocks, kThreads, 0, st>>>(m.x, m.P);
-        CK(cudaGetLastError(), "parameter packing launch");
         rc = csmc::mlp_tc_launch(1, static_cast<const csmc::MlpRow *>(rows), n_rows, m.P, nullptr, m.partials,
                                  m.objective, m.error, grid, st);
         if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "tensor-core kernel launch");
-        reduce_mlp_partials<<<(kGradFloats + 255) / 256, 256, 0, st>>>(m.partials, m.objective, grid, pf, m.grad,
-                                                                        m.Js + (s == 0 ? 0 : 1));
-        CK(cudaGetLastError(), "gradient reduction launch");
         ++tt;
         const double c1 = 1.0 - std::pow(0.9, static_cast<double>(tt));
         const double c2 = 1.0 - std::pow(0.999, static_cast<double>(tt));
-        mlp_adam_ascend<<<kBlocks, kThreads, 0, st>>>(m.x, m.moments, m.moments + kGradFloats, m.grad, lr, c1, c2);
+        mlp_adam_ascend<<<kEntryBlocks, kEntryThreads, 0, st>>>(m.partials, m.objective, grid, pf, m.x, m.moments,
+                                                                m.moments + kGradFloats, lr, c1, c2, m.P,
+                                                                m.Js + (s == 0 ? 0 : 1));
         CK(cudaGetLastError(), "Adam step launch");
     }
     int err = 0;

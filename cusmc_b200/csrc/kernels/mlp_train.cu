@@ -19,12 +19,26 @@
 // GELU derivatives stay in the registers of the thread that computed them,
 // and the output layer's gradient is accumulated per thread in registers
 // and reduced once at the end in a fixed order (the gradient is
-// deterministic).  Operands live in shared memory in the no-swizzle K-major
-// canonical layout (8-row x 16-byte core matrices; core matrix (row group g,
-// K chunk c) at ((c * rows/8) + g) * 128 bytes), one thread issues the MMAs,
-// completion is signalled through an mbarrier, and every wait is bounded: on
-// a timeout the kernel records an error, waits (bounded) for its MMAs, frees
-// its tensor memory and returns.
+// deterministic).
+//
+// Operands live in shared memory without swizzle, in core matrices of 8 rows
+// x 16 bytes: tile F = [H1 | X | 1] and tile Z = [dZ2 | dZ1], 128 rows each,
+// core matrix (row group g, column chunk c) at (16 c + g) * 128 bytes.  The
+// layer MMAs read them K-major (columns are the contraction); the weight-
+// gradient MMA contracts over the rows and reads the same bytes MN-major, so
+// no transposed copy exists: a thread stores its sixteen columns of a layer as
+// two 16-byte words, rows next to each other.  F is double-buffered: the
+// weight-gradient MMA of a tile overlaps the next tile's first layer.
+//
+// One thread issues the MMAs, completion is signalled through an mbarrier
+// (the weight-gradient MMA's with the next tile's first), and every wait is
+// bounded: on a timeout the kernel records an error, skips its further waits,
+// waits (bounded) for its MMAs, frees its tensor memory and returns.
+//
+// What bounds it: the CUDA-core epilogues (two GELUs with their derivatives
+// per hidden unit and row); the tensor pipe is nearly idle.  Measured (B200):
+// 1e6 rows 613 us with transposed operand copies stored 2 bytes at a time
+// (2,830 instructions per warp and tile), see below for the present form.
 #include "../include/csmc_mlp.h"
 #include "sim.cuh"
 
@@ -41,21 +55,16 @@ constexpr uint32_t kTmemCols = 256;             // D1/D3 [0,64), D2 [64,128), D4
 constexpr uint32_t kColD1 = 0, kColD2 = 64, kColD4 = 128;
 constexpr int kN4 = 96;                         // [H1 (64) | X (16) | 1 | 0 x 15]
 
-// shared-memory carve-up (bytes).  The dZ2 tile (A3) reuses the H1 tile's
-// space (A2): the layer-2 MMA that reads A2 has completed before the
-// epilogue writes A3, and the next tile writes A2 only after the MMA that
-// reads A3 has completed.  The allocation extends far beyond the last
-// operand tile (kSmemBytes), so operand accesses stay inside it even under a
-// transposed reading of the descriptor strides.
-constexpr uint32_t kA1 = 0;                     // X tile      128 x 16
-constexpr uint32_t kB1 = kA1 + 128 * 16 * 2;    // W1          64 x 16
-constexpr uint32_t kA2 = kB1 + 64 * 16 * 2;     // H1 tile     128 x 64; later dZ2 (A3)
-constexpr uint32_t kA3 = kA2;
-constexpr uint32_t kB2 = kA2 + 128 * 64 * 2;    // W2          64 x 64 (out x in)
+// shared-memory carve-up (bytes)
+constexpr uint32_t kChunk = 128 * 16;           // one column chunk: 8 columns of 128 rows
+constexpr uint32_t kFBytes = (kN4 / 8) * kChunk;
+constexpr uint32_t kF = 0;                      // F tiles, two buffers: chunks 0..7 H1, 8..9 X, 10..11 [1 | 0]
+constexpr uint32_t kX = 8 * kChunk;             // X within F
+constexpr uint32_t kZ = kF + 2 * kFBytes;       // Z tile: chunks 0..7 dZ2, 8..15 dZ1
+constexpr uint32_t kB1 = kZ + 16 * kChunk;      // W1          64 x 16
+constexpr uint32_t kB2 = kB1 + 64 * 16 * 2;     // W2          64 x 64 (out x in)
 constexpr uint32_t kB3 = kB2 + 64 * 64 * 2;     // W2^T        64 x 64 (in x out)
-constexpr uint32_t kA4 = kB3 + 64 * 64 * 2;     // dZ^T        128 x 128 (neuron x row)
-constexpr uint32_t kB4 = kA4 + 128 * 128 * 2;   // F^T         96 x 128 (feature x row)
-constexpr uint32_t kTh = kB4 + kN4 * 128 * 2;   // theta partials [group][row] (floats)
+constexpr uint32_t kTh = kB3 + 64 * 64 * 2;     // theta partials [group][row] (floats)
 constexpr uint32_t kMisc = kTh + kGroups * 128 * 4;  // mbarrier, tmem address, biases, reductions
 constexpr uint32_t kMiscBytes = 4096;
 constexpr uint32_t kRedStride = 17;             // per-warp output-layer sums: 16 columns, db3
@@ -81,9 +90,11 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
            (static_cast<uint64_t>((sbo >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
 
-// instruction descriptor: FP32 accumulator, BF16 A and B, both K-major, M=128
-__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+// instruction descriptor: FP32 accumulator, BF16 A and B, M=128; both operands
+// K-major, or both MN-major
+__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t N, bool mn_major = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? (1u << 15) | (1u << 16) : 0u) | ((N >> 3) << 17) |
+           ((128u >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -131,18 +142,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void st_bf16(uint8_t *base, uint32_t off, float v) {
-    *reinterpret_cast<uint16_t *>(base + off) = f_to_bf16(v);
+// Two floats rounded to BF16 (to nearest even), the first in the low half.
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
-// Waits for the MMAs committed to mbar, block-uniformly: false when any
-// thread's bounded wait gave up.
-__device__ __forceinline__ bool wait_all(uint32_t mbar, uint32_t &phase) {
-    const int mine = mbar_wait(mbar, phase) ? 1 : 0;
-    phase ^= 1u;
-    const bool all = __syncthreads_and(mine) != 0;
-    tc_after_sync();
-    return all;
+// Stores this thread's sixteen columns (chunks c and c + 1) of row r.
+__device__ __forceinline__ void st_cols(uint8_t *tile, uint32_t c, uint32_t r, const float *v) {
+    uint4 *o = reinterpret_cast<uint4 *>(tile + c * kChunk + r * 16u);
+    o[0] = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+    o[kChunk / 16] = make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]), pack2(v[14], v[15]));
 }
 
 // mode 0: forward only (clipped theta per row into theta_out); mode 1:
@@ -175,7 +186,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         *reinterpret_cast<uint16_t *>(sm + kB2 + kmaj(o, in, 64)) = P->w2[o][in];
         *reinterpret_cast<uint16_t *>(sm + kB3 + kmaj(in, o, 64)) = P->w2[o][in];
     }
-    for (uint32_t nn = 80 + grp * 4; nn < 84 + grp * 4; ++nn) st_bf16(sm + kB4, kmaj(nn, r, kN4), nn == 80 ? 1.0f : 0.0f);
+    {  // chunks 10 and 11 of both F buffers: the ones column, then zeros
+        uint8_t *f = sm + kF + (grp >> 1) * kFBytes + (10u + (grp & 1u)) * kChunk + r * 16u;
+        *reinterpret_cast<uint4 *>(f) = make_uint4((grp & 1u) ? 0u : 0x3f80u, 0u, 0u, 0u);
+    }
     if (tid < 64) {
         b1s[tid] = P->b1[tid];
         b2s[tid] = P->b2[tid];
@@ -202,52 +216,63 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
     for (int i = 0; i < kCols; ++i) dw3[i] = 0.0f;
     float db3 = 0.0f;
-    uint32_t phase = 0;
+    uint32_t phase = 0, buf = 0;
     bool ok = true, first = true;
+    // a wait that gave up leaves ok false: no further waits
+    auto wait_mma = [&]() {
+        if (ok) ok = mbar_wait(mbar_a, phase);
+        phase ^= 1u;
+        tc_after_sync();
+    };
 
+    // the row's four features of this group and its a, b, one tile ahead
     const uint64_t tiles = (n_rows + kRows - 1) / kRows;
+    uint32_t xf[2] = {0u, 0u};
+    float ra = 0.0f, rb = 0.0f;
+    auto load_row = [&](uint64_t tile) {
+        const uint64_t i = tile * kRows + r;
+        xf[0] = xf[1] = 0u;
+        ra = rb = 0.0f;
+        if (tile < tiles && i < n_rows) {
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(rows + i);
+            xf[0] = w[2 * grp];
+            xf[1] = w[2 * grp + 1];
+            ra = __uint_as_float(w[8]);
+            rb = __uint_as_float(w[9]);
+        }
+    };
+    load_row(blockIdx.x);
     for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint64_t row_i = tile * kRows + r;
         const bool valid = row_i < n_rows;
-        MlpRow row;
-        if (valid) {
-            row = rows[row_i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) row.x[i] = 0;
-            row.a = row.b = 0.0f;
-        }
+        uint8_t *const F = sm + kF + buf * kFBytes;
+        buf ^= 1u;
+        const float row_a = ra, row_b = rb;
         // each group stores four of the row's sixteen features
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t f = grp * 4u + i;
-            *reinterpret_cast<uint16_t *>(sm + kA1 + kmaj(r, f, kRows)) = row.x[f];
-            if (MODE == 1) *reinterpret_cast<uint16_t *>(sm + kB4 + kmaj(64 + f, r, kN4)) = row.x[f];
-        }
+        *reinterpret_cast<uint2 *>(F + kX + (grp >> 1) * kChunk + r * 16u + (grp & 1u) * 8u) = make_uint2(xf[0], xf[1]);
+        load_row(tile + gridDim.x);
         fence_async_smem();
         tc_before_sync();
         __syncthreads();
         // ---- layer 1
         if (tid == 0) {
             tc_after_sync();
-            mma_bf16(tmem + kColD1, sdesc(smem_u32(sm + kA1), 2048, 128), sdesc(smem_u32(sm + kB1), 1024, 128),
+            mma_bf16(tmem + kColD1, sdesc(smem_u32(F + kX), kChunk, 128), sdesc(smem_u32(sm + kB1), 1024, 128),
                      idesc_bf16(64), 0);
-            mma_commit(mbar_a);
+            mma_commit(mbar_a);  // and the previous tile's weight-gradient MMAs
         }
-        if (!(ok = wait_all(mbar_a, phase))) break;
+        wait_mma();
         float dg1[kCols];  // GELU'(z1) of this thread's columns
         {
             float z[16];
             tmem_ld16(tmem + lane_base + kColD1 + c0, z);
 #pragma unroll
             for (int i = 0; i < kCols; ++i) {
-                const uint32_t j = c0 + i;
                 float gv;
-                gelu_both(f_add(z[i], b1s[j]), gv, dg1[i]);
-                const float h = bf16_round(gv);
-                st_bf16(sm + kA2, kmaj(r, j, kRows), h);
-                if (MODE == 1) st_bf16(sm + kB4, kmaj(j, r, kN4), h);
+                gelu_both(f_add(z[i], b1s[c0 + i]), gv, dg1[i]);
+                z[i] = gv;
             }
+            st_cols(F, 2u * grp, r, z);
         }
         fence_async_smem();
         tc_before_sync();
@@ -257,11 +282,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_after_sync();
 #pragma unroll
             for (uint32_t kk = 0; kk < 4; ++kk)
-                mma_bf16(tmem + kColD2, sdesc(smem_u32(sm + kA2 + kk * 4096), 2048, 128),
+                mma_bf16(tmem + kColD2, sdesc(smem_u32(F + kk * 2 * kChunk), kChunk, 128),
                          sdesc(smem_u32(sm + kB2 + kk * 2048), 1024, 128), idesc_bf16(64), kk > 0);
             mma_commit(mbar_a);
         }
-        if (!(ok = wait_all(mbar_a, phase))) break;
+        wait_mma();
         float h2[kCols], dg2[kCols];
         {
             float z2[16];
@@ -274,27 +299,27 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             thp[grp * 128 + r] = part;
         }
+        tc_before_sync();
         __syncthreads();
         const float th = f_add(f_add(f_add(f_add(b3, thp[r]), thp[128 + r]), thp[256 + r]), thp[384 + r]);
         const bool inside = th >= -CSMC_MLP_THETA_MAX && th <= CSMC_MLP_THETA_MAX;
         const float thc = inside ? th : (th < 0.0f ? -CSMC_MLP_THETA_MAX : CSMC_MLP_THETA_MAX);
         if (MODE == 0) {
             if (valid && grp == 0) theta_out[row_i] = thc;
-            tc_before_sync();
-            __syncthreads();
             continue;
         }
         const float e = exp2_f(f_mul(thc, 1.44269502f));
-        if (valid && grp == 0) J += static_cast<double>(row.b) * thc - static_cast<double>(row.a) * e;
-        const float g = (valid && inside) ? f_add(row.b, -f_mul(row.a, e)) : 0.0f;
+        if (valid && grp == 0) J += static_cast<double>(row_b) * thc - static_cast<double>(row_a) * e;
+        const float g = (valid && inside) ? f_add(row_b, -f_mul(row_a, e)) : 0.0f;
         if (grp == 0) db3 = f_add(db3, g);
+        {
+            float dz[kCols];
 #pragma unroll
-        for (int i = 0; i < kCols; ++i) {
-            const uint32_t k = c0 + i;
-            dw3[i] = f_fma(g, h2[i], dw3[i]);
-            const float dz = f_mul(f_mul(g, w3s[k]), dg2[i]);
-            st_bf16(sm + kA3, kmaj(r, k, kRows), dz);
-            st_bf16(sm + kA4, kmaj(k, r, kRows), dz);
+            for (int i = 0; i < kCols; ++i) {
+                dw3[i] = f_fma(g, h2[i], dw3[i]);
+                dz[i] = f_mul(f_mul(g, w3s[c0 + i]), dg2[i]);
+            }
+            st_cols(sm + kZ, 2u * grp, r, dz);
         }
         fence_async_smem();
         tc_before_sync();
@@ -304,37 +329,42 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_after_sync();
 #pragma unroll
             for (uint32_t kk = 0; kk < 4; ++kk)
-                mma_bf16(tmem + kColD1, sdesc(smem_u32(sm + kA3 + kk * 4096), 2048, 128),
+                mma_bf16(tmem + kColD1, sdesc(smem_u32(sm + kZ + kk * 2 * kChunk), kChunk, 128),
                          sdesc(smem_u32(sm + kB3 + kk * 2048), 1024, 128), idesc_bf16(64), kk > 0);
             mma_commit(mbar_a);
         }
-        if (!(ok = wait_all(mbar_a, phase))) break;
+        wait_mma();
         {
             float dh[16];
             tmem_ld16(tmem + lane_base + kColD1 + c0, dh);
 #pragma unroll
-            for (int i = 0; i < kCols; ++i) st_bf16(sm + kA4, kmaj(64 + c0 + i, r, kRows), f_mul(dh[i], dg1[i]));
+            for (int i = 0; i < kCols; ++i) dh[i] = f_mul(dh[i], dg1[i]);
+            st_cols(sm + kZ, 8u + 2u * grp, r, dh);
         }
         fence_async_smem();
         tc_before_sync();
         __syncthreads();
-        // ---- weight gradients: D4 += dZ^T . F
+        // ---- weight gradients: D4 += Z^T . F, sixteen rows at a time
         if (tid == 0) {
             tc_after_sync();
 #pragma unroll
             for (uint32_t kk = 0; kk < 8; ++kk)
-                mma_bf16(tmem + kColD4, sdesc(smem_u32(sm + kA4 + kk * 4096), 2048, 128),
-                         sdesc(smem_u32(sm + kB4 + kk * 3072), 1536, 128), idesc_bf16(kN4), (!first || kk > 0));
-            mma_commit(mbar_a);
+                mma_bf16(tmem + kColD4, sdesc(smem_u32(sm + kZ + kk * 256), 128, kChunk),
+                         sdesc(smem_u32(F + kk * 256), 128, kChunk), idesc_bf16(kN4, true), (!first || kk > 0));
         }
         first = false;
-        if (!(ok = wait_all(mbar_a, phase))) break;
     }
-    if (!ok) {
-        if (error) atomicExch(error, 1);
+    if (MODE == 1 && !first) {  // the last tile's weight gradients
+        if (tid == 0) mma_commit(mbar_a);
+        wait_mma();
+    }
+    if (__syncthreads_or(ok ? 0 : 1)) {
+        if (!ok && error) atomicExch(error, 1);
         // one more bounded wait for the MMAs still in flight before freeing
         (void)mbar_wait(mbar_a, phase ^ 1u);
+        ok = false;
     }
+    tc_after_sync();
 
     if (MODE == 1) {
         float *out = partials + static_cast<size_t>(blockIdx.x) * (128 * kN4 + 66);
