@@ -411,32 +411,56 @@ __device__ __forceinline__ int partial_of(int k) {
     return 128 * N4 + 64;                                                                    // db3
 }
 
-// Entry k of the gradient: the CTAs' partials in order, FP64.  The loads are
-// independent of the sum: 37 in flight (148 CTAs in four rounds).
-__device__ __forceinline__ float partial_sum(const float *partials, int grid, int pf, int k) {
-    const float *p = partials + partial_of(k);
+// The per-entry kernels: a CTA takes kEntries entries and four threads load
+// each entry's partials (37 of 148 CTAs' each, all in flight at once; one
+// thread per entry measured 14 us of a 73 us Adam step); one thread then adds
+// them in CTA order, FP64.  Entry kGradFloats is the objective.
+constexpr int kEntries = 64, kLoaders = 4, kEntryThreads = kEntries * kLoaders;
+constexpr int kEntryBlocks = (kGradFloats + 3 + kEntries - 1) / kEntries;
+constexpr int kMaxGrid = 160;  // gradient CTAs the kernels hold partials of at once
+
+__device__ __forceinline__ double entry_sum(const float *partials, const double *objective, int grid, int pf) {
+    __shared__ float part[kMaxGrid][kEntries];
+    const int e = static_cast<int>(threadIdx.x % kEntries), q = static_cast<int>(threadIdx.x / kEntries);
+    const int k = static_cast<int>(blockIdx.x) * kEntries + e;
     double acc = 0.0;
-#pragma unroll 37
-    for (int c = 0; c < grid; ++c) acc = csmc::d_add(acc, static_cast<double>(p[static_cast<size_t>(c) * pf]));
-    return static_cast<float>(acc);
+    for (int c0 = 0; c0 < grid; c0 += kMaxGrid) {
+        const int n = grid - c0 < kMaxGrid ? grid - c0 : kMaxGrid;
+        if (k < kGradFloats) {
+            // (into registers first: a store to shared memory between two loads would order them)
+            const float *p = partials + static_cast<size_t>(c0) * pf + partial_of(k);
+            float v[kMaxGrid / kLoaders];
+#pragma unroll
+            for (int i = 0; i < kMaxGrid / kLoaders; ++i) {
+                const int c = q + kLoaders * i;
+                v[i] = c < n ? p[static_cast<size_t>(c) * pf] : 0.0f;
+            }
+#pragma unroll
+            for (int i = 0; i < kMaxGrid / kLoaders; ++i) part[q + kLoaders * i][e] = v[i];
+        }
+        __syncthreads();
+        if (q == 0) {
+            if (k < kGradFloats) {
+#pragma unroll 16
+                for (int c = 0; c < n; ++c) acc = csmc::d_add(acc, static_cast<double>(part[c][e]));
+            } else if (k == kGradFloats) {
+#pragma unroll 8
+                for (int c = 0; c < n; ++c) acc = csmc::d_add(acc, objective[c0 + c]);
+            }
+        }
+        __syncthreads();
+    }
+    return acc;
 }
 
-__device__ __forceinline__ double objective_sum(const double *objective, int grid) {
-    double s = 0.0;
-#pragma unroll 37
-    for (int c = 0; c < grid; ++c) s = csmc::d_add(s, objective[c]);
-    return s;
-}
-
-constexpr int kEntryThreads = 64;  // threads per CTA of the per-entry kernels: 84 CTAs, so the loads come from many SMs
-constexpr int kEntryBlocks = (kGradFloats + 3 + kEntryThreads - 1) / kEntryThreads;
-
-// The gradient (one thread per entry) and the objective J.
+// The gradient and the objective J.
 __global__ void reduce_mlp_partials(const float *partials, const double *objective, int grid, int pf, float *grad,
                                     double *J) {
-    const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (k < kGradFloats) grad[k] = partial_sum(partials, grid, pf, k);
-    if (k == kGradFloats) *J = objective_sum(objective, grid);
+    const double s = entry_sum(partials, objective, grid, pf);
+    if (threadIdx.x >= kEntries) return;
+    const int k = static_cast<int>(blockIdx.x * kEntries + threadIdx.x);
+    if (k < kGradFloats) grad[k] = static_cast<float>(s);
+    else if (k == kGradFloats) *J = s;
 }
 
 // Entry k of the FP32 master vector into the BF16 parameter block, the host
@@ -464,10 +488,12 @@ __global__ void mlp_pack_params(const float *x, csmc::MlpParams *P) {
 __global__ void mlp_adam_ascend(const float *partials, const double *objective, int grid, int pf, float *x, double *m,
                                 double *v, double lr, double c1, double c2, csmc::MlpParams *P, double *J) {
     constexpr double b1 = 0.9, b2 = 0.999, eps = 1e-8;
-    const int k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (k == kGradFloats) *J = objective_sum(objective, grid);
+    const double s = entry_sum(partials, objective, grid, pf);
+    if (threadIdx.x >= kEntries) return;
+    const int k = static_cast<int>(blockIdx.x * kEntries + threadIdx.x);
+    if (k == kGradFloats) *J = s;
     if (k >= kGradFloats) return;
-    const double gi = static_cast<double>(partial_sum(partials, grid, pf, k));
+    const double gi = static_cast<double>(static_cast<float>(s));
     const double mk = csmc::d_add(csmc::d_mul(b1, m[k]), csmc::d_mul(1.0 - b1, gi));
     const double vk = csmc::d_add(csmc::d_mul(b2, v[k]), csmc::d_mul(csmc::d_mul(1.0 - b2, gi), gi));
     m[k] = mk;
@@ -592,7 +618,7 @@ int mlp_adam(const void *rows, uint64_t n_rows, int32_t steps, double lr, float 
     CK(cudaMemcpyAsync(m.moments, mom1, mb, cudaMemcpyHostToDevice, st), "upload moments");
     CK(cudaMemcpyAsync(m.moments + kGradFloats, mom2, mb, cudaMemcpyHostToDevice, st), "upload moments");
     int32_t tt = *t;
-    mlp_pack_params<<<kEntryBlocks, kEntryThreads, 0, st>>>(m.x, m.P);
+    mlp_pack_params<<<kEntryBlocks, kEntries, 0, st>>>(m.x, m.P);
     CK(cudaGetLastError(), "parameter packing launch");
     for (int32_t s = 0; s < steps; ++s) {
         rc = csmc::mlp_tc_launch(1, static_cast<const csmc::MlpRow *>(rows), n_rows, m.P, nullptr, m.partials,

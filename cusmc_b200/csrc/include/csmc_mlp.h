@@ -55,7 +55,7 @@ namespace csmc {
  *   b2[HID]       FP32
  *   w3[HID]       FP32 output weights (applied on CUDA cores)
  *   b3            FP32 */
-struct MlpParams {
+struct alignas(16) MlpParams {
     uint16_t w1[CSMC_MLP_HID][CSMC_MLP_IN];
     float b1[CSMC_MLP_HID];
     uint16_t w2[CSMC_MLP_HID][CSMC_MLP_HID];

@@ -38,7 +38,8 @@
 // What bounds it: the CUDA-core epilogues (two GELUs with their derivatives
 // per hidden unit and row); the tensor pipe is nearly idle.  Measured (B200):
 // 1e6 rows 613 us with transposed operand copies stored 2 bytes at a time
-// (2,830 instructions per warp and tile), see below for the present form.
+// (2,830 instructions per warp and tile), 269 us in this form (1,515; issue
+// slots 69 % busy).
 #include "../include/csmc_mlp.h"
 #include "sim.cuh"
 
@@ -55,6 +56,8 @@ constexpr uint32_t kTmemCols = 256;             // D1/D3 [0,64), D2 [64,128), D4
 constexpr uint32_t kColD1 = 0, kColD2 = 64, kColD4 = 128;
 constexpr int kN4 = 96;                         // [H1 (64) | X (16) | 1 | 0 x 15]
 
+constexpr int kPartial = 128 * kN4 + 68;        // floats of a CTA's partials: D4, dw3, db3, padded to 16 bytes
+
 // shared-memory carve-up (bytes)
 constexpr uint32_t kChunk = 128 * 16;           // one column chunk: 8 columns of 128 rows
 constexpr uint32_t kFBytes = (kN4 / 8) * kChunk;
@@ -63,8 +66,7 @@ constexpr uint32_t kX = 8 * kChunk;             // X within F
 constexpr uint32_t kZ = kF + 2 * kFBytes;       // Z tile: chunks 0..7 dZ2, 8..15 dZ1
 constexpr uint32_t kB1 = kZ + 16 * kChunk;      // W1          64 x 16
 constexpr uint32_t kB2 = kB1 + 64 * 16 * 2;     // W2          64 x 64 (out x in)
-constexpr uint32_t kB3 = kB2 + 64 * 64 * 2;     // W2^T        64 x 64 (in x out)
-constexpr uint32_t kTh = kB3 + 64 * 64 * 2;     // theta partials [group][row] (floats)
+constexpr uint32_t kTh = kB2 + 64 * 64 * 2;     // theta partials [group][row] (floats)
 constexpr uint32_t kMisc = kTh + kGroups * 128 * 4;  // mbarrier, tmem address, biases, reductions
 constexpr uint32_t kMiscBytes = 4096;
 constexpr uint32_t kRedStride = 17;             // per-warp output-layer sums: 16 columns, db3
@@ -90,10 +92,10 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
            (static_cast<uint64_t>((sbo >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
 
-// instruction descriptor: FP32 accumulator, BF16 A and B, M=128; both operands
-// K-major, or both MN-major
-__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t N, bool mn_major = false) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? (1u << 15) | (1u << 16) : 0u) | ((N >> 3) << 17) |
+// instruction descriptor: FP32 accumulator, BF16 A and B, M=128; each operand
+// K-major or MN-major
+__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t N, bool a_mn = false, bool b_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u) | ((N >> 3) << 17) |
            ((128u >> 4) << 24);
 }
 
@@ -176,16 +178,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     float *thp = reinterpret_cast<float *>(sm + kTh);           // [group][row]
     const uint32_t mbar_a = smem_u32(mbar);
 
-    // ---- constant operands: W1 (B1), W2 (B2), W2^T (B3), the ones column of B4
-    for (uint32_t i = tid; i < 64 * 16; i += blockDim.x) {
-        const uint32_t o = i / 16, in = i % 16;
-        *reinterpret_cast<uint16_t *>(sm + kB1 + kmaj(o, in, 64)) = P->w1[o][in];
+    // ---- constant operands: W1 (B1), W2 (B2; read MN-major as W2^T in the
+    // back-propagation), eight inputs of a unit at a time, the ones columns
+    if (tid < 128) {
+        const uint32_t o = tid >> 1, c = tid & 1u;
+        *reinterpret_cast<uint4 *>(sm + kB1 + kmaj(o, 8u * c, 64)) = reinterpret_cast<const uint4 *>(&P->w1[0][0])[tid];
     }
-    for (uint32_t i = tid; i < 64 * 64; i += blockDim.x) {
-        const uint32_t o = i / 64, in = i % 64;
-        *reinterpret_cast<uint16_t *>(sm + kB2 + kmaj(o, in, 64)) = P->w2[o][in];
-        *reinterpret_cast<uint16_t *>(sm + kB3 + kmaj(in, o, 64)) = P->w2[o][in];
-    }
+    *reinterpret_cast<uint4 *>(sm + kB2 + kmaj(tid >> 3, 8u * (tid & 7u), 64)) =
+        reinterpret_cast<const uint4 *>(&P->w2[0][0])[tid];
+    static_assert(kThreads == CSMC_MLP_HID * CSMC_MLP_HID / 8, "one 16-byte word of W2 per thread");
     {  // chunks 10 and 11 of both F buffers: the ones column, then zeros
         uint8_t *f = sm + kF + (grp >> 1) * kFBytes + (10u + (grp & 1u)) * kChunk + r * 16u;
         *reinterpret_cast<uint4 *>(f) = make_uint4((grp & 1u) ? 0u : 0x3f80u, 0u, 0u, 0u);
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (uint32_t kk = 0; kk < 4; ++kk)
                 mma_bf16(tmem + kColD1, sdesc(smem_u32(sm + kZ + kk * 2 * kChunk), kChunk, 128),
-                         sdesc(smem_u32(sm + kB3 + kk * 2048), 1024, 128), idesc_bf16(64), kk > 0);
+                         sdesc(smem_u32(sm + kB2 + kk * 256), 128, 1024), idesc_bf16(64, false, true), kk > 0);
             mma_commit(mbar_a);
         }
         wait_mma();
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (uint32_t kk = 0; kk < 8; ++kk)
                 mma_bf16(tmem + kColD4, sdesc(smem_u32(sm + kZ + kk * 256), 128, kChunk),
-                         sdesc(smem_u32(F + kk * 256), 128, kChunk), idesc_bf16(kN4, true), (!first || kk > 0));
+                         sdesc(smem_u32(F + kk * 256), 128, kChunk), idesc_bf16(kN4, true, true), (!first || kk > 0));
         }
         first = false;
     }
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_after_sync();
 
     if (MODE == 1) {
-        float *out = partials + static_cast<size_t>(blockIdx.x) * (128 * kN4 + 66);
+        float *out = partials + static_cast<size_t>(blockIdx.x) * kPartial;
         if (grp < 3) {  // groups 0..2 read 32 of D4's 96 columns each
             if (ok && !first) {  // block-uniform
                 float v[16];
@@ -376,7 +377,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint32_t col = grp * 32u + 16u * c;
                     tmem_ld16(tmem + lane_base + kColD4 + col, v);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) out[r * kN4 + col + i] = v[i];
+                    for (int i = 0; i < 16; i += 4)
+                        *reinterpret_cast<float4 *>(out + r * kN4 + col + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
             } else {
                 for (int i = 0; i < 32; ++i) out[r * kN4 + grp * 32 + i] = 0.0f;
@@ -411,6 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncthreads();
         if (tid == 0) {
             double sum = 0.0;
+#pragma unroll 32
             for (int i = 0; i < 128; ++i) sum += jred[i];
             objective[blockIdx.x] = sum;
         }
@@ -424,7 +427,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }  // namespace
 
 size_t mlp_tc_smem_bytes() { return kSmemBytes; }
-int mlp_tc_partial_floats() { return 128 * kN4 + 66; }
+int mlp_tc_partial_floats() { return kPartial; }
 
 int mlp_tc_launch(int mode, const MlpRow *rows, uint64_t n_rows, const MlpParams *P, float *theta_out,
                   float *partials, double *objective, int *error, int grid, void *stream) {
