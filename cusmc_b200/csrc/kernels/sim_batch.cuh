@@ -83,7 +83,7 @@ static __device__ __forceinline__ void batch_group_phase(const BatchParams &p, c
         const unsigned long long local = r - J.run_begin;
         const SeedKeys keys{J.seed};
         const uint32_t bits = ceil_log2(n.n_comps);
-        g.init(n, J);
+        g.init(n, J, keys, J.first_run + local);
         while (!g.finish(n, J, local, acc_hits, acc_steps, acc_capped)) g.advance(n, J, keys, J.first_run + local, bits);
     }
     if (lane == 0) flush_counters(jobs[jb], acc_hits, acc_steps, acc_capped);

@@ -113,6 +113,10 @@ struct GroupRun {
     bool dirty;        // variables changed since the rate table was evaluated
     uint32_t pm;       // bit k: this lane's component k has its rate from the table
     uint32_t cap;      // components the state is laid out for
+    // one block per lane (NB 1): the next step's draws and their -log2, drawn
+    // while the step before waits for its race and its tables
+    uint32_t nx[NB == 1 ? B : 1];
+    float nl[NB == 1 ? B : 1];
 
     __device__ __forceinline__ GroupRun(RunState *state, uint32_t lane, uint32_t capacity) {
         cap = NB ? G * B * NB : capacity;
@@ -176,9 +180,22 @@ struct GroupRun {
         *rec_of(k) = make_uint2(inv, form);
     }
 
+    template <class KEYS>
+    __device__ __forceinline__ void draw(const KEYS &keys, uint64_t run, uint32_t at) {
+        if constexpr (NB == 1) {
+            const uint32_t c = gl * B;
+            const u32x4 blk = keys.block(at, run, c >> 2);
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                nx[i] = B == 4 ? word_of(blk, i) : word_of(blk, (c + i) & 3u);
+                nl[i] = neg_log2_draw(nx[i]);
+            }
+        }
+    }
+
     // run initialisation (simulation.cu:766-831)
-    template <class Q>
-    __device__ __forceinline__ void init(const Net &n, const Q &q) {
+    template <class Q, class KEYS>
+    __device__ __forceinline__ void init(const Net &n, const Q &q, const KEYS &keys, uint64_t run) {
         const uint32_t C = n.n_comps, V = n.n_vars;
         uint8_t *tail = reinterpret_cast<uint8_t *>(s) + group_vars_bytes(V, n.n_rate_prog);
         rec = reinterpret_cast<uint2 *>(tail);
@@ -211,6 +228,7 @@ struct GroupRun {
         eval_rates(n);
         look_up_all(n);
         dirty = false;
+        draw(keys, run, 0u);
     }
 
     // distinct rate programs, spread over the lanes
@@ -299,18 +317,29 @@ struct GroupRun {
                     form[2 * h + 1] = r.w;
                 }
             }
-            const u32x4 blk = keys.block(step, run, c >> 2);
+            uint32_t xs[B];
             float d[B];
             uint32_t special = 0;
+            if constexpr (NB == 1) {
 #pragma unroll
-            for (int i = 0; i < B; ++i) {
-                d[i] = exp_delay(B == 4 ? word_of(blk, i) : word_of(blk, (c + i) & 3u), __uint_as_float(iv[i]));
-                special |= form[i];
+                for (int i = 0; i < B; ++i) {
+                    xs[i] = nx[i];
+                    d[i] = f_mul(nl[i], __uint_as_float(iv[i]));
+                    special |= form[i];
+                }
+            } else {
+                const u32x4 blk = keys.block(step, run, c >> 2);
+#pragma unroll
+                for (int i = 0; i < B; ++i) {
+                    xs[i] = B == 4 ? word_of(blk, i) : word_of(blk, (c + i) & 3u);
+                    d[i] = exp_delay(xs[i], __uint_as_float(iv[i]));
+                    special |= form[i];
+                }
             }
             if (special) {
 #pragma unroll
                 for (int i = 0; i < B; ++i) {
-                    const uint32_t x = B == 4 ? word_of(blk, i) : word_of(blk, (c + i) & 3u);
+                    const uint32_t x = xs[i];
                     if (form[i] >= kFormInv1) {
                         // uniform on (0, bound - clock] while the bound lies
                         // ahead (comp_delay's arithmetic, inv1_delay)
@@ -393,6 +422,7 @@ struct GroupRun {
         float bd;
         lane_min(n, keys, run, bits, bkey, bbr, bd);
         const uint32_t m = group_min(bkey, gmask);
+        draw(keys, run, step + 1u);
         if (m == 0xffffffffu) {
             bbr = lowest_brev(n.n_comps, bits);
             bd = __uint_as_float(0x7fffffffu);
@@ -492,23 +522,34 @@ __global__ void __launch_bounds__(512, 1) sim_kernel(const __grid_constant__ Sim
 
     unsigned long long acc_hits = 0, acc_steps = 0, acc_capped = 0;
     unsigned long long ridx = 0;
-    bool have = false, drained = false;
-    for (;;) {
-        __syncwarp();
-        if (!have && !drained) {
+    if constexpr (G == 32) {  // one run per warp: no other group to meet
+        for (;;) {
             if (r.gl == 0) ridx = atomicAdd(p.scratch, 1ull);
-            ridx = __shfl_sync(r.gmask, ridx, 0, G);
-            if (ridx >= p.n_runs) {
-                drained = true;
-            } else {
-                have = true;
-                r.init(n, p);
-            }
+            ridx = __shfl_sync(0xffffffffu, ridx, 0);
+            if (ridx >= p.n_runs) break;
+            const uint64_t run = p.first_run + ridx;
+            r.init(n, p, keys, run);
+            while (!r.finish(n, p, ridx, acc_hits, acc_steps, acc_capped)) r.advance(n, p, keys, run, bits);
         }
-        if (__all_sync(0xffffffffu, drained)) break;
-        if (have) {
-            if (r.finish(n, p, ridx, acc_hits, acc_steps, acc_capped)) have = false;
-            else r.advance(n, p, keys, p.first_run + ridx, bits);
+    } else {
+        bool have = false, drained = false;
+        for (;;) {
+            __syncwarp();
+            if (!have && !drained) {
+                if (r.gl == 0) ridx = atomicAdd(p.scratch, 1ull);
+                ridx = __shfl_sync(r.gmask, ridx, 0, G);
+                if (ridx >= p.n_runs) {
+                    drained = true;
+                } else {
+                    have = true;
+                    r.init(n, p, keys, p.first_run + ridx);
+                }
+            }
+            if (__all_sync(0xffffffffu, drained)) break;
+            if (have) {
+                if (r.finish(n, p, ridx, acc_hits, acc_steps, acc_capped)) have = false;
+                else r.advance(n, p, keys, p.first_run + ridx, bits);
+            }
         }
     }
     if (r.gl == 0) {
