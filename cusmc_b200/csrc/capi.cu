@@ -327,7 +327,7 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
     }
     CK(cudaMemsetAsync(n->d_scratch, 0, CSMC_SCRATCH_WORDS * sizeof(unsigned long long), st), "cudaMemsetAsync");
     csmc::SimParams p{};
-    p.net = csmc::layout_of(n->h);
+    p.net = csmc::layout_of(*n);
     p.blob = n->d_blob;
     p.blob_bytes = n->bytes;
     p.state_stride = pl.state_stride;
@@ -561,6 +561,7 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
     CK(cudaGetDevice(&n->device), "cudaGetDevice");
     n->h = *h;
     n->bytes = (h->total_bytes + 15u) & ~15u;
+    n->clock_base = csmc::clock_base_of(*h, blob);
     n->slots = h->max_edges_per_loc >= 2;
     n->loc8 = h->max_locs_per_comp <= 256;
     n->classes = (h->flags & CSMC_NET_RACE_CLASSES) != 0 && h->n_comps <= 256;

@@ -186,7 +186,7 @@ std::vector<csmc::BatchJob> build_table(const csmc_batch *b, const std::vector<u
         const csmc_query &q = b->qs[j];
         csmc::BatchJob &J = t[k];
         std::memset(&J, 0, sizeof J);
-        J.net = csmc::layout_of(n->h);
+        J.net = csmc::layout_of(*n);
         J.blob = n->d_blob;
         J.run_begin = begin[b->group[j] ? 1 : 0];
         J.n_runs = runs[j];

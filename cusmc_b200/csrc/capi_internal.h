@@ -31,6 +31,7 @@ struct csmc_net {
     uint8_t *d_blob = nullptr;
     uint32_t bytes = 0;       // staged bytes (multiple of 16)
     csmc_net_header h{};
+    uint32_t clock_base = csmc::kNoClockBase;  // the clocks are consecutive variables from this one on
     unsigned long long *d_scratch = nullptr;
     // internal per-run buffers used when the caller passes none
     uint8_t *d_flags = nullptr;
@@ -76,5 +77,10 @@ struct csmc_net {
 };
 
 namespace csmc {
+inline NetLayout layout_of(const csmc_net &n) {
+    NetLayout l = layout_of(n.h);
+    l.clock_base = n.clock_base;
+    return l;
+}
 void set_last_error(const std::string &m);  // capi.cu
 }

@@ -193,7 +193,7 @@ csmc::IsParams base_params(const csmc_net *n, const csmc_query *q, uint64_t seed
                            uint64_t n_runs) {
     csmc::IsParams ip{};
     csmc::SimParams &p = ip.s;
-    p.net = csmc::layout_of(n->h);
+    p.net = csmc::layout_of(*n);
     p.blob = n->d_blob;
     p.blob_bytes = n->bytes;
     p.loc_mode = q->kind == CSMC_QUERY_LOCATION;

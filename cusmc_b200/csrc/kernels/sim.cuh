@@ -41,7 +41,10 @@ struct NetLayout {
     uint32_t n_comps, n_vars, n_rate_prog, flags, n_clocks, recv_lo, recv_hi;
     uint32_t n_classes;  // race classes in use (CSMC_RACE_CLASSES when the blob does not record it)
     uint32_t off_loc_inv1;  // one-invariant table (0: none)
+    uint32_t clock_base;    // clock j is variable clock_base + j (kNoClockBase: as listed at off_clock)
+    uint32_t pad;
 };
+constexpr uint32_t kNoClockBase = 0xffffffffu;
 
 inline NetLayout layout_of(const csmc_net_header &h) {
     const uint32_t ncls = (h.n_classes && h.n_classes <= CSMC_RACE_CLASSES) ? h.n_classes : CSMC_RACE_CLASSES;
@@ -49,7 +52,16 @@ inline NetLayout layout_of(const csmc_net_header &h) {
                      h.off_var,      h.off_const,   h.off_code,      h.off_loc_rate, h.off_inv_lit,
                      h.off_rate_prog, h.off_clock,  h.off_loc_desc,  h.n_comps,      h.n_vars,
                      h.n_rate_prog,  h.flags,       h.n_clocks,      h.recv_chan_lo, h.recv_chan_hi,
-                     ncls,           h.off_loc_inv1};
+                     ncls,           h.off_loc_inv1, kNoClockBase,    0u};
+}
+// Whether the clocks of a blob (host memory) are consecutive variables: the
+// first one's id, else kNoClockBase.
+inline uint32_t clock_base_of(const csmc_net_header &h, const void *blob) {
+    if (!h.n_clocks || h.off_clock + 2ull * h.n_clocks > h.total_bytes) return kNoClockBase;
+    const uint8_t *p = static_cast<const uint8_t *>(blob) + h.off_clock;
+    for (uint32_t j = 0; j < h.n_clocks; ++j)
+        if (p[2 * j] + 256u * p[2 * j + 1] != p[0] + 256u * p[1] + j) return kNoClockBase;
+    return p[0] + 256u * p[1];
 }
 
 struct SimParams {
@@ -148,6 +160,7 @@ struct BatchJob {
     uint64_t *digests;             // verification outputs (may be null)
     uint32_t *final_state;
     unsigned long long *counters;  // [0] hits [1] steps [2] capped
+    uint64_t pad;
 };
 static_assert(sizeof(BatchJob) % 16 == 0, "BatchJob is copied in 16-byte words");
 

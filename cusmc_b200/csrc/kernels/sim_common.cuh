@@ -35,7 +35,7 @@ struct Net {
     const uint16_t *clock;
     const uint64_t *loc_desc;
     const uint32_t *loc_inv1;  // CSMC_DESC_INV1 locations' invariant (null in blobs without the table)
-    uint32_t n_comps, n_vars, n_rate_prog, flags, n_clocks, recv_lo, recv_hi;
+    uint32_t n_comps, n_vars, n_rate_prog, flags, n_clocks, recv_lo, recv_hi, clock_base;
 };
 
 static __device__ __forceinline__ Net net_view(const uint8_t *base) {
@@ -63,6 +63,7 @@ static __device__ __forceinline__ Net net_view(const uint8_t *base) {
     n.n_clocks = h->n_clocks;
     n.recv_lo = h->recv_chan_lo;
     n.recv_hi = h->recv_chan_hi;
+    n.clock_base = kNoClockBase;
     return n;
 }
 
@@ -91,6 +92,7 @@ static __device__ __forceinline__ Net net_view(const uint8_t *base, const NetLay
     n.n_clocks = l.n_clocks;
     n.recv_lo = l.recv_lo;
     n.recv_hi = l.recv_hi;
+    n.clock_base = l.clock_base;
     return n;
 }
 
@@ -109,6 +111,29 @@ struct VarView {
     uint32_t stride;
     __device__ __forceinline__ float &operator[](uint32_t i) const { return base[i * stride]; }
 };
+
+// Clocks j0, j0 + dj, .. advance by d (simulation.cu:632-651).  FOUR, for
+// consecutive clocks: four are loaded before any is stored, without a look at
+// the list (one at a time, each waits for two dependent loads).
+template <bool FOUR>
+static __device__ __forceinline__ void advance_clocks(const Net &n, uint32_t n_clocks, VarView vars, float d,
+                                                      uint32_t j0, uint32_t dj) {
+    uint32_t j = j0;
+    if (FOUR && n.clock_base != kNoClockBase) {
+        for (; j + 3u * dj < n_clocks; j += 4u * dj) {
+            const uint32_t v = n.clock_base + j;
+            const float a = vars[v], b = vars[v + dj], c = vars[v + 2u * dj], e = vars[v + 3u * dj];
+            vars[v] = time_add(a, d);
+            vars[v + dj] = time_add(b, d);
+            vars[v + 2u * dj] = time_add(c, d);
+            vars[v + 3u * dj] = time_add(e, d);
+        }
+    }
+    for (; j < n_clocks; j += dj) {
+        const uint32_t v = n.clock[j];
+        vars[v] = time_add(vars[v], d);
+    }
+}
 
 // Key of a delay for 32-bit comparisons (delay_key): one OR unless the
 // delay is negative or NaN.

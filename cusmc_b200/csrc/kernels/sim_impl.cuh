@@ -438,10 +438,8 @@ struct GroupRun {
         if (dmin < __uint_as_float(0x7f800000u)) {
             // clocks advance (simulation.cu:632-651)
             if (n.n_clocks) {
-                for (uint32_t j = gl; j < n.n_clocks; j += G) {
-                    const uint32_t v = n.clock[j];
-                    s->vars[v] = time_add(s->vars[v], dmin);
-                }
+                // (a full warp with many clocks per lane; narrower groups have no registers to spare)
+                advance_clocks<(G == 32 && NB != 1)>(n, n.n_clocks, vars, dmin, gl, G);
                 __syncwarp(gmask);
             }
             // the winner's enabled edges (simulation.cu:268-305), one lane per edge

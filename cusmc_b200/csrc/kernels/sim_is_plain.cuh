@@ -357,10 +357,7 @@ __global__ void __launch_bounds__(CSMC_IS_BLOCK, CSMC_IS_MIN_CTAS_PER_SM)
             // ---- clocks, the winner's transition, time
             if (finite) {
                 if (n.n_clocks) {
-                    for (uint32_t j = lane; j < n.n_clocks; j += 32u) {
-                        const uint32_t v = n.clock[j];
-                        rv.vars[v] = time_add(rv.vars[v], dmin);
-                    }
+                    advance_clocks<false>(n, n.n_clocks, rv.vars, dmin, lane, 32u);
                     __syncwarp();
                     new_feat = true;
                     new_rates = rates_read_clocks;

@@ -180,10 +180,7 @@ static __device__ __forceinline__ bool run_commit(const Net &n, uint32_t n_clock
         mix(sc.digest, f_bits(dmin));
     }
     if (static_cast<double>(dmin) < kDblMax) {
-        for (uint32_t j = 0; j < n_clocks; ++j) {
-            const uint32_t v = n.clock[j];
-            vars[v] = time_add(vars[v], dmin);
-        }
+        advance_clocks<true>(n, n_clocks, vars, dmin, 0u, 1u);
         const uint32_t li = rv.loc(n, win);
         const uint32_t en = enabled_edges(n, vars, li);
         uint32_t sm = 0;

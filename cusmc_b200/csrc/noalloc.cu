@@ -191,6 +191,7 @@ extern "C" int csmc_run_noalloc(const void *blob_host, const void *blob_device, 
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(scratch)");
         csmc::SimParams p{};
         p.net = csmc::layout_of(h);
+        p.net.clock_base = csmc::clock_base_of(h, blob_host);
         p.blob = static_cast<const uint8_t *>(blob_device);
         p.blob_bytes = blob_bytes;
         p.state_stride = static_cast<uint32_t>(slab);
