@@ -79,8 +79,8 @@ bool configure_plan(const csmc_net *n, csmc_launch_plan &p, int family, int lane
             return false;
         }
         // per-group run state: 48 bytes of scalars, the variables, one
-        // inverse rate per rate program (evaluated once per step), the slot
-        // masks
+        // inverse rate per rate program, then the components' delay records,
+        // slot masks and locations
         const uint32_t stride = csmc::group_state_stride(h.n_vars, h.n_rate_prog, lanes, cpl);
         const size_t smem = n->bytes + static_cast<size_t>(block / lanes) * stride;
         if (smem > max_smem) {
@@ -212,7 +212,7 @@ void find_shapes(csmc_net *n) {
 //   groups:     S = (12 + K) (1 + d log2(32 / G)), the groups of a warp
 //               branching apart (d = 0.33; 0.5 in networks without race
 //               classes, whose steps differ more)
-//   one thread: S = 48 + 0.7 C (every location classed), 42 + 4.5 C (classes
+//   one thread: S = 48 + 0.7 C (every location classed), 46 + 2.25 C (classes
 //               and descriptors), 30 + 7.5 C (no classes)
 // and a launch takes S times the larger of its latency, 3.9 (2.8 one thread),
 // and its waves + 1, a wave being one warp per scheduler (waves count for more
@@ -223,11 +223,11 @@ void find_shapes(csmc_net *n) {
 // makes the latency 1.7 times that.  Fitted to the epidemic (12 to 200
 // agents), the mutex (8 to 256) and random networks (2 to 64 components) at
 // 100 to 131,072 runs on B200.  One thread per run / the best group: 100
-// agents 100 runs 14.3 / 3.0 ms, 16,384 runs 16.2 / 13.8, 32,768 runs 19.6 /
-// 23.5; mutex 32, 100 runs 28.4 / 2.8, 32,768 runs 30.8 / 20.4, 65,536 runs
-// 39.7 / 39.6; random 8, 100 runs 2.2 / 0.43 (0.70 with groups of 8 lanes),
-// 131,072 runs 6.3 / 6.0; random 24, 65,536 runs 19.7 / 24.0; random 64,
-// 131,072 runs 288 / 90.
+// agents 100 runs 14.4 / 2.7 ms, 16,384 runs 16.3 / 12.5, 32,768 runs 19.8 /
+// 23.1; mutex 32, 100 runs 34.6 / 4.8, 16,384 runs (a quarter of the time) 9.4
+// / 5.4, 32,768 runs 38.6 / 40.3, 65,536 runs 52.4 / 79.3; random 8, 100 runs
+// 2.2 / 0.37 (0.71 with groups of 8 lanes), 16,384 runs 2.4 / 1.5; random 64,
+// 131,072 runs 565 / 186.
 csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
     if (n->plan_forced || n->plan.family == 2 || n->n_shapes == 0) return n->plan;
     const double C = n->h.n_comps, unit = 128.0 * n->sms, runs = static_cast<double>(n_runs);
@@ -252,7 +252,7 @@ csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
         }
     }
     if (n->thread_warps > 0) {
-        const double S = n->plan.family != 4 ? 30.0 + 7.5 * C : n->only_classes ? 48.0 + 0.7 * C : 42.0 + 4.5 * C;
+        const double S = n->plan.family != 4 ? 30.0 + 7.5 * C : n->only_classes ? 48.0 + 0.7 * C : 46.0 + 2.25 * C;
         const double t = launch_time(S, std::ceil(runs / 32.0), 2.8, n->thread_warps, 10.0);
         // (where both fill the GPU a group is taken only when it is clearly the better one)
         if (t < best * (runs > 1.75 * unit ? 1.3 : 1.0)) return n->plan;

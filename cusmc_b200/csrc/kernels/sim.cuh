@@ -2,21 +2,22 @@
 // (simulation/simulation.cu:674-901) re-mapped onto lane groups.
 //
 // Mapping.  One run is simulated by a group of G lanes (G a power of two,
-// G <= 32); lane l of a group owns components l*K .. l*K+K-1.  Several groups
-// share a warp when G < 32.  The packed network (read-only, a few KB to a few
-// hundred KB) is staged once per CTA into shared memory; each group keeps its
-// run's variables, broadcast channel, goal flag and query extrema in shared
-// memory, and each lane keeps its components' locations and enabled-edge slot
-// masks in registers.  There are no block-wide barriers in the loop: a step is
+// G <= 32); lane l of a group owns components l*K .. l*K+K-1 (many per lane:
+// every G-th block of four).  Several groups share a warp when G < 32.  The
+// packed network (read-only, a few KB to a few hundred KB) is staged once per
+// CTA into shared memory; each group keeps its run's variables, rate table,
+// broadcast channel, goal flag and query extrema there, and its components'
+// delay records, locations and enabled-edge slot masks.  There are no
+// block-wide barriers in the loop: a step is
 //   1. broadcast receivers of the previous step's sender (enabled sets in
 //      parallel, transitions serially in component order);
 //   2. per-component delays (lane-parallel);
-//   3. the race: a segmented xor-butterfly min over (delay key, bit-reversed
-//      component index), which reproduces the reference's strided
-//      shared-memory tree argmin (simulation/simulation.cu:576-628) exactly,
-//      ties included;
-//   4. clock advance (lane-parallel over variables) and the winner's
-//      transition (one lane).
+//   3. the race: the smallest delay key, then the smallest bit-reversed
+//      component index among its holders, which reproduces the reference's
+//      strided shared-memory tree argmin (simulation/simulation.cu:576-628)
+//      exactly, ties included;
+//   4. clock advance (lane-parallel over variables), the guards of the
+//      winner's edges (lane-parallel) and its transition (one lane).
 // Runs are pulled from a device work counter, so groups whose runs end early
 // refill immediately (persistent kernel, grid = resident CTAs).
 #pragma once

@@ -39,6 +39,15 @@
 // runs (B200): 223 ms with one load-update-store per member in turn, 180 ms
 // with a block's four loads first (and one flat-spot check per step).
 //
+// Members outside the classes race with a delay of their own, some 80
+// instructions.  Evaluated where they come up in the race loop, a warp went
+// through them for nearly every component, since some lane's run had that
+// component in such a location; so the loop only notes their draws, and they
+// are gone through afterwards, a run's first with another run's first: as many
+// turns as the run with the most has.  Mutex of 8, 32, 64 and 128 processes,
+// 400,000, 200,000, 100,000 and 65,536 runs: 50 -> 41, 214 -> 143, 131 -> 80
+// and 213 -> 115 ms.
+//
 // Results are those of serial_kernel: the same draws, the same race
 // outcome, the same transitions.
 //
@@ -51,6 +60,7 @@ namespace detail {
 
 constexpr uint32_t kCodeGeneral = 7u;  // delay through the location's descriptor
 constexpr uint32_t kCodePad = 6u;      // no component
+constexpr uint32_t kMaxCodedComps = 256u;
 #ifndef CSMC_CODED_UNROLL
 #define CSMC_CODED_UNROLL 2
 #endif
@@ -136,41 +146,31 @@ static __device__ __forceinline__ uint32_t key_addr(const CodedView &rv, uint32_
     return rv.keys + (k == 0 ? f << 6 : f >> (8u * k - 6u));
 }
 
-// The four members of Philox block q, all of them class members.  cb: 255
-// minus the bit-reversed q, the low byte of their keys.
-static __device__ __forceinline__ void race_block(const CodedView &rv, uint32_t wd, const u32x4 &x, uint32_t cb) {
+// The members of a location word whose delay goes through its descriptor
+// (code 7; padding has 6): bit 8k + 7 for member k.
+static __device__ __forceinline__ uint32_t general_members(uint32_t wd) {
+    static_assert(kCodeGeneral == 7u && kCodePad == 6u, "bits 7 and 5 of a byte");
+    return wd & (wd << 2) & 0x80808080u;
+}
+
+// The four members of Philox block q.  cb: 255 minus the bit-reversed q, the
+// low byte of their keys.  ALLCLS: all of them class members; else the bytes
+// of the others are zero in wd and their bits set in out (bit 8k + 7 for
+// member k): they leave class 0's key as it is.
+template <bool ALLCLS>
+static __device__ __forceinline__ void race_block(const CodedView &rv, uint32_t wd, uint32_t out, const u32x4 &x,
+                                                  uint32_t cb) {
     const uint32_t a0 = key_addr<0>(rv, wd), a1 = key_addr<1>(rv, wd), a2 = key_addr<2>(rv, wd),
                    a3 = key_addr<3>(rv, wd);
     const uint32_t o0 = ld_key(a0), o1 = ld_key(a1 + kKeyChain), o2 = ld_key(a2 + 2u * kKeyChain),
                    o3 = ld_key(a3 + 3u * kKeyChain);
-    st_key(a0, max(o0, (x.x & 0xffffff00u) | cb));
-    st_key(a1 + kKeyChain, max(o1, (x.y & 0xffffff00u) | cb));
-    st_key(a2 + 2u * kKeyChain, max(o2, (x.z & 0xffffff00u) | cb));
-    st_key(a3 + 3u * kKeyChain, max(o3, (x.w & 0xffffff00u) | cb));
-}
-
-// One member of a block with members outside the classes: a class member
-// updates its key, a general one races with its own delay, padding is
-// skipped.
-template <uint32_t k>
-static __device__ __forceinline__ void race_member(const Net &n, const CodedView &rv, uint32_t wd, uint32_t cc,
-                                                   uint32_t x, uint32_t cb, uint32_t hi_shift,
-                                                   unsigned long long &best, float &bestd) {
-    const uint32_t b = (wd >> (8u * k)) & 0xffu;
-    const uint32_t code = b >> 5;
-    if (code < CSMC_RACE_CLASSES) {
-        const uint32_t a = key_addr<k>(rv, wd) + k * kKeyChain;
-        st_key(a, max(ld_key(a), (x & 0xffffff00u) | cb));
-    } else if (code == kCodeGeneral) {
-        const float d = desc_delay(n, rv, n.comp[cc].loc_begin + (b & 31u), x);
-        constexpr uint32_t kr = ((k & 1u) << 1) | (k >> 1);
-        const unsigned long long key =
-            (static_cast<unsigned long long>(delay_key(d)) << 32) | (255u - cb + (kr << hi_shift));
-        if (key < best) {
-            best = key;
-            bestd = d;
-        }
-    }
+    const auto key = [&](uint32_t w, uint32_t k) {
+        return ALLCLS || !(out & (0x80u << (8u * k))) ? (w & 0xffffff00u) | cb : 0u;
+    };
+    st_key(a0, max(o0, key(x.x, 0u)));
+    st_key(a1 + kKeyChain, max(o1, key(x.y, 1u)));
+    st_key(a2 + 2u * kKeyChain, max(o2, key(x.z, 2u)));
+    st_key(a3 + 3u * kKeyChain, max(o3, key(x.w, 3u)));
 }
 
 // race_exact out of line: the view of the network is rebuilt, the run state's
@@ -208,18 +208,48 @@ static __device__ __forceinline__ bool race_coded(const Net &n, uint32_t C, uint
     // bits (k) become the top two, q the low bits - 2 reversed
     const uint32_t hi_shift = bits - 2u;  // bits >= 2: the plan needs at least four components
     const uint32_t Q = (C + 3u) >> 2;
+    // members outside the classes: the blocks that have some, their draws
+    uint64_t general_blocks = 0;
+    uint32_t n_general = 0, draws[ALLCLS ? 1 : kMaxCodedComps];
 #pragma unroll kCodedUnroll
     for (uint32_t q = 0; q < Q; ++q) {
         const uint32_t wd = rv.lw[q * T];
         const u32x4 blk = philox_block(K, ps, q);
         const uint32_t cb = 255u - (hi_shift ? (__brev(q) >> (32u - hi_shift)) : 0u);
-        if (ALLCLS || !(wd & 0x80808080u)) {
-            race_block(rv, wd, blk, cb);
-        } else {
-            race_member<0>(n, rv, wd, 4u * q, blk.x, cb, hi_shift, best, bestd);
-            race_member<1>(n, rv, wd, 4u * q + 1u, blk.y, cb, hi_shift, best, bestd);
-            race_member<2>(n, rv, wd, 4u * q + 2u, blk.z, cb, hi_shift, best, bestd);
-            race_member<3>(n, rv, wd, 4u * q + 3u, blk.w, cb, hi_shift, best, bestd);
+        const uint32_t out = ALLCLS ? 0u : wd & 0x80808080u;
+        race_block<ALLCLS>(rv, ALLCLS ? wd : wd & ~((out >> 7) * 0xffu), out, blk, cb);
+        if (!ALLCLS) {
+            const uint32_t general = general_members(wd);
+            if (general) {
+                general_blocks |= 1ull << q;
+                if (general & 0x80u) draws[n_general++] = blk.x;
+                if (general & 0x8000u) draws[n_general++] = blk.y;
+                if (general & 0x800000u) draws[n_general++] = blk.z;
+                if (general & 0x80000000u) draws[n_general++] = blk.w;
+            }
+        }
+    }
+    // their delays, one member of each run at a time: a warp goes through as
+    // many as its run with the most has, not through every component that is
+    // outside the classes in one of its runs
+    if (!ALLCLS && n_general) {
+        uint32_t q = 0, wd = 0, general = 0;
+        for (uint32_t i = 0; i < n_general; ++i) {
+            if (!general) {
+                q = static_cast<uint32_t>(__ffsll(static_cast<long long>(general_blocks))) - 1u;
+                general_blocks &= general_blocks - 1u;
+                wd = rv.lw[q * T];
+                general = general_members(wd);
+            }
+            const uint32_t m = (static_cast<uint32_t>(__ffs(static_cast<int>(general))) >> 3) - 1u, c = 4u * q + m;
+            general &= general - 1u;
+            const float d = desc_delay(n, rv, n.comp[c].loc_begin + ((wd >> (8u * m)) & 31u), draws[i]);
+            const unsigned long long key =
+                (static_cast<unsigned long long>(delay_key(d)) << 32) | bitrev_bits(c, bits);
+            if (key < best) {
+                best = key;
+                bestd = d;
+            }
         }
     }
     // each class races with its largest key
