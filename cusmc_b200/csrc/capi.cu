@@ -212,9 +212,10 @@ void find_shapes(csmc_net *n) {
 //   groups:     S = (12 + K) (1 + d log2(32 / G)), the groups of a warp
 //               branching apart (d = 0.33; 0.5 in networks without race
 //               classes, whose steps differ more)
-//   one thread: S = 48 + 0.7 C (every location classed), 46 + 2.25 C (classes
-//               and descriptors), 30 + 7.5 C (no classes)
-// and a launch takes S times the larger of its latency, 3.9 (2.8 one thread),
+//   one thread: S = 48 + 0.7 C (every location classed), 48 + 1.9 C (classes
+//               and descriptors), 29 + 3.9 C (no classes)
+// and a launch takes S times the larger of its latency, 3.9 (2.8 one thread,
+// 3.6 without classes),
 // and its waves + 1, a wave being one warp per scheduler (waves count for more
 // where too few warps are resident to hide the latency).  Runs of networks
 // with clocks are about equally long: what does not fit on the SMs at once
@@ -224,10 +225,11 @@ void find_shapes(csmc_net *n) {
 // agents), the mutex (8 to 256) and random networks (2 to 64 components) at
 // 100 to 131,072 runs on B200.  One thread per run / the best group: 100
 // agents 100 runs 14.4 / 2.7 ms, 16,384 runs 16.3 / 12.5, 32,768 runs 19.8 /
-// 23.1; mutex 32, 100 runs 34.6 / 4.8, 16,384 runs (a quarter of the time) 9.4
-// / 5.4, 32,768 runs 38.6 / 40.3, 65,536 runs 52.4 / 79.3; random 8, 100 runs
-// 2.2 / 0.37 (0.71 with groups of 8 lanes), 16,384 runs 2.4 / 1.5; random 64,
-// 131,072 runs 565 / 186.
+// 23.1; mutex 32 (to time 30) 200 runs 4.7 / 0.8, 16,000 runs 5.1 / 3.3;
+// mutex 64 (to time 10) 16,000 runs 4.9 / 3.4, 32,768 runs 5.4 / 6.6; random 8,
+// 200 runs 1.7 / 0.39, 16,000 runs 1.9 / 1.4, 65,536 runs 2.3 / 3.2; random 24
+// (to time 60) 16,000 runs 6.6 / 3.9, 32,768 runs 7.0 / 7.5; random 64 (to time
+// 20) 131,072 runs 75 / 34.
 csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
     if (n->plan_forced || n->plan.family == 2 || n->n_shapes == 0) return n->plan;
     const double C = n->h.n_comps, unit = 128.0 * n->sms, runs = static_cast<double>(n_runs);
@@ -252,8 +254,9 @@ csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
         }
     }
     if (n->thread_warps > 0) {
-        const double S = n->plan.family != 4 ? 30.0 + 7.5 * C : n->only_classes ? 48.0 + 0.7 * C : 46.0 + 2.25 * C;
-        const double t = launch_time(S, std::ceil(runs / 32.0), 2.8, n->thread_warps, 10.0);
+        const double S = n->plan.family != 4 ? 29.0 + 3.9 * C : n->only_classes ? 48.0 + 0.7 * C : 48.0 + 1.9 * C;
+        const double t =
+            launch_time(S, std::ceil(runs / 32.0), n->plan.family != 4 ? 3.6 : 2.8, n->thread_warps, 10.0);
         // (where both fill the GPU a group is taken only when it is clearly the better one)
         if (t < best * (runs > 1.75 * unit ? 1.3 : 1.0)) return n->plan;
     }

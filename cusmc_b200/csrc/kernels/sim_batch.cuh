@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(128, GROUPS ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM
     const uint32_t lane = threadIdx.x & 31u;
     unsigned long long acc_hits = 0, acc_steps = 0, acc_capped = 0;
     uint32_t jb = 0;  // job of this lane's current run
-    bool have = false;
+    bool have = false, drained = false;
     unsigned long long local = 0;  // run index within the job
     uint64_t run = 0;
     float time = 0.0f;
@@ -121,33 +121,38 @@ __global__ void __launch_bounds__(128, GROUPS ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM
     RunScalars sc{0.0, 0.0, 0, 0, -1, 0, 0};
 
     for (;;) {
+        __syncwarp();  // one stream per warp, as in serial_kernel
         // ---- refill finished lanes from the shared run counter
-        const bool need = !have;
-        const unsigned act = __activemask();
-        const unsigned want = __ballot_sync(act, need);
+        const bool need = !have && !drained;
+        const unsigned want = __ballot_sync(0xffffffffu, need);
         if (want) {
             const int leader = __ffs(want) - 1;
             unsigned long long base = 0;
             if (static_cast<int>(lane) == leader) base = atomicAdd(p.queue, static_cast<unsigned long long>(__popc(want)));
-            base = __shfl_sync(act, base, leader);
+            base = __shfl_sync(0xffffffffu, base, leader);
             if (need) {
                 const unsigned long long r = base + __popc(want & ((1u << lane) - 1u));
-                if (r >= p.total_runs) break;
-                const uint32_t j = find_job(jobs, n_jobs, r);
-                if (j != jb) {
-                    flush_counters(jobs[jb], acc_hits, acc_steps, acc_capped);
-                    jb = j;
+                if (r >= p.total_runs) {
+                    drained = true;
+                } else {
+                    const uint32_t j = find_job(jobs, n_jobs, r);
+                    if (j != jb) {
+                        flush_counters(jobs[jb], acc_hits, acc_steps, acc_capped);
+                        jb = j;
+                    }
+                    const BatchJob &J = jobs[jb];
+                    have = true;
+                    local = r - J.run_begin;
+                    run = J.first_run + local;
+                    const Net n = net_view(J.blob, J.net);
+                    run_init<true>(n, J.net.n_comps, J.net.n_vars, rv, sc, J.var_id);
+                    time = 0.0f;
+                    step = 0;
                 }
-                const BatchJob &J = jobs[jb];
-                have = true;
-                local = r - J.run_begin;
-                run = J.first_run + local;
-                const Net n = net_view(J.blob, J.net);
-                run_init<true>(n, J.net.n_comps, J.net.n_vars, rv, sc, J.var_id);
-                time = 0.0f;
-                step = 0;
             }
+            if (__all_sync(0xffffffffu, drained)) break;
         }
+        if (!have) continue;
 
         const BatchJob &J = jobs[jb];
         const Net n = net_view(J.blob, J.net);
@@ -172,8 +177,8 @@ __global__ void __launch_bounds__(128, GROUPS ? CSMC_BATCH_GROUP_MIN_CTAS_PER_SM
 
         const uint32_t P = J.net.n_rate_prog;
         const bool rate_table = (J.net.flags & CSMC_NET_RATE_TABLE) && P > 0;
-        run_step<VERIFY, true, false>(n, C, V, P, J.net.n_clocks, rate_table, rv, sc, J.seed, J.var_id, run, step,
-                                      time);
+        run_step<VERIFY, true, false>(n, C, V, P, J.net.n_clocks, rate_table, rv, sc, SeedDraws{J.seed}, J.seed,
+                                      J.var_id, run, step, time);
     }
     flush_counters(jobs[jb], acc_hits, acc_steps, acc_capped);
 }

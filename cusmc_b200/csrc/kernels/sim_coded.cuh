@@ -46,7 +46,8 @@
 // are gone through afterwards, a run's first with another run's first: as many
 // turns as the run with the most has.  Mutex of 8, 32, 64 and 128 processes,
 // 400,000, 200,000, 100,000 and 65,536 runs: 50 -> 41, 214 -> 143, 131 -> 80
-// and 213 -> 115 ms.
+// and 213 -> 115 ms; with the one-invariant form inline instead of a call, the
+// first three 35, 127 and 70.
 //
 // Results are those of serial_kernel: the same draws, the same race
 // outcome, the same transitions.
@@ -133,7 +134,10 @@ static __device__ __forceinline__ float desc_delay(const Net &n, const CodedView
     const uint64_t dsc = n.loc_desc[li];
     const uint32_t lo = static_cast<uint32_t>(dsc), fl = static_cast<uint32_t>(dsc >> 32);
     if (fl & CSMC_DESC_ZERO) return 0.0f;
-    if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) return bounded_delay(n.base, rv.vars, rv.rates, li, lo, fl, x);
+    float d;
+    if ((fl & CSMC_DESC_INV1) && inv1_uniform(n, rv.vars, li, x, d)) return d;
+    if ((fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) && !(fl & CSMC_DESC_INV1))
+        return bounded_delay(n.base, rv.vars, rv.rates, li, x);
     const float inv = (fl & CSMC_DESC_PROG) ? rv.rates[lo] : __uint_as_float(lo);
     return exp_delay(x, inv);
 }
@@ -183,7 +187,7 @@ static __device__ __noinline__ RaceOutcome coded_race_exact(const uint8_t *base,
                                                             uint64_t run, uint32_t step) {
     const Net n = net_view(base);
     RaceOutcome r;
-    race_exact(n, n.n_comps, ceil_log2(n.n_comps), rv, seed, run, step, r.best, r.d);
+    race_exact(n, n.n_comps, ceil_log2(n.n_comps), rv, SeedBlocks{seed, run, step}, r.best, r.d);
     return r;
 }
 

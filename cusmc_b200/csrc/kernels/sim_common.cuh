@@ -319,13 +319,19 @@ static __device__ __forceinline__ float comp_delay(const Net &n, VarView vars, V
 
 // Delay of a CSMC_DESC_INV1 location (comp_delay's arithmetic for one
 // invariant clock <= / < literal): uniform on (0, bound - clock] while the
-// bound lies ahead, else exponential with the descriptor's 1/rate.
-static __device__ __forceinline__ float inv1_delay(const Net &n, VarView vars, VarView rates, uint32_t li,
-                                                   uint32_t lo, uint32_t fl, uint32_t x) {
+// bound lies ahead (true), else exponential with the descriptor's 1/rate.
+static __device__ __forceinline__ bool inv1_uniform(const Net &n, VarView vars, uint32_t li, uint32_t x, float &d) {
     const uint32_t w = n.loc_inv1[li];
     double ttb = d_sub(n.konst[CSMC_INV1_CONST(w)], static_cast<double>(vars[CSMC_INV1_VAR(w)]));
     if (CSMC_INV1_STRICT(w)) ttb = d_sub(ttb, 1e-6);
-    if (ttb >= 0) return uniform_delay(x, ttb);
+    if (!(ttb >= 0)) return false;
+    d = uniform_delay(x, ttb);
+    return true;
+}
+static __device__ __forceinline__ float inv1_delay(const Net &n, VarView vars, VarView rates, uint32_t li,
+                                                   uint32_t lo, uint32_t fl, uint32_t x) {
+    float d;
+    if (inv1_uniform(n, vars, li, x, d)) return d;
     return exp_delay(x, (fl & CSMC_DESC_PROG) ? rates[lo] : __uint_as_float(lo));
 }
 

@@ -17,14 +17,11 @@
 namespace csmc {
 namespace detail {
 
-// Delay of a component whose descriptor flags INV or EVAL: the one-
-// invariant form inline here, the rest through comp_delay.  One call site
-// per component keeps the race loops' register budget.
+// Delay of a component whose descriptor flags INV (other than INV1) or EVAL.
+// One call site per component keeps the race loops' register budget.
 static __device__ __noinline__ float bounded_delay(const uint8_t *base, VarView vars, VarView rates, uint32_t li,
-                                                   uint32_t lo, uint32_t fl, uint32_t x) {
-    const Net n = net_view(base);
-    if (fl & CSMC_DESC_INV1) return inv1_delay(n, vars, rates, li, lo, fl, x);
-    return comp_delay(n, vars, rates, li, x);
+                                                   uint32_t x) {
+    return comp_delay(net_view(base), vars, rates, li, x);
 }
 
 template <bool LOC8>
@@ -202,33 +199,60 @@ static __device__ __forceinline__ bool run_commit(const Net &n, uint32_t n_clock
     return took;
 }
 
+// A step's Philox blocks, block q of components 4q .. 4q + 3: from the round
+// keys in the kernel's parameter bank (one seed), the counter words the
+// blocks share folded once, or from the seed (a batch job).
+struct BankBlocks {
+    const PhiloxKeys &k;
+    PhiloxStep ps;
+    __device__ __forceinline__ u32x4 operator()(uint32_t q) const { return philox_block(k, ps, q); }
+};
+struct SeedBlocks {
+    uint64_t seed, run;
+    uint32_t step;
+    __device__ __forceinline__ u32x4 operator()(uint32_t q) const { return delay_block(seed, run, step, q); }
+};
+struct BankDraws {
+    const PhiloxKeys &k;
+    __device__ __forceinline__ BankBlocks at(uint32_t step, uint64_t run) const {
+        return BankBlocks{k, philox_step(k, step, run)};
+    }
+};
+struct SeedDraws {
+    uint64_t seed;
+    __device__ __forceinline__ SeedBlocks at(uint32_t step, uint64_t run) const { return SeedBlocks{seed, run, step}; }
+};
+
 // The race over every component (simulation.cu:409-628): per-component
-// delays, minimum of (delay key, bit-reversed index).
-template <class RV>
+// delays, minimum of (delay key, bit-reversed index).  draws(q): the step's
+// Philox block of components 4q .. 4q + 3.  It is bound by issue; a call for
+// the one-invariant form cost as much as the form (random networks of 8 and
+// 24 components, 400,000 and 65,536 runs: 17.1 -> 13.0 and 19.9 -> 16.5 ms).
+template <class RV, class DRAWS>
 static __device__ __forceinline__ void race_exact(const Net &n, uint32_t C, uint32_t bits, const RV &rv,
-                                                  uint64_t seed, uint64_t run, uint32_t step, unsigned long long &best,
-                                                  float &bestd) {
+                                                  const DRAWS &draws, unsigned long long &best, float &bestd) {
     best = ~0ull;
     bestd = 0.0f;
     for (uint32_t c = 0; c < C; c += 4) {
-        const u32x4 blk = delay_block(seed, run, step, c >> 2);
+        const u32x4 blk = draws(c >> 2);
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k) {
             const uint32_t cc = c + k;
             if (cc < C) {
-                // fast path from the location's delay descriptor: the
-                // exponential delay with the literal 1/rate or the step's
-                // evaluated rate; zero-delay types and bounded locations
-                // take the general path
+                // from the location's delay descriptor: one invariant's bound
+                // (inv1_delay) or the exponential delay with the literal
+                // 1/rate or the step's evaluated rate, inline; zero-delay
+                // types and other bounded locations take the general path
                 const uint32_t li = rv.loc(n, cc);
                 const uint64_t dsc = n.loc_desc[li];
                 const uint32_t lo = static_cast<uint32_t>(dsc), fl = static_cast<uint32_t>(dsc >> 32);
                 const uint32_t x = word_of(blk, k);
-                float inv = __uint_as_float(lo);
-                if (fl & CSMC_DESC_PROG) inv = rv.rates[lo];
-                float d = exp_delay(x, inv);
-                if (fl & (CSMC_DESC_ZERO | CSMC_DESC_INV | CSMC_DESC_EVAL))
-                    d = (fl & CSMC_DESC_ZERO) ? 0.0f : bounded_delay(n.base, rv.vars, rv.rates, li, lo, fl, x);
+                float d;
+                if (!((fl & CSMC_DESC_INV1) && inv1_uniform(n, rv.vars, li, x, d))) {
+                    d = exp_delay(x, (fl & CSMC_DESC_PROG) ? rv.rates[lo] : __uint_as_float(lo));
+                    if ((fl & (CSMC_DESC_ZERO | CSMC_DESC_INV | CSMC_DESC_EVAL)) && !(fl & CSMC_DESC_INV1))
+                        d = (fl & CSMC_DESC_ZERO) ? 0.0f : bounded_delay(n.base, rv.vars, rv.rates, li, x);
+                }
                 const unsigned long long key =
                     (static_cast<unsigned long long>(delay_key(d)) << 32) | bitrev_bits(cc, bits);
                 if (key < best) {
@@ -249,16 +273,15 @@ static __device__ __forceinline__ void race_exact(const Net &n, uint32_t C, uint
 // when that cannot be ruled out from the two largest keys (or when a class's
 // 1/rate is not finite and positive and the class could take part in the
 // minimum) the function returns false and the caller runs race_exact.
-template <class RV>
+template <class RV, class DRAWS>
 static __device__ __forceinline__ bool race_classes(const Net &n, uint32_t C, uint32_t bits, const RV &rv,
-                                                    uint64_t seed, uint64_t run, uint32_t step,
-                                                    unsigned long long &best, float &bestd) {
+                                                    const DRAWS &draws, unsigned long long &best, float &bestd) {
     const uint32_t T = rv.T;
     uint32_t pres = 0, pres2 = 0;
     best = ~0ull;
     bestd = 0.0f;
     for (uint32_t c = 0; c < C; c += 4) {
-        const u32x4 blk = delay_block(seed, run, step, c >> 2);
+        const u32x4 blk = draws(c >> 2);
 #pragma unroll
         for (uint32_t k = 0; k < 4; ++k) {
             const uint32_t cc = c + k;
@@ -288,7 +311,8 @@ static __device__ __forceinline__ bool race_classes(const Net &n, uint32_t C, ui
                     if (fl & CSMC_DESC_ZERO) {
                         d = 0.0f;
                     } else if (fl & (CSMC_DESC_INV | CSMC_DESC_EVAL)) {
-                        d = bounded_delay(n.base, rv.vars, rv.rates, li, lo, fl, x);
+                        d = (fl & CSMC_DESC_INV1) ? inv1_delay(n, rv.vars, rv.rates, li, lo, fl, x)
+                                                  : bounded_delay(n.base, rv.vars, rv.rates, li, x);
                     } else {
                         const float inv = (fl & CSMC_DESC_PROG) ? rv.rates[lo] : __uint_as_float(lo);
                         d = exp_delay(x, inv);
@@ -336,9 +360,9 @@ static __device__ __forceinline__ bool race_classes(const Net &n, uint32_t C, ui
 // One step of a run: pending broadcast receivers, the per-step rate table,
 // the race, the clock advance and the winner's transition, the time update.
 // CLASSES: the network's descriptors carry race classes (C <= 256).
-template <bool VERIFY, bool SLOTS, bool CLASSES, class RV>
+template <bool VERIFY, bool SLOTS, bool CLASSES, class RV, class KEYS>
 static __device__ __forceinline__ void run_step(const Net &n, uint32_t C, uint32_t V, uint32_t P, uint32_t n_clocks,
-                                                bool rate_table, const RV &rv, RunScalars &sc,
+                                                bool rate_table, const RV &rv, RunScalars &sc, const KEYS &keys,
                                                 uint64_t seed, int var_id, uint64_t run, uint32_t &step,
                                                 float &time) {
     const uint32_t bits = ceil_log2(C);
@@ -351,11 +375,12 @@ static __device__ __forceinline__ void run_step(const Net &n, uint32_t C, uint32
     // ---- delays and the race
     unsigned long long best;
     float bestd;
+        const auto draws = keys.at(step, run);
     if (CLASSES) {
-        if (!race_classes(n, C, bits, rv, seed, run, step, best, bestd))
-            race_exact(n, C, bits, rv, seed, run, step, best, bestd);
+        if (!race_classes(n, C, bits, rv, draws, best, bestd))
+            race_exact(n, C, bits, rv, draws, best, bestd);
     } else {
-        race_exact(n, C, bits, rv, seed, run, step, best, bestd);
+        race_exact(n, C, bits, rv, draws, best, bestd);
     }
     const uint32_t win = bitrev_bits(static_cast<uint32_t>(best & 0xffffffffull), bits);
     run_commit<VERIFY, SLOTS>(n, n_clocks, rv, sc, seed, var_id, run, step, time, win, bestd);
