@@ -254,7 +254,7 @@ csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
         }
     }
     if (n->thread_warps > 0) {
-        const double S = n->plan.family != 4 ? 29.0 + 3.9 * C : n->only_classes ? 48.0 + 0.7 * C : 48.0 + 1.9 * C;
+        const double S = n->plan.family != 4 ? 29.0 + 3.9 * C : n->all_classed ? 48.0 + 0.7 * C : 48.0 + 1.9 * C;
         const double t =
             launch_time(S, std::ceil(runs / 32.0), n->plan.family != 4 ? 3.6 : 2.8, n->thread_warps, 10.0);
         // (where both fill the GPU a group is taken only when it is clearly the better one)
@@ -595,8 +595,6 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
             }
             n->class_src[g] = (fl & CSMC_DESC_PROG) ? (CSMC_CLASS_SRC_PROG | lo) : lo;
         }
-        n->only_classes = n->all_classed;
-        n->all_classed = n->all_classed && h->n_comps % 4 == 0;
         // tilt groups of importance sampling one thread per run: the
         // (race class, location class) pairs in order of first appearance,
         // the first CSMC_IS_GROUPS of them; later pairs take the

@@ -48,8 +48,7 @@ struct csmc_net {
     bool slots = false;
     bool loc8 = false;     // every automaton has at most 256 locations
     bool classes = false;  // delay descriptors carry race classes
-    bool only_classes = false; // every location belongs to a race class
-    bool all_classed = false;  // every location belongs to a race class, components a multiple of four
+    bool all_classed = false;  // every location belongs to a race class
     uint32_t class_src[CSMC_RACE_CLASSES] = {};  // 1/rate source of each class (SimParams::class_src)
     uint8_t *d_state = nullptr;  // thread-per-run state slabs (global-state plans)
     size_t state_bytes = 0;
@@ -66,7 +65,7 @@ struct csmc_net {
     // importance sampling one thread per run (sim_is_coded.cuh): the tilt
     // groups of the network (is_groups < 0: the network does not qualify)
     int is_groups = -1;
-    bool is_all_grouped = false;  // every location in a tilt group, components a multiple of 4
+    bool is_all_grouped = false;  // every location in a tilt group
     uint64_t is_group_map = 0;
     uint32_t is_group_l = 0;
     uint32_t is_group_src[CSMC_IS_GROUPS] = {};

@@ -112,14 +112,17 @@ bool plan_is_coded(const csmc_net *n, uint64_t n_runs, Launch &L) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device) != cudaSuccess)
         return false;
     // a small launch is bound by its single runs' steps, which one warp per
-    // run takes faster.  The crossover, measured on the epidemic under a
-    // trained proposal: with every location in a tilt group (no descriptor
-    // path), one thread per run takes ~45 ms per launch up to a full GPU
-    // and one warp per run ~6.1 us per run (5e3 runs: 44.5 against 33.4 ms;
-    // 1e4 runs: 45.3 against 60.8 ms), so one thread per run from 48 runs
-    // per SM; with the descriptor path, from 128 runs per SM (1e4 runs:
-    // 134k runs/s against 165k; 2e4 runs: 242k against 179k)
-    const uint64_t min_runs = (n->is_all_grouped ? 48ull : 128ull) * static_cast<uint64_t>(sms);
+    // run takes faster.  One thread per run / one warp per run, epidemics
+    // under a trained proposal: 99 agents 10,000 runs 35 / 21 ms, 19,000 runs
+    // 36 / 38; 49 agents 14,000 runs 18.3 / 17.1, 19,000 runs 18.6 / 22.9; 23
+    // agents 10,000 runs 7.3 / 6.3, 14,000 runs 7.6 / 8.5: from 100 runs per SM
+    // where every location is in a tilt group.  A multiple of four components
+    // keeps 48, the crossing before the one-warp kernel kept its sums (it was
+    // 60.8 ms at 1e4 runs of 100 agents): which kernel runs there is reported
+    // to the caller.  With the descriptor path, from 128 (1e4 runs: 134k runs/s
+    // against 165k; 2e4 runs: 242k against 179k)
+    const uint64_t per_sm = !n->is_all_grouped ? 128 : h.n_comps % 4 ? 100 : 48;
+    const uint64_t min_runs = per_sm * static_cast<uint64_t>(sms);
     if (n->is_kernel == 0 && n_runs < min_runs) return false;
     // threads per CTA: 384 (one CTA, twelve warps per SM) from 1.5 runs
     // per thread of such a grid, 128 (two CTAs per SM) when the runs fill

@@ -116,8 +116,7 @@ int serial_max_active_ctas(bool verify, bool slots, bool loc8, bool gstate, bool
 // Class-coded thread-per-run kernel (sim_coded.cuh): networks with race
 // classes, at most 256 components and at most 32 locations per automaton,
 // run state in shared memory.
-// all_classed: every location of the network belongs to a race class and the
-// component count is a multiple of four.
+// all_classed: every location of the network belongs to a race class.
 int coded_launch(bool verify, bool slots, bool all_classed, const SimParams &p, int grid, int block, size_t smem,
                  void *stream);
 int coded_max_active_ctas(bool verify, bool slots, bool all_classed, int block, size_t smem, int *ctas);

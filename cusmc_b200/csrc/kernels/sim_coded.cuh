@@ -177,6 +177,15 @@ static __device__ __forceinline__ void race_block(const CodedView &rv, uint32_t 
     st_key(a3 + 3u * kKeyChain, max(o3, key(x.w, 3u)));
 }
 
+// The last block of a network of 4 Q + m components, m = 1 .. 3 (all lanes
+// alike), all of them class members: a0, a1, a2 are the members' key addresses.
+static __device__ __forceinline__ void race_tail(uint32_t m, uint32_t a0, uint32_t a1, uint32_t a2, const u32x4 &x,
+                                                 uint32_t cb) {
+    st_key(a0, max(ld_key(a0), (x.x & 0xffffff00u) | cb));
+    if (m > 1u) st_key(a1, max(ld_key(a1), (x.y & 0xffffff00u) | cb));
+    if (m > 2u) st_key(a2, max(ld_key(a2), (x.z & 0xffffff00u) | cb));
+}
+
 // race_exact out of line: the view of the network is rebuilt, the run state's
 // view passed by value.
 struct RaceOutcome {
@@ -194,8 +203,8 @@ static __device__ __noinline__ RaceOutcome coded_race_exact(const uint8_t *base,
 // The race decided from the class keys (race_classes' decision over the
 // same keys); false: the caller runs race_exact.  src: each class's 1/rate
 // source (CSMC_CLASS_SRC_PROG | slot, or float bits).  ALLCLS: every
-// location is classed and the component count is a multiple of four, so no
-// block has a general member or padding.
+// location is classed, so no block has a general member; the padding of a last
+// block of one to three components is left out there.
 template <bool ALLCLS>
 static __device__ __forceinline__ bool race_coded(const Net &n, uint32_t C, uint32_t bits, uint32_t NG,
                                                   const CodedView &rv, const PhiloxKeys &K, const uint32_t *src,
@@ -211,7 +220,7 @@ static __device__ __forceinline__ bool race_coded(const Net &n, uint32_t C, uint
     // bit reversal of component 4q + k over `bits` (>= 2) bits: the two low
     // bits (k) become the top two, q the low bits - 2 reversed
     const uint32_t hi_shift = bits - 2u;  // bits >= 2: the plan needs at least four components
-    const uint32_t Q = (C + 3u) >> 2;
+    const uint32_t Q = ALLCLS ? C >> 2 : (C + 3u) >> 2;
     // members outside the classes: the blocks that have some, their draws
     uint64_t general_blocks = 0;
     uint32_t n_general = 0, draws[ALLCLS ? 1 : kMaxCodedComps];
@@ -232,6 +241,12 @@ static __device__ __forceinline__ bool race_coded(const Net &n, uint32_t C, uint
                 if (general & 0x80000000u) draws[n_general++] = blk.w;
             }
         }
+    }
+    if (ALLCLS && (C & 3u)) {
+        const uint32_t wd = rv.lw[Q * T];
+        const u32x4 blk = philox_block(K, ps, Q);
+        race_tail(C & 3u, key_addr<0>(rv, wd), key_addr<1>(rv, wd) + kKeyChain, key_addr<2>(rv, wd) + 2u * kKeyChain, blk,
+                  255u - (__brev(Q) >> (32u - hi_shift)));
     }
     // their delays, one member of each run at a time: a warp goes through as
     // many as its run with the most has, not through every component that is

@@ -1,0 +1,73 @@
+"""Class-coded races of networks whose last Philox block is partly filled, and
+of networks with members outside the classes (none, some or all components of
+a block at a time): traces and importance-sampling runs equal the CPU
+oracle's bit for bit."""
+import os
+import tempfile
+
+import numpy as np
+import pytest
+
+import oracle
+from cusmc_b200 import api, netgen
+from cusmc_b200 import proposal as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _blob(w):
+    with tempfile.NamedTemporaryFile("w", suffix=".xml", delete=False) as f:
+        f.write(w.xml)
+    try:
+        return api.compile_model(f.name)
+    finally:
+        os.unlink(f.name)
+
+
+NETS = {f"epidemic{n}": (lambda n=n: netgen.epidemic(n_agents=n, horizon=20, r_threshold=max(1, n // 3)))
+        for n in (4, 5, 6, 7, 33, 99, 254, 255)}
+NETS.update({f"mutex{n}": (lambda n=n: netgen.mutex(n, horizon=8)) for n in (4, 5, 6, 7, 33, 66)})
+
+
+@pytest.mark.parametrize("name", sorted(NETS))
+def test_class_coded_traces_match_the_oracle(name):
+    w = NETS[name]()
+    blob = _blob(w)
+    q = api.variable_query(w.var_id, w.horizon, threshold=w.threshold, is_max=True, max_steps=3000)
+    m = 200
+    _, want, _ = oracle.run(blob, q, 13, m, threads=0, digests=True, final_state=True)
+    net = api.Network(blob)
+    try:
+        net.set_plan(4, 1, 1, 64)
+        r, got = net.run_verify(q, 13, m)
+        assert r.family == 4
+    finally:
+        net.close()
+    for key in ("steps", "flags", "digests", "final_state"):
+        assert np.array_equal(got[key], want[key]), key
+    assert np.array_equal(got["values"].view(np.uint64), want["values"].view(np.uint64))
+
+
+@pytest.mark.parametrize("name", sorted(n for n in NETS if n not in ("epidemic254", "mutex66")))
+def test_weighted_runs_match_the_oracle(name):
+    import torch
+    w = NETS[name]()
+    blob = _blob(w)
+    q = api.variable_query(w.var_id, w.horizon, threshold=w.threshold, is_max=True, max_steps=3000)
+    prop = P.Proposal.init(3)
+    prop.w3 = (np.random.default_rng(4).standard_normal(P.HID) * 0.1).astype(np.float32)
+    params = prop.pack()
+    m = 200
+    cpu, _ = oracle.is_run(blob, q, params, 17, m, 40)
+    net = api.Network(blob)
+    try:
+        P.set_inference(net, False)
+        P.set_kernel(net, 5)
+        logw = torch.zeros(m, dtype=torch.float64, device="cuda")
+        steps = torch.zeros(m, dtype=torch.int32, device="cuda")
+        r = P.is_run(net, q, params, 17, m, 40, logw=logw, steps=steps)
+        assert r.family == 5
+    finally:
+        net.close()
+    assert np.array_equal(steps.cpu().numpy().view(np.uint32), cpu["steps"])
+    assert np.array_equal(logw.cpu().numpy().view(np.uint64), cpu["logw"].view(np.uint64))
