@@ -80,13 +80,23 @@ bool configure_plan(const csmc_net *n, csmc_launch_plan &p, int family, int lane
         }
         // per-group run state: 48 bytes of scalars, the variables, one
         // inverse rate per rate program, then the components' delay records,
-        // slot masks and locations
+        // slot masks and locations.  A plan is taken when the network, the
+        // groups' variables and their slot masks fit in shared memory; where
+        // the records and locations do not fit beside them, with fewer groups
+        // per CTA (random network of 500 components, 32 x 16: 128 threads for
+        // 256), and where a single warp's do not, one thread per run
         const uint32_t stride = csmc::group_state_stride(h.n_vars, h.n_rate_prog, lanes, cpl);
-        const size_t smem = n->bytes + static_cast<size_t>(block / lanes) * stride;
-        if (smem > max_smem) {
+        const size_t least = csmc::group_vars_bytes(h.n_vars, h.n_rate_prog) + 4u * static_cast<size_t>(lanes) * cpl;
+        if (n->bytes + static_cast<size_t>(block / lanes) * ((least + 15u) & ~static_cast<size_t>(15)) > max_smem) {
             why = "network and run state do not fit in shared memory";
             return false;
         }
+        const auto smem_of = [&](int b) { return n->bytes + static_cast<size_t>(b / lanes) * stride; };
+        const int asked = block;
+        while (block > 32 && smem_of(block) > max_smem) block = block % 64 ? 32 : block / 2;
+        const size_t smem = smem_of(block);
+        if (smem > max_smem)
+            return configure_plan(n, p, 1, 1, static_cast<int>(h.n_comps), std::min(asked, 128), why);
         p.family = 0;
         p.lanes = lanes;
         p.comps_per_lane = cpl;
@@ -107,12 +117,19 @@ bool configure_plan(const csmc_net *n, csmc_launch_plan &p, int family, int lane
             return false;
         }
         const csmc::NetLayout L = csmc::layout_of(h);
-        const size_t slab = csmc::coded_slab_bytes(h.n_comps, h.n_vars, h.n_rate_prog, n->slots, block, L.n_classes,
-                                                   (h.recv_chan_lo | h.recv_chan_hi) != 0, CSMC_CODED_KEY_BYTES);
-        if (n->bytes + slab > max_smem) {
+        const auto slab_of = [&](uint32_t key_bytes) {
+            return csmc::coded_slab_bytes(h.n_comps, h.n_vars, h.n_rate_prog, n->slots, block, L.n_classes,
+                                          (h.recv_chan_lo | h.recv_chan_hi) != 0, key_bytes);
+        };
+        const size_t slab = slab_of(CSMC_CODED_KEY_BYTES);
+        if (n->bytes + slab_of(16u * block) > max_smem) {
             why = "network and run state do not fit in shared memory";
             return false;
         }
+        // CTAs of fewer than 128 threads keep the key space of 128: where only
+        // that does not fit, the general one-thread-per-run kernel
+        if (n->bytes + slab > max_smem)
+            return configure_plan(n, p, 1, 1, static_cast<int>(h.n_comps), block, why);
         p.family = 4;
         p.lanes = 1;
         p.comps_per_lane = static_cast<int>(h.n_comps);
@@ -231,6 +248,24 @@ void find_shapes(csmc_net *n) {
 // (to time 60) 16,000 runs 6.6 / 3.9, 32,768 runs 7.0 / 7.5; random 64 (to time
 // 20) 131,072 runs 75 / 34.
 csmc_launch_plan launch_plan(const csmc_net *n, uint64_t n_runs) {
+    if (n->plan.state_in_global && !n->plan_forced && n->h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS) {
+        // the network or the state of one thread per run is beyond shared
+        // memory: the batch kernel's warp-per-run form at every size, the
+        // network read through the caches.  One thread per run with its state in
+        // global memory / one warp per run, random networks to time 5: 507
+        // components 100 runs 366 / 4.3 ms, 20,000 runs 451 / 54; 303
+        // components 110 / 1.9, 137 / 24; 364 components (the network fits, its
+        // state does not) 141 / 2.2, 247 / 27
+        csmc_launch_plan p;
+        p.family = 2;
+        p.lanes = 32;
+        p.comps_per_lane = n->h.n_comps <= 128 ? 4 : n->h.n_comps <= 256 ? 8 : 16;
+        p.block = 128;
+        p.state_stride = csmc::group_state_stride(n->h.n_vars + n->h.n_rate_prog, 0, 32, p.comps_per_lane);
+        p.smem = csmc::batch_smem_bytes(1, p.state_stride, p.block);
+        p.state_in_global = false;
+        if (p.smem <= static_cast<size_t>(max_smem_optin(n->device))) return p;
+    }
     if (n->plan_forced || n->plan.family == 2 || n->n_shapes == 0) return n->plan;
     const double C = n->h.n_comps, unit = 128.0 * n->sms, runs = static_cast<double>(n_runs);
     const bool even = n->h.n_clocks > 0;
@@ -353,7 +388,7 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
     p.keys = csmc::philox_keys(seed);
     for (int g = 0; g < CSMC_RACE_CLASSES; ++g) p.class_src[g] = n->class_src[g];
     int rc = pl.family == 0 ? csmc::sim_max_active_ctas(pl.lanes, pl.comps_per_lane, verify, pl.block, pl.smem, &ctas)
-             : pl.family == 2 ? csmc::batch_max_active_ctas(verify, 0, pl.block, pl.smem, &ctas)
+             : pl.family == 2 ? csmc::batch_max_active_ctas(verify, pl.lanes == 32 ? pl.comps_per_lane : 0, pl.block, pl.smem, &ctas)
              : pl.family == 4 ? csmc::coded_max_active_ctas(verify, n->slots, n->all_classed, pl.block, pl.smem, &ctas)
                               : csmc::serial_max_active_ctas(verify, n->slots, n->loc8, pl.state_in_global, n->classes,
                                                              pl.block, pl.smem, &ctas);
@@ -402,7 +437,15 @@ int run_impl(const csmc_net *cn, const csmc_query *q, uint64_t seed, uint64_t fi
         bp.jobs = n->d_job;
         bp.n_jobs = 1;
         bp.state_stride = pl.state_stride;
-        bp.total_runs = n_runs;
+        if (pl.lanes == 32) {  // one warp per run
+            bp.n_group_jobs = 1;
+            bp.group_runs = n_runs;
+            bp.group_queue = n->d_scratch;
+            bp.group_stride = pl.state_stride;
+            bp.group_k = static_cast<uint32_t>(pl.comps_per_lane);
+        } else {
+            bp.total_runs = n_runs;
+        }
         bp.queue = n->d_scratch;
         bp.state = n->d_state;
         bp.max_vars = n->h.n_vars;

@@ -658,6 +658,16 @@ int csmc_autotune(csmc_net *n, const csmc_query *q, uint64_t seed, uint64_t prob
             pick[3] = c.block;
         }
     }
+    if (!saved_forced && saved.state_in_global) {
+        // a network beyond shared memory: its default (launch_plan) may be none of these
+        n->plan = saved;
+        n->plan_forced = false;
+        if (csmc_run(n, q, seed, 0, probe_runs, nullptr, nullptr, nullptr, &r, nullptr) == CSMC_OK &&
+            (!have || r.kernel_ms < top.kernel_ms)) {
+            *best = r;
+            return CSMC_OK;
+        }
+    }
     if (!have) {
         n->plan = saved;
         n->plan_forced = saved_forced;

@@ -71,13 +71,15 @@ int plan_is(const csmc_net *n, bool trace, uint64_t n_runs, Launch &L) {
     L.loc8 = h.max_locs_per_comp <= 256;
     const size_t per = csmc::serial_state_bytes_per_thread(h.n_comps, h.n_vars, h.n_rate_prog, L.slots, L.loc8);
     const bool recv = (h.recv_chan_lo | h.recv_chan_hi) != 0;
-    L.plain = n->is_plain;
-    L.slab = static_cast<uint32_t>(L.plain ? csmc::is_plain_slab_bytes(h.n_comps, h.n_vars, h.n_rate_prog, recv, n->is_tc)
-                                           : csmc::is_warp_slab_bytes(per, n->is_tc));
     const size_t base = n->bytes + csmc::is_mlp_smem_bytes();
     int max_smem = 0, sms = 0, ctas = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, n->device), "device attribute");
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device), "device attribute");
+    // (what the kernel of networks without invariants keeps between steps
+    // takes more shared memory; where one run's does not fit, the other one)
+    const size_t plain_slab = csmc::is_plain_slab_bytes(h.n_comps, h.n_vars, h.n_rate_prog, recv, n->is_tc);
+    L.plain = n->is_plain && base + plain_slab <= static_cast<size_t>(max_smem);
+    L.slab = static_cast<uint32_t>(L.plain ? plain_slab : csmc::is_warp_slab_bytes(per, n->is_tc));
     int warps = CSMC_IS_BLOCK / 32;
     // few runs: CTAs of fewer warps, spread over the SMs (a run's steps are a
     // serial chain: it gains from a scheduler of its own)

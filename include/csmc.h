@@ -176,8 +176,9 @@ int csmc_plan(const csmc_net *net, int32_t *lanes_per_run, int32_t *comps_per_la
  * network and run state in global memory (networks larger than shared
  * memory); family 1 = one thread per run; family 4 = one thread per run with
  * class-coded locations (networks with race classes, at most 256 components
- * and 32 locations per automaton; the default for them).  For families 1, 2
- * and 4 lanes and comps_per_lane are ignored.  threads_per_cta: CTA size.
+ * and 32 locations per automaton; their default for large launches).  For
+ * families 1, 2 and 4 lanes and comps_per_lane are ignored.  threads_per_cta:
+ * CTA size (lane groups take a smaller one where shared memory asks for it).
  * Every family gives the same per-run results. */
 int csmc_set_plan(csmc_net *net, int32_t family, int32_t lanes_per_run, int32_t comps_per_lane,
                   int32_t threads_per_cta);

@@ -1,6 +1,7 @@
 """Class-coded races of networks whose last Philox block is partly filled, and
 of networks with members outside the classes (none, some or all components of
-a block at a time): traces and importance-sampling runs equal the CPU
+a block at a time), and lane groups of the largest networks: traces and
+importance-sampling runs equal the CPU
 oracle's bit for bit."""
 import os
 import tempfile
@@ -71,3 +72,44 @@ def test_weighted_runs_match_the_oracle(name):
         net.close()
     assert np.array_equal(steps.cpu().numpy().view(np.uint32), cpu["steps"])
     assert np.array_equal(logw.cpu().numpy().view(np.uint64), cpu["logw"].view(np.uint64))
+
+
+@pytest.mark.parametrize("n_comps", [450, 500])
+def test_lane_groups_of_networks_near_the_shared_memory_limit(n_comps):
+    """The network, the variables and the slot masks of a 256-thread CTA's
+    groups fit, their delay records do not: lane groups all the same."""
+    w = netgen.random_network(8, n_comps=n_comps, horizon=1)
+    blob = _blob(w)
+    q = api.variable_query(w.var_id, w.horizon, threshold=w.threshold, is_max=True, max_steps=300)
+    _, want, _ = oracle.run(blob, q, 13, 40, threads=0, digests=True, final_state=True)
+    net = api.Network(blob)
+    try:
+        for plan in (None, (0, 32, 16, 256), (0, 32, 16, 64)):
+            if plan:
+                net.set_plan(*plan)
+            r, got = net.run_verify(q, 13, 40)
+            assert (r.family, r.lanes_per_run) == (0, 32)
+            for key in ("steps", "flags", "digests", "final_state"):
+                assert np.array_equal(got[key], want[key]), (plan, key)
+    finally:
+        net.close()
+
+
+def test_networks_beyond_shared_memory_run_a_warp_per_run():
+    w = max(netgen.batch_networks(64, base_seed=1000), key=lambda w: len(w.xml))
+    blob = _blob(w)
+    assert len(blob) > 232_448
+    q = api.variable_query(w.var_id, 1, threshold=w.threshold, is_max=True, max_steps=300)
+    _, want, _ = oracle.run(blob, q, 13, 40, threads=0, digests=True, final_state=True)
+    net = api.Network(blob)
+    try:
+        for plan, lanes in ((None, 32), ((2, 1, 1, 128), 1)):
+            if plan:
+                net.set_plan(*plan)
+            r, got = net.run_verify(q, 13, 40)
+            assert (r.family, r.lanes_per_run) == (2, lanes)
+            for key in ("steps", "flags", "digests", "final_state"):
+                assert np.array_equal(got[key], want[key]), (plan, key)
+            assert np.array_equal(got["values"].view(np.uint64), want["values"].view(np.uint64))
+    finally:
+        net.close()
