@@ -276,8 +276,7 @@ def run_ours(args):
     peak, peak_kind = load_peaks()
     info = api.blob_info(blob)
     n_comps = info["n_comps"]
-    plan = net.plan()
-    lanes, cpl, rpc = plan
+    lanes, cpl, rpc = r.lanes_per_run, r.comps_per_lane, r.runs_per_cta  # of the launch (chosen by its runs)
     launch_ms = t_kernel / args.steps
     # algorithmic HBM bytes of one simulation launch: one flag byte and one
     # 8-byte value per run written, the network read once

@@ -130,7 +130,8 @@ bool plan_is_coded(const csmc_net *n, uint64_t n_runs, Launch &L) {
     // per thread of such a grid, 128 (two CTAs per SM) when the runs fill
     // two of those per SM; a launch of fewer runs is bound by the steps of
     // single runs, and smaller CTAs (64, 32) spread its warps over more SMs.
-    // Measured on the epidemic under a trained proposal: 1e6 runs 1.27M
+    // Measured on the epidemic under a trained proposal, before the sums were
+    // the warp's (now 1.96M and 1.41M at 1e6 and 1e5 runs): 1e6 runs 1.27M
     // runs/s with 384 threads against 1.04M with 128; 1e5 runs 886k
     // against 901k, and ten CE rounds of 1e5 runs 3.6 % faster in all
     const bool recv = (h.recv_chan_lo | h.recv_chan_hi) != 0;

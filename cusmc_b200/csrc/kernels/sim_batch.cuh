@@ -23,8 +23,8 @@
 // Memory.  Networks stay in global memory (read-only, L1/L2-resident while
 // in use); each CTA's thread-per-run state is a global slab laid out for the
 // largest thread-per-run job (interleaved by thread, so warp accesses
-// coalesce); a warp-per-run run keeps its scalars, variables and rate table
-// in shared memory after the job table.  Results depend only on the job and
+// coalesce); a warp-per-run run keeps its state (GroupRun) in shared memory
+// after the job table.  Results depend only on the job and
 // the run index, never on which mode ran it.
 #pragma once
 #include "sim_impl.cuh"

@@ -22,9 +22,9 @@
 // runs end at different steps keep advancing together.
 // Measured (B200), against the form with a 64-bit butterfly, per-component
 // location records read every step and every step's rate table evaluated:
-// 100 agents, 32 lanes x 4, 64 runs 9.3 -> 3.0 ms, 65,536 runs 142 -> 49 ms
-// (355 warp instructions a step); 256-process mutex, 32 x 8, 2,000 runs
-// 237 -> 157 ms (1,370 -> 729 instructions a step).
+// 100 agents, 32 lanes x 4, 64 runs 9.3 -> 2.7 ms, 65,536 runs 142 -> 45 ms;
+// 256-process mutex, 32 x 8, 2,000 runs 237 -> 80 ms (1,370 -> 685 warp
+// instructions a step).
 #pragma once
 #include "sim_common.cuh"
 

@@ -2,7 +2,7 @@
 //
 // Every thread simulates one run at a time and walks that run's components
 // in a loop, so a warp advances 32 independent runs in lockstep through the
-// same instruction stream: no shuffles, no warp barriers, and the winner's
+// same instruction stream: no shuffles, one warp barrier a step, and the winner's
 // transition is executed by all 32 lanes for their own runs at once.  A lane
 // whose run ends takes the next run index from the device work counter
 // immediately (warp-aggregated atomic), so uneven run lengths do not idle the
