@@ -202,6 +202,7 @@ extern "C" int csmc_run_noalloc(const void *blob_host, const void *blob_device, 
         p.horizon = static_cast<float>(q->horizon);
         p.max_steps = q->max_steps ? q->max_steps : 10000000ull;
         p.seed = seed;
+        p.keys = csmc::philox_keys(seed);  // (the kernel draws from the round keys)
         p.first_run = first_run;
         p.n_runs = n_runs;
         p.flags = flags;
