@@ -152,12 +152,15 @@ struct GroupRun {
 #pragma unroll 1
         for (uint32_t k = 0; k < kn; ++k) {
             const uint32_t c = comp_of(k);
-            if (c < n.n_comps) look_up(n, static_cast<int>(k), locv[c]);
+            if (c < n.n_comps) look_up<true>(n, static_cast<int>(k), locv[c]);
             else *rec_of(static_cast<int>(k)) = make_uint2(0x7fffffffu, kFormExp);  // no component: a delay of NaN
         }
     }
 
-    // Writes component k's record from its location li.
+    // Writes component k's record from its location li.  RATE false: a rate
+    // from the table is left out (the next step evaluates the table and writes
+    // it, and other lanes may be storing that table already).
+    template <bool RATE>
     __device__ __forceinline__ void look_up(const Net &n, int k, uint32_t li) {
         const uint64_t dsc = n.loc_desc[li];
         const uint32_t lo = static_cast<uint32_t>(dsc), fl = static_cast<uint32_t>(dsc >> 32);
@@ -174,7 +177,7 @@ struct GroupRun {
             }
             if (fl & CSMC_DESC_PROG) {
                 pm |= 1u << k;
-                inv = __float_as_uint(rates[lo]);
+                if (RATE) inv = __float_as_uint(rates[lo]);
             }
         }
         *rec_of(k) = make_uint2(inv, form);
@@ -227,6 +230,7 @@ struct GroupRun {
         pm = 0;
         eval_rates(n);
         look_up_all(n);
+        __syncwarp(gmask);  // before the first step may evaluate the rate table again
         dirty = false;
         draw(keys, run, 0u);
     }
@@ -248,6 +252,10 @@ struct GroupRun {
         const int sender = s->sc.sender;
         uint32_t *const rmv = reinterpret_cast<uint32_t *>(rec);  // the records are written again below
         const uint32_t kn = n_k(C), kmax = !kStrided ? B * NB : 4u * (((C + 3u) >> 2) + G - 1u) / G;
+        // the masks overwrite the records: one lane's mask lies in another
+        // lane's record, which that lane may have written at the end of the
+        // step before
+        __syncwarp(gmask);
 #pragma unroll 1
         for (uint32_t k = 0; k < kn; ++k) {
             const uint32_t c = comp_of(k);
@@ -467,7 +475,7 @@ struct GroupRun {
                 dirty = true;
                 chan = static_cast<uint32_t>(s->sc.chan);
                 goal = static_cast<uint32_t>(s->sc.goal);
-                if (gl == owner) look_up(n, k_of(win), locv[win]);
+                if (gl == owner) look_up<false>(n, k_of(win), locv[win]);
             } else if (VERIFY && gl == 0) {
                 mix(s->sc.digest, 0xffffffffu);
             }
