@@ -54,6 +54,8 @@ struct csmc_batch {
     uint8_t *d_state = nullptr;
     size_t state_bytes = 0;
     int block = 128, ctas_per_sm = 0, grid = 0;
+    int threads = 128;                 // threads per CTA in effect: `block`, fewer where shared memory asks for it
+    size_t max_smem = 0;               // shared memory a CTA of the device can have
     uint32_t state_stride = 0;
     cudaStream_t cap = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -97,6 +99,30 @@ void drop_graph(csmc_batch *b) {
     b->exec = nullptr;
 }
 
+// Shared memory of a launch in which the networks of min_comps components and
+// more run one warp per run: as it is laid out, and without the records and
+// locations.
+struct GroupSmem {
+    int k = 0;            // components per lane
+    uint32_t stride = 0;  // of one warp
+    size_t least = 0;     // a CTA's, without the records, the locations and a table entry's first clock (16 bytes)
+};
+GroupSmem group_smem(const csmc_batch *b, uint32_t min_comps) {
+    uint32_t max_c = 0, max_vp = 0;
+    for (const csmc_net *n : b->nets)
+        if (min_comps > 0 && n->h.n_comps >= min_comps && n->h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS) {
+            max_c = std::max(max_c, n->h.n_comps);
+            max_vp = std::max(max_vp, n->h.n_vars + n->h.n_rate_prog);
+        }
+    GroupSmem g;
+    if (max_c == 0) return g;
+    g.k = max_c <= 128 ? 4 : max_c <= 256 ? 8 : 16;
+    g.stride = csmc::group_state_stride(max_vp, 0, 32, g.k);
+    g.least = csmc::batch_smem_bytes(b->n_jobs, csmc::group_vars_bytes(max_vp, 0) + 4u * 32u * g.k, b->block) -
+              16u * static_cast<size_t>(b->n_jobs);
+    return g;
+}
+
 // Which jobs run one warp per run (networks of group_min_comps ..
 // CSMC_BATCH_GROUP_MAX_COMPS components), the job-table order (those jobs
 // first, each part by falling cost), the lanes' component count and the
@@ -111,11 +137,20 @@ void drop_graph(csmc_batch *b) {
 // networks); a warp's step takes 2 + 4 ceil(C / 128) issue slots and 4.4 (3 +
 // 4 ceil(C / 128)) of latency, 32 threads' step 1 + 1.85 C (latency 5 times
 // that); each part lasts max(longest run, work / schedulers).  In units of
-// launch_plan (capi.cu).
+// launch_plan (capi.cu).  A threshold whose runs' state does not fit in
+// shared memory beside the job table is passed over.
+//
+// A threshold (the default one or the caller's) is taken when the job table,
+// the groups' variables and their slot masks fit in shared memory; where the
+// delay records and locations do not fit beside them, with fewer warps per
+// CTA, and where a single warp's do not, every job runs one thread per run.
 uint32_t auto_min_comps(const csmc_batch *b) {
     double best = -1.0;
     uint32_t pick = b->group_min_comps;
     for (uint32_t m : {b->group_min_comps, 64u, 32u, 16u, 8u, 4u}) {
+        if (m != b->group_min_comps &&
+            csmc::batch_smem_bytes(b->n_jobs, group_smem(b, m).stride, b->block) > b->max_smem)
+            continue;
         double warp_work = 0, warp_long = 0, thread_work = 0, thread_long = 0;
         for (int j = 0; j < b->n_jobs; ++j) {
             const double C = b->nets[j]->h.n_comps, runs = static_cast<double>(b->n_runs[j]);
@@ -143,24 +178,32 @@ void assign_modes(csmc_batch *b) {
     b->group.assign(b->n_jobs, 0);
     b->n_group = 0;
     b->max_v = b->max_p = b->max_c = 0;
-    uint32_t gmax_c = 0, gmax_vp = 0;
-    const uint32_t min_comps = b->group_auto ? auto_min_comps(b) : b->group_min_comps;
+    uint32_t min_comps = b->group_auto ? auto_min_comps(b) : b->group_min_comps;
+    GroupSmem g = group_smem(b, min_comps);
+    const auto fits = [&] { return csmc::batch_smem_bytes(b->n_jobs, g.stride, b->threads) <= b->max_smem; };
+    b->threads = b->block;
+    if (g.least <= b->max_smem) {
+        while (b->threads > 32 && !fits()) b->threads = b->threads % 64 ? 32 : b->threads / 2;
+        if (!fits()) {
+            b->threads = b->block;
+            min_comps = 0;
+            g = GroupSmem{};
+        }
+    }
     for (int j = 0; j < b->n_jobs; ++j) {
         const csmc_net_header &h = b->nets[j]->h;
-        const bool g = min_comps > 0 && h.n_comps >= min_comps && h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS;
-        b->group[j] = g;
-        if (g) {
+        const bool warp = min_comps > 0 && h.n_comps >= min_comps && h.n_comps <= CSMC_BATCH_GROUP_MAX_COMPS;
+        b->group[j] = warp;
+        if (warp) {
             ++b->n_group;
-            gmax_c = std::max(gmax_c, h.n_comps);
-            gmax_vp = std::max(gmax_vp, h.n_vars + h.n_rate_prog);
         } else {
             b->max_v = std::max(b->max_v, h.n_vars);
             b->max_p = std::max(b->max_p, h.n_rate_prog);
             b->max_c = std::max(b->max_c, h.n_comps);
         }
     }
-    b->group_k = gmax_c == 0 ? 0 : gmax_c <= 128 ? 4 : gmax_c <= 256 ? 8 : 16;
-    b->group_stride = b->n_group ? csmc::group_state_stride(gmax_vp, 0, 32, b->group_k) : 0;
+    b->group_k = g.k;
+    b->group_stride = g.stride;
     std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) {
         if (b->group[x] != b->group[y]) return b->group[x] > b->group[y];
         return b->cost[x] > b->cost[y];
@@ -217,15 +260,15 @@ int upload_table(csmc_batch *b, const std::vector<uint64_t> &runs, uint64_t step
     return CSMC_OK;
 }
 
-size_t launch_smem(const csmc_batch *b, int block) {
-    return csmc::batch_smem_bytes(b->n_jobs, b->n_group ? b->group_stride : 0u, block);
+size_t launch_smem(const csmc_batch *b) {
+    return csmc::batch_smem_bytes(b->n_jobs, b->n_group ? b->group_stride : 0u, b->threads);
 }
 
 // Grid and state slabs for the current geometry.
 int configure(csmc_batch *b) {
     int ctas = 0, sms = 0;
-    const size_t smem = launch_smem(b, b->block);
-    int rc = csmc::batch_max_active_ctas(b->verify, b->n_group ? b->group_k : 0, b->block, smem, &ctas);
+    const size_t smem = launch_smem(b);
+    int rc = csmc::batch_max_active_ctas(b->verify, b->n_group ? b->group_k : 0, b->threads, smem, &ctas);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "occupancy query");
     if (ctas < 1) return fail(CSMC_ERR_LIMIT, "batch kernel cannot be resident");
     if (b->ctas_per_sm > 0) ctas = std::min(ctas, b->ctas_per_sm);
@@ -233,11 +276,11 @@ int configure(csmc_batch *b) {
     uint64_t grid = static_cast<uint64_t>(sms) * ctas;
     uint64_t thread_runs = 0, group_runs = 0;
     part_totals(b, b->n_runs, &thread_runs, &group_runs);
-    const uint64_t warps = b->block / 32;
-    const uint64_t needed = (thread_runs + b->block - 1) / b->block + (group_runs + warps - 1) / warps;
+    const uint64_t warps = b->threads / 32;
+    const uint64_t needed = (thread_runs + b->threads - 1) / b->threads + (group_runs + warps - 1) / warps;
     grid = std::max<uint64_t>(1, std::min(grid, needed));
     const size_t per = b->n_group == b->n_jobs ? 0 : csmc::batch_state_bytes_per_thread(b->max_c, b->max_v, b->max_p);
-    b->state_stride = static_cast<uint32_t>((per * b->block + 15) & ~static_cast<size_t>(15));
+    b->state_stride = static_cast<uint32_t>((per * b->threads + 15) & ~static_cast<size_t>(15));
     const size_t need = std::max<size_t>(16, grid * static_cast<size_t>(b->state_stride));
     if (need > b->state_bytes) {
         cudaFree(b->d_state);
@@ -272,7 +315,7 @@ int launch_impl(csmc_batch *b, cudaStream_t st, const std::vector<uint64_t> &run
     p.group_queue = b->n_group ? b->d_counters + 1 : nullptr;
     p.group_stride = b->group_stride;
     p.group_k = static_cast<uint32_t>(b->group_k);
-    int rc = csmc::batch_launch(b->verify, p, b->grid, b->block, st);
+    int rc = csmc::batch_launch(b->verify, p, b->grid, b->threads, st);
     if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "batch kernel launch");
     reduce_jobs<<<dim3(csmc::kReduceBlocks, b->n_jobs), 256, 0, st>>>(b->d_jobs, b->d_partials);
     CK(cudaGetLastError(), "reduce launch");
@@ -307,7 +350,7 @@ void fill_results(const csmc_batch *b, const std::vector<uint64_t> &runs, float 
         r.kernel_ms = ms;
         r.lanes_per_run = b->group[j] ? 32 : 1;
         r.comps_per_lane = b->group[j] ? b->group_k : static_cast<int32_t>(b->nets[j]->h.n_comps);
-        r.runs_per_cta = b->group[j] ? b->block / 32 : b->block;
+        r.runs_per_cta = b->group[j] ? b->threads / 32 : b->threads;
         r.family = 2;
     }
 }
@@ -350,6 +393,9 @@ int csmc_batch_create(csmc_net *const *nets, const csmc_query *qs, const uint64_
         return fail(CSMC_ERR_LIMIT, "a batch holds 1 to " + std::to_string(CSMC_BATCH_MAX_JOBS) + " jobs");
     auto b = std::make_unique<csmc_batch>();
     CK(cudaGetDevice(&b->device), "cudaGetDevice");
+    int max_smem = 0;
+    CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device), "cudaDeviceGetAttribute");
+    b->max_smem = static_cast<size_t>(max_smem);
     b->n_jobs = n_jobs;
     b->verify = verify != 0;
     uint64_t fs_words = 0;
@@ -413,7 +459,11 @@ int csmc_batch_set_plan(csmc_batch *b, int32_t threads_per_cta, int32_t ctas_per
     CK(cudaSetDevice(b->device), "cudaSetDevice");
     b->block = threads_per_cta;
     b->ctas_per_sm = ctas_per_sm;
-    return configure(b);
+    const std::vector<char> before = b->group;
+    assign_modes(b);  // (which networks fit one warp per run depends on the CTA)
+    int rc = configure(b);
+    if (rc) return rc;
+    return b->group == before ? CSMC_OK : upload_table(b, b->n_runs);
 }
 
 int csmc_batch_plan(const csmc_batch *b, int32_t *threads_per_cta, int32_t *ctas_per_sm) {
@@ -556,10 +606,11 @@ int csmc_batch_autotune(csmc_batch *b, double probe_fraction, int32_t *threads_p
     float best_ms = -1.0f;
     for (int block : {64, 128}) {
         int maxc = 0;
-        rc = csmc::batch_max_active_ctas(b->verify, b->n_group ? b->group_k : 0, block, launch_smem(b, block), &maxc);
+        b->block = block;
+        assign_modes(b);
+        rc = csmc::batch_max_active_ctas(b->verify, b->n_group ? b->group_k : 0, b->threads, launch_smem(b), &maxc);
         if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "occupancy query");
         for (int c = maxc; c >= 1 && c >= maxc - 3; --c) {
-            b->block = block;
             b->ctas_per_sm = c;
             rc = configure(b);
             if (rc) return rc;

@@ -220,8 +220,11 @@ int csmc_batch_plan(const csmc_batch *b, int32_t *threads_per_cta, int32_t *ctas
  * run queue.  0: every job runs one thread per run.  Default 128; until the
  * threshold is set (here or by csmc_batch_autotune), smaller networks run one
  * warp per run too where the batch is estimated to end earlier so (reported
- * per job in csmc_result.lanes_per_run).  The per-run results do not depend
- * on it.  csmc_batch_group_comps reports the threshold and how many jobs it
+ * per job in csmc_result.lanes_per_run).  Where the runs' state does not fit
+ * in shared memory, CTAs take fewer threads (csmc_result.runs_per_cta) or
+ * every job runs one thread per run; CSMC_ERR_* only where the variables and
+ * slot masks of the plan's CTA alone do not fit.  The per-run results do not
+ * depend on it.  csmc_batch_group_comps reports the threshold and how many jobs it
  * selects. */
 int csmc_batch_set_group_comps(csmc_batch *b, int32_t min_comps);
 int csmc_batch_group_comps(const csmc_batch *b, int32_t *min_comps, int32_t *group_jobs);

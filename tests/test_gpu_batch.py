@@ -220,3 +220,44 @@ def test_batch_rejects_bad_jobs():
             api.Batch([(net, bad, 1, 10)])
     finally:
         net.close()
+
+
+def _many_variables(w, n):
+    """The workload's network with n more shared variables, used by nobody."""
+    w.xml = w.xml.replace("int id = 0;", "int id = 0;\n" + "\n".join(f"int u{i} = {i % 9};" for i in range(n)), 1)
+    return w
+
+
+@pytest.mark.parametrize("procs,variables,plan,lanes,per_cta", [
+    # the estimate's one warp per run, and where four warps' variables do not fit one thread per run
+    (8, 1000, None, 32, 4),
+    (8, 15_000, None, 1, 128),
+    # the default threshold: four warps' variables and slot masks fit, with their delay records or without
+    (130, 13_000, None, 32, 4),
+    (130, 13_868, None, 32, 2),
+    # a threshold of the caller's, CTAs of one warp whose records do not fit
+    (100, 57_000, (32, 64), 32, 1),
+    (100, 57_600, (32, 64), 1, 32),
+])
+def test_batches_near_the_shared_memory_limit_are_accepted(procs, variables, plan, lanes, per_cta):
+    import oracle
+    w = _many_variables(netgen.mutex(procs, horizon=3), variables)
+    blob = _blob(w)
+    net, small = api.Network(blob), api.Network(_blob(netgen.mutex(5, horizon=3)))
+    q = api.variable_query(w.var_id, 3, threshold=1, is_max=True, max_steps=300)
+    _, want, _ = oracle.run(blob, q, 3, 40, threads=0, digests=True, final_state=True)
+    batch = api.Batch([(net, q, 3, 40), (small, q, 4, 40)], verify=True)
+    try:
+        if plan:
+            batch.set_plan(plan[0], 0)
+            batch.set_group_comps(plan[1])
+        res = batch.run()
+        out = batch.outputs(0)
+    finally:
+        batch.close()
+        net.close()
+        small.close()
+    assert (res[0].lanes_per_run, res[0].runs_per_cta) == (lanes, per_cta)
+    for key in ("steps", "flags", "digests"):
+        assert np.array_equal(out[key], want[key]), key
+    assert np.array_equal(np.asarray(out["final_state"]).ravel(), np.asarray(want["final_state"]).ravel())
