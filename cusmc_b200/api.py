@@ -137,8 +137,9 @@ class Network:
         check(lib().csmc_set_plan(self._h, family, lanes_per_run, comps_per_lane, threads_per_cta))
 
     def autotune(self, query: Query, seed: int, probe_runs: int) -> Result:
-        """Times every feasible launch plan on runs 0..probe_runs-1 and keeps
-        the fastest (csmc_autotune); returns the winning probe's result."""
+        """Times the default launch plan and every feasible fixed one on runs
+        0..probe_runs-1 and keeps the fastest (csmc_autotune); returns the
+        winning probe's result."""
         r = Result()
         check(lib().csmc_autotune(self._h, ctypes.byref(query), seed & (2**64 - 1), probe_runs, ctypes.byref(r)))
         return r

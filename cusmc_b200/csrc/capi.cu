@@ -690,6 +690,7 @@ int csmc_net_upload(const void *blob, size_t bytes, csmc_net **out) {
     if (!ok) ok = configure_plan(n.get(), pl, 1, 1, static_cast<int>(h->n_comps), 128, why);
     if (!ok) ok = configure_plan(n.get(), pl, 2, 1, static_cast<int>(h->n_comps), 128, why);
     if (!ok) return fail(CSMC_ERR_LIMIT, "no launch plan for this network: " + why);
+    n->own_plan = pl;
     CK(cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, n->device), "cudaDeviceGetAttribute");
     find_shapes(n.get());
     if ((pl.family == 1 && !pl.state_in_global) || pl.family == 4) {

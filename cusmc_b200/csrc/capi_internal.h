@@ -41,6 +41,7 @@ struct csmc_net {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     csmc_launch_plan plan;     // the plan set by csmc_set_plan, else the default of launches that fill the GPU
     bool plan_forced = false;  // csmc_set_plan: every launch uses `plan`
+    csmc_launch_plan own_plan;  // the default `plan` had before csmc_set_plan
     csmc_group_shape shapes[6];  // lane-group shapes for launches that do not fill the GPU one thread per run
     int n_shapes = 0;
     int sms = 0;               // SMs of the device

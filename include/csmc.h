@@ -185,11 +185,13 @@ int csmc_set_plan(csmc_net *net, int32_t family, int32_t lanes_per_run, int32_t 
 
 /* Autotuner for one network (no counterpart in the reference, which has one
  * fixed launch shape: one CTA per run, one thread per component).  Times
- * csmc_run on runs 0 .. probe_runs-1 for every feasible plan — one thread
- * per run at 64 and 128 threads per CTA, lane groups at 128 and 256 threads
- * per CTA, and the global-memory plan at 64 and 128 — keeps the fastest on
- * the handle and reports it in best (family, lanes_per_run, comps_per_lane,
- * runs_per_cta, kernel_ms of its probe). */
+ * csmc_run on runs 0 .. probe_runs-1 with the default plan (chosen by the
+ * number of runs) and with every feasible fixed plan of these: one thread per
+ * run at 64 and 128 threads per CTA, lane groups at 128 and 256 threads per
+ * CTA, and the global-memory plan at 64 and 128.  Where a fixed plan is the
+ * fastest by more than 3 % it is kept on the handle for every launch, else the
+ * default stays.  The fastest is reported in best (family, lanes_per_run,
+ * comps_per_lane, runs_per_cta, kernel_ms of its probe). */
 int csmc_autotune(csmc_net *net, const csmc_query *q, uint64_t seed, uint64_t probe_runs, csmc_result *best);
 
 /* ---- Batches: many (network, query) jobs in one persistent launch --------
