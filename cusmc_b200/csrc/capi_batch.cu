@@ -360,9 +360,14 @@ void fill_results(const csmc_batch *b, const std::vector<uint64_t> &runs, float 
 // Probes cap every run at kProbeSteps race steps, so that a probe costs a
 // bounded amount of work even when single runs of a job take seconds.
 constexpr uint64_t kProbeSteps = 2000;
+// The autotuner's last comparison takes probes of at least this long, or all
+// runs of the batch, and at most this cap.
+constexpr float kConfirmMs = 100.0f;
+constexpr uint64_t kMaxProbeSteps = 10000000;
 
-int probe(csmc_batch *b, const std::vector<uint64_t> &runs, float *ms, std::vector<uint64_t> *steps_out) {
-    int rc = upload_table(b, runs, kProbeSteps);
+int probe(csmc_batch *b, const std::vector<uint64_t> &runs, float *ms, std::vector<uint64_t> *steps_out,
+          uint64_t step_cap = kProbeSteps) {
+    int rc = upload_table(b, runs, step_cap);
     if (rc) return rc;
     cudaStream_t st = nullptr;
     CK(cudaEventRecord(b->ev0, st), "cudaEventRecord");
@@ -585,70 +590,127 @@ int csmc_batch_autotune(csmc_batch *b, double probe_fraction, int32_t *threads_p
     if (!(probe_fraction > 0.0 && probe_fraction <= 1.0)) return fail(CSMC_ERR_ARG, "probe fraction must be in (0, 1]");
     CK(cudaSetDevice(b->device), "cudaSetDevice");
     std::vector<uint64_t> runs(b->n_jobs);
-    for (int j = 0; j < b->n_jobs; ++j)
-        runs[j] = b->n_runs[j] ? std::max<uint64_t>(1, static_cast<uint64_t>(b->n_runs[j] * probe_fraction)) : 0;
-    const int save_block = b->block, save_ctas = b->ctas_per_sm;
-    b->group_auto = false;  // the probes choose the threshold
-    assign_modes(b);
-    int rc = configure(b);
-    if (rc) return rc;
+    const auto scale_runs = [&](double f) {
+        for (int j = 0; j < b->n_jobs; ++j)
+            runs[j] = b->n_runs[j] ? std::max<uint64_t>(1, static_cast<uint64_t>(b->n_runs[j] * f)) : 0;
+    };
+    scale_runs(probe_fraction);
+    // a geometry and an assignment of the jobs to the two modes
+    struct Tuned {
+        int block, ctas;
+        uint32_t min_comps;
+        bool automatic;
+    };
+    int rc = CSMC_OK;
+    const auto set = [&](const Tuned &t) {
+        b->block = t.block;
+        b->ctas_per_sm = t.ctas;
+        b->group_min_comps = t.min_comps;
+        b->group_auto = t.automatic;
+        assign_modes(b);
+        return configure(b);
+    };
+    const auto max_ctas = [&](int *ctas) {
+        return csmc::batch_max_active_ctas(b->verify, b->n_group ? b->group_k : 0, b->threads, launch_smem(b), ctas);
+    };
+    float ms = 0.0f;
+    const Tuned start{b->block, b->ctas_per_sm, b->group_min_comps, b->group_auto};
     // 1. measure the cost per run of every job at the current geometry
     std::vector<uint64_t> steps;
-    float ms = 0.0f;
     rc = probe(b, runs, &ms, &steps);
     if (rc) return rc;
+    const std::vector<double> cost = b->cost;
+    std::vector<double> measured = cost;
     for (int j = 0; j < b->n_jobs; ++j)  // measured cost per run where no probe run was capped
         if (runs[j] && steps[j])
-            b->cost[j] = static_cast<double>(steps[j]) / runs[j] * std::max<uint32_t>(1, b->nets[j]->h.n_comps);
-    assign_modes(b);
+            measured[j] = static_cast<double>(steps[j]) / runs[j] * std::max<uint32_t>(1, b->nets[j]->h.n_comps);
+    b->cost = measured;
     // 2. geometry: threads per CTA x CTAs per SM
-    int best_block = save_block, best_ctas = save_ctas;
+    Tuned best = start;
     float best_ms = -1.0f;
     for (int block : {64, 128}) {
+        Tuned t = start;
+        t.block = block;
+        t.ctas = 0;
+        rc = set(t);
+        if (rc) return rc;
         int maxc = 0;
-        b->block = block;
-        assign_modes(b);
-        rc = csmc::batch_max_active_ctas(b->verify, b->n_group ? b->group_k : 0, b->threads, launch_smem(b), &maxc);
+        rc = max_ctas(&maxc);
         if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "occupancy query");
         for (int c = maxc; c >= 1 && c >= maxc - 3; --c) {
-            b->ctas_per_sm = c;
-            rc = configure(b);
-            if (rc) return rc;
-            rc = probe(b, runs, &ms, nullptr);
+            t.ctas = c;
+            rc = set(t);
+            if (!rc) rc = probe(b, runs, &ms, nullptr);
             if (rc) return rc;
             if (best_ms < 0.0f || ms < best_ms) {
                 best_ms = ms;
-                best_block = block;
-                best_ctas = c;
+                best = t;
             }
         }
     }
-    b->block = best_block;
-    b->ctas_per_sm = best_ctas;
-    // 3. which networks run one warp per run, at that geometry
-    const uint32_t save_min = b->group_min_comps;
-    uint32_t best_min = save_min;
-    for (uint32_t m : {0u, 64u, 128u, 256u}) {
-        if (m == save_min) continue;
-        b->group_min_comps = m;
-        assign_modes(b);
-        rc = configure(b);
-        if (rc) return rc;
-        rc = probe(b, runs, &ms, nullptr);
+    // 3. which networks run one warp per run, at that geometry (thresholds
+    // that set_group_comps would take)
+    rc = set(best);
+    if (rc) return rc;
+    std::vector<Tuned> modes;
+    for (uint32_t m : {0u, 64u, 128u, 256u})
+        if ((start.automatic || m != start.min_comps) && group_smem(b, m).least <= b->max_smem)
+            modes.push_back({best.block, best.ctas, m, false});
+    if (!start.automatic) modes.push_back({best.block, best.ctas, kDefaultGroupMinComps, true});
+    for (const Tuned &t : modes) {
+        rc = set(t);
+        if (!rc) rc = probe(b, runs, &ms, nullptr);
         if (rc) return rc;
         if (ms < best_ms) {
             best_ms = ms;
-            best_min = m;
+            best = t;
         }
     }
-    b->group_min_comps = best_min;
-    assign_modes(b);
-    rc = configure(b);
+    // 4. against what the batch had, and that with the measured costs, in turn,
+    // on a probe that fills the GPU as the batch does (a short one prefers few
+    // CTAs per SM: 16 random networks of 1000 runs, 38 ms untuned, 91 ms with
+    // the one per SM that a probe of 20 runs each picked) and ends as many of
+    // its runs: first the cap grows, then the number of runs
+    const auto use = [&](int i) {
+        b->cost = i == 0 ? cost : measured;
+        return set(i == 2 ? best : start);
+    };
+    uint64_t cap = kProbeSteps;
+    rc = use(0);
+    for (double f = probe_fraction; !rc;) {
+        rc = probe(b, runs, &ms, &steps, cap);
+        if (rc || ms >= kConfirmMs) break;
+        bool capped = false;
+        for (int j = 0; j < b->n_jobs; ++j) capped = capped || (runs[j] && !steps[j]);
+        if (capped && cap < kMaxProbeSteps) {
+            cap *= 4;
+        } else if (f < 1.0) {
+            f = std::min(1.0, 4.0 * f);
+            scale_runs(f);
+        } else {
+            break;
+        }
+    }
     if (rc) return rc;
+    float of[3] = {-1.0f, -1.0f, -1.0f};
+    for (int i = 0; i < 9; ++i) {
+        rc = use(i % 3);
+        if (!rc) rc = probe(b, runs, &ms, nullptr, cap);
+        if (rc) return rc;
+        if (of[i % 3] < 0.0f || ms < of[i % 3]) of[i % 3] = ms;
+    }
+    // (a choice is kept where it is faster by more than probes of one geometry differ)
+    const int kept = of[2] < 0.97f * std::min(of[0], of[1]) ? 2 : of[1] < 0.97f * of[0] ? 1 : 0;
+    rc = use(kept);
+    if (rc) return rc;
+    if (b->ctas_per_sm == 0) {  // (as many as fit: reported as their number)
+        rc = max_ctas(&b->ctas_per_sm);
+        if (rc) return cuda_fail(static_cast<cudaError_t>(rc), "occupancy query");
+    }
     rc = upload_table(b, b->n_runs);
     if (rc) return rc;
-    if (threads_per_cta) *threads_per_cta = best_block;
-    if (ctas_per_sm) *ctas_per_sm = best_ctas;
+    if (threads_per_cta) *threads_per_cta = b->block;
+    if (ctas_per_sm) *ctas_per_sm = b->ctas_per_sm;
     return CSMC_OK;
 }
 

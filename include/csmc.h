@@ -258,11 +258,12 @@ int csmc_batch_outputs_host(const csmc_batch *b, int32_t job, uint8_t *flags, do
 
 /* Autotuner for the batch: runs a probe batch (each job's runs scaled by
  * probe_fraction, at least one run, every run capped at 2000 race steps) at
- * each candidate geometry (64 and 128 threads per CTA, every CTAs-per-SM
- * count that fits), keeps the fastest, then at that geometry tries the
- * warp-per-run thresholds 0, 64, 128 and 256 components
- * (csmc_batch_set_group_comps) and keeps the fastest; it orders the jobs of
- * each run space by measured cost per run (where no probe run reached the
+ * each candidate geometry (64 and 128 threads per CTA, the largest
+ * CTAs-per-SM counts that fit), then at the fastest tries the warp-per-run
+ * thresholds 0, 64, 128 and 256 components (csmc_batch_set_group_comps), and
+ * keeps the fastest where it is more than 3 % faster than the batch as it was
+ * (its geometry and its choice by estimate, or the caller's) on a probe of
+ * 100 ms or all runs; it orders the jobs of each run space by measured cost per run (where no probe run reached the
  * cap), most expensive first, so that the cheapest runs fill the end of the
  * batch. */
 int csmc_batch_autotune(csmc_batch *b, double probe_fraction, int32_t *threads_per_cta, int32_t *ctas_per_sm);

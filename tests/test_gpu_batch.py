@@ -261,3 +261,24 @@ def test_batches_near_the_shared_memory_limit_are_accepted(procs, variables, pla
     for key in ("steps", "flags", "digests"):
         assert np.array_equal(out[key], want[key]), key
     assert np.array_equal(np.asarray(out["final_state"]).ravel(), np.asarray(want["final_state"]).ravel())
+
+
+def test_autotuner_keeps_an_assignment_that_is_the_fastest():
+    """16 random networks, 1000 runs each: the estimate's assignment ends in
+    38 ms, the thresholds the autotuner tries at best in 46."""
+    jobs = []
+    for i, w in enumerate(netgen.batch_networks(16, base_seed=1000)):
+        q = api.variable_query(w.var_id, 50, threshold=w.threshold, is_max=True, max_steps=1_000_000)
+        jobs.append((api.Network(_blob(w)), q, 1 + i, 1000))
+    batch = api.Batch(jobs)
+    try:
+        before = batch.run()
+        batch.autotune(0.02)
+        after = batch.run()
+    finally:
+        batch.close()
+        for j in jobs:
+            j[0].close()
+    assert [r.lanes_per_run for r in after] == [r.lanes_per_run for r in before]
+    assert {r.lanes_per_run for r in before if r.comps_per_lane < 128} == {1, 32}
+    assert [(r.hits, r.steps, r.sum) for r in after] == [(r.hits, r.steps, r.sum) for r in before]
