@@ -133,7 +133,8 @@ class Network:
                  threads_per_cta: int = 128) -> None:
         """Selects the kernel family and launch shape (0: lane groups, 1: one
         thread per run, 2: one thread per run with the network in global
-        memory)."""
+        memory, 4: class-coded).  At the limit of shared memory another shape
+        may run; a launch's result reports it."""
         check(lib().csmc_set_plan(self._h, family, lanes_per_run, comps_per_lane, threads_per_cta))
 
     def autotune(self, query: Query, seed: int, probe_runs: int) -> Result:

@@ -178,8 +178,13 @@ int csmc_plan(const csmc_net *net, int32_t *lanes_per_run, int32_t *comps_per_la
  * class-coded locations (networks with race classes, at most 256 components
  * and 32 locations per automaton; their default for large launches).  For
  * families 1, 2 and 4 lanes and comps_per_lane are ignored.  threads_per_cta:
- * CTA size (lane groups take a smaller one where shared memory asks for it).
- * Every family gives the same per-run results. */
+ * CTA size.  At the limit of shared memory a plan is taken, not refused, in
+ * another shape: lane groups take a smaller CTA where their delay records do
+ * not fit beside the variables and slot masks, and family 1 where one warp's do
+ * not; family 4 with fewer than 128 threads becomes family 1 where the keys of
+ * 128 threads do not fit.  csmc_plan and csmc_result (family, lanes_per_run,
+ * runs_per_cta) report what runs.  Every family gives the same per-run
+ * results. */
 int csmc_set_plan(csmc_net *net, int32_t family, int32_t lanes_per_run, int32_t comps_per_lane,
                   int32_t threads_per_cta);
 

@@ -113,3 +113,28 @@ def test_networks_beyond_shared_memory_run_a_warp_per_run():
             assert np.array_equal(got["values"].view(np.uint64), want["values"].view(np.uint64))
     finally:
         net.close()
+
+
+@pytest.mark.parametrize("workload,first,variables,plan,family", [
+    # class-coded CTAs of 32 threads: the keys of 128 fit, or only those of 32
+    (lambda: netgen.epidemic(n_agents=40, horizon=20, r_threshold=10), "int S = 39;", 1500, (4, 1, 1, 32), 4),
+    (lambda: netgen.epidemic(n_agents=40, horizon=20, r_threshold=10), "int S = 39;", 1600, (4, 1, 1, 32), 1),
+    # one warp per run: its records fit, or only its variables and slot masks
+    (lambda: netgen.mutex(300, horizon=3), "int id = 0;", 10_000, (0, 32, 16, 32), 0),
+    (lambda: netgen.mutex(300, horizon=3), "int id = 0;", 11_016, (0, 32, 16, 32), 1),
+])
+def test_plans_at_the_shared_memory_limit_report_what_runs(workload, first, variables, plan, family):
+    w = workload()
+    w.xml = w.xml.replace(first, first + "\n" + "\n".join(f"int u{i} = {i % 9};" for i in range(variables)), 1)
+    blob = _blob(w)
+    q = api.variable_query(w.var_id, w.horizon, threshold=w.threshold, is_max=True, max_steps=300)
+    _, want, _ = oracle.run(blob, q, 13, 40, threads=0, digests=True, final_state=True)
+    net = api.Network(blob)
+    try:
+        net.set_plan(*plan)
+        r, got = net.run_verify(q, 13, 40)
+        assert r.family == family and r.lanes_per_run == net.plan()[0]
+    finally:
+        net.close()
+    for key in ("steps", "flags", "digests", "final_state"):
+        assert np.array_equal(got[key], want[key]), key
