@@ -35,6 +35,8 @@ NUM_EXP2_F32 = 6
 NUM_GELU_F32 = 7
 NUM_GELU_GRAD_F32 = 8
 NUM_PHILOX_STEP = 9
+NUM_RCP_F32 = 10
+NUM_TIME_ADD = 11
 
 
 class Query(ctypes.Structure):

@@ -1,7 +1,7 @@
 // csmc_numeric_eval: the numeric primitives whose exact bits define a run —
 // Philox4x32-10, the exponential delay and its float log2, the double
-// log2/exp2/pow of the expression language, and the proposal network's
-// exp2 and GELU — evaluated by the device code the kernels inline, over
+// log2/exp2/pow of the expression language, the clocks' addition, and the
+// proposal network's exp2, GELU and the sigmoid's reciprocal — evaluated by the device code the kernels inline, over
 // device arrays.  A host compares these bits with its own evaluation of the
 // same definitions (the CPU oracle compiles the same headers) and with
 // independent references (published Philox known-answer vectors, libm).
@@ -73,6 +73,13 @@ __global__ void numeric_eval_kernel(int32_t fn, const void *a, const void *b, ui
         case CSMC_NUM_GELU_GRAD_F32:
             static_cast<float *>(out)[i] = csmc::gelu_grad_f(static_cast<const float *>(a)[i]);
             break;
+        case CSMC_NUM_RCP_F32:
+            static_cast<float *>(out)[i] = csmc::rcp_from_one(static_cast<const float *>(a)[i]);
+            break;
+        case CSMC_NUM_TIME_ADD:
+            static_cast<float *>(out)[i] =
+                csmc::time_add(static_cast<const float *>(a)[i], static_cast<const float *>(b)[i]);
+            break;
         default:
             break;
         }
@@ -82,11 +89,12 @@ __global__ void numeric_eval_kernel(int32_t fn, const void *a, const void *b, ui
 }  // namespace
 
 extern "C" int csmc_numeric_eval(int32_t fn, const void *a, const void *b, uint64_t n, void *out, void *stream) {
-    if (fn < CSMC_NUM_PHILOX || fn > CSMC_NUM_PHILOX_STEP) {
+    if (fn < CSMC_NUM_PHILOX || fn > CSMC_NUM_TIME_ADD) {
         csmc::set_last_error("unknown numeric function " + std::to_string(fn));
         return CSMC_ERR_ARG;
     }
-    const bool two = fn == CSMC_NUM_PHILOX || fn == CSMC_NUM_PHILOX_STEP || fn == CSMC_NUM_EXP_DELAY || fn == CSMC_NUM_POW_F64;
+    const bool two = fn == CSMC_NUM_PHILOX || fn == CSMC_NUM_PHILOX_STEP || fn == CSMC_NUM_EXP_DELAY || fn == CSMC_NUM_POW_F64 ||
+                     fn == CSMC_NUM_TIME_ADD;
     if (n && (!a || !out || (two && !b))) {
         csmc::set_last_error("null argument");
         return CSMC_ERR_ARG;

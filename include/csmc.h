@@ -469,7 +469,10 @@ int csmc_smc_is(const char *model_path, int seed, int sims, const csmc_query *q,
  *   CSMC_NUM_GELU_GRAD_F32 a: f32[n] -> f32 GELU'
  *   CSMC_NUM_PHILOX_STEP   as CSMC_NUM_PHILOX, through the per-step
  *                          factorisation the simulation kernels use
- *                          (counter = step, component group, run low, run high) */
+ *                          (counter = step, component group, run low, run high)
+ *   CSMC_NUM_RCP_F32       a: f32[n] in [1, 2^126] -> f32 1/a (the sigmoid's)
+ *   CSMC_NUM_TIME_ADD      a, b: f32[n] -> f32 a + b (clocks and time: the
+ *                          double sum rounded to float) */
 #define CSMC_NUM_PHILOX 0
 #define CSMC_NUM_EXP_DELAY 1
 #define CSMC_NUM_LOG2_F32 2
@@ -480,6 +483,8 @@ int csmc_smc_is(const char *model_path, int seed, int sims, const csmc_query *q,
 #define CSMC_NUM_GELU_F32 7
 #define CSMC_NUM_GELU_GRAD_F32 8
 #define CSMC_NUM_PHILOX_STEP 9
+#define CSMC_NUM_RCP_F32 10
+#define CSMC_NUM_TIME_ADD 11
 int csmc_numeric_eval(int32_t fn, const void *a, const void *b, uint64_t n, void *out, void *stream);
 
 /* Measures the shared-memory bandwidth of the current device (no

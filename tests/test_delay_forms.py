@@ -7,7 +7,11 @@ the bits of the definitions they replace.
 * GELU: its sigmoid's reciprocal is an approximation and a Newton step; a
   grid of 2^24 floats over the exponents where the sigmoid is neither 0 nor
   1, and the clamped ends, are compared with the host's form (none).
-* time_add: one float addition instead of a double sum rounded to float.
+* The reciprocal itself: every float of [1, 2^126] against the double
+  quotient rounded to float (none; 53 bits rounded to 24 is the quotient
+  rounded once).
+* time_add: one float addition instead of a double sum rounded to float, in
+  numpy and in the device's form.
 """
 import numpy as np
 import pytest
@@ -65,3 +69,37 @@ def test_float_sum_equals_the_double_sum_rounded_to_float():
         once = a + b
         twice = (a.astype(np.float64) + b.astype(np.float64)).astype(np.float32)
     assert np.array_equal(once.view(np.uint32), twice.view(np.uint32))
+
+
+@pytest.mark.gpu
+def test_reciprocal_of_every_float_from_one_to_2_126_equals_the_quotient():
+    import torch
+    from cusmc_b200 import _native
+    from cusmc_b200._native import check, lib
+    mantissas = torch.arange(1 << 23, dtype=torch.int32, device="cuda")
+    got = torch.empty(1 << 23, dtype=torch.float32, device="cuda")
+    for e in range(127):  # (at the last exponent 2^126 alone)
+        x = (mantissas if e < 126 else torch.zeros_like(mantissas)).add((e + 127) << 23).view(torch.float32)
+        check(lib().csmc_numeric_eval(_native.NUM_RCP_F32, x.data_ptr(), None, x.numel(), got.data_ptr(), None))
+        want = (1.0 / x.double()).float()
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32)), e
+
+
+@pytest.mark.gpu
+def test_device_time_add_equals_the_double_sum_rounded_to_float():
+    import torch
+    from cusmc_b200 import _native
+    from cusmc_b200._native import check, lib
+    rng = np.random.default_rng(6)
+    n = 4_000_000
+    a = rng.integers(0, 2**32, n, dtype=np.uint64).astype(np.uint32).view(np.float32)
+    m = (1.0 + rng.integers(0, 2**23, n) * 2.0 ** -23) * rng.choice([-1.0, 1.0], n)
+    with np.errstate(all="ignore"):
+        b = np.where(np.isfinite(a), np.ldexp(m, np.frexp(a)[1] + rng.integers(-60, 61, n)), 1.0).astype(np.float32)
+        ok = np.isfinite(a) & np.isfinite(b)
+        a, b = a[ok], b[ok]
+        want = (a.astype(np.float64) + b.astype(np.float64)).astype(np.float32)
+    ad, bd = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    got = torch.empty(a.size, dtype=torch.float32, device="cuda")
+    check(lib().csmc_numeric_eval(_native.NUM_TIME_ADD, ad.data_ptr(), bd.data_ptr(), a.size, got.data_ptr(), None))
+    assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
