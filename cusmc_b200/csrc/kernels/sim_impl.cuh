@@ -251,7 +251,7 @@ struct GroupRun {
         const uint32_t C = n.n_comps;
         const int sender = s->sc.sender;
         uint32_t *const rmv = reinterpret_cast<uint32_t *>(rec);  // the records are written again below
-        const uint32_t kn = n_k(C), kmax = !kStrided ? B * NB : 4u * (((C + 3u) >> 2) + G - 1u) / G;
+        const uint32_t kn = n_k(C), kmax = !kStrided ? B * NB : 4u * ((((C + 3u) >> 2) + G - 1u) / G);
         // the masks overwrite the records: one lane's mask lies in another
         // lane's record, which that lane may have written at the end of the
         // step before

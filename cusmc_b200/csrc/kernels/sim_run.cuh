@@ -375,7 +375,7 @@ static __device__ __forceinline__ void run_step(const Net &n, uint32_t C, uint32
     // ---- delays and the race
     unsigned long long best;
     float bestd;
-        const auto draws = keys.at(step, run);
+    const auto draws = keys.at(step, run);
     if (CLASSES) {
         if (!race_classes(n, C, bits, rv, draws, best, bestd))
             race_exact(n, C, bits, rv, draws, best, bestd);
