@@ -114,15 +114,16 @@ bool plan_is_coded(const csmc_net *n, uint64_t n_runs, Launch &L) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device) != cudaSuccess)
         return false;
     // a small launch is bound by its single runs' steps, which one warp per
-    // run takes faster.  One thread per run / one warp per run, epidemics
-    // under a trained proposal: 99 agents 10,000 runs 35 / 21 ms, 19,000 runs
-    // 36 / 38; 49 agents 14,000 runs 18.3 / 17.1, 19,000 runs 18.6 / 22.9; 23
-    // agents 10,000 runs 7.3 / 6.3, 14,000 runs 7.6 / 8.5: from 100 runs per SM
-    // where every location is in a tilt group.  A multiple of four components
-    // keeps 48, the crossing before the one-warp kernel kept its sums (it was
-    // 60.8 ms at 1e4 runs of 100 agents): which kernel runs there is reported
-    // to the caller.  With the descriptor path, from 128 (1e4 runs: 134k runs/s
-    // against 165k; 2e4 runs: 242k against 179k)
+    // run takes faster.  One thread per run / one warp per run, ms, epidemics to
+    // time 75 under a proposal at 8,104, 14,000 and 20,000 runs: 99 agents 32 /
+    // 16, 32 / 26, 32 / 36; 48 agents 15.1 / 9.7, 15.1 / 15.2, 16.2 / 21.4; 20
+    // agents 7.9 / 5.3, 7.9 / 8.6, 8.2 / 12.0: from 100 runs per SM where every
+    // location is in a tilt group.  Networks of a multiple of four components
+    // would cross there too (100 agents 32 / 16 and 32 / 26): they keep the 48
+    // that csmc.h has promised them since the crossing lay there, and callers
+    // that want the other kernel set it (csmc_is_set_kernel).  With the
+    // descriptor path, from 128 (1e4 runs: 134k runs/s against 165k; 2e4 runs:
+    // 242k against 179k)
     const uint64_t per_sm = !n->is_all_grouped ? 128 : h.n_comps % 4 ? 100 : 48;
     const uint64_t min_runs = per_sm * static_cast<uint64_t>(sms);
     if (n->is_kernel == 0 && n_runs < min_runs) return false;

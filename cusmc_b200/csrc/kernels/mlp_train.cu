@@ -70,7 +70,7 @@ constexpr uint32_t kTh = kB2 + 64 * 64 * 2;     // theta partials [group][row] (
 constexpr uint32_t kMisc = kTh + kGroups * 128 * 4;  // mbarrier, tmem address, biases, reductions
 constexpr uint32_t kMiscBytes = 4096;
 constexpr uint32_t kRedStride = 17;             // per-warp output-layer sums: 16 columns, db3
-constexpr uint32_t kSmemBytes = 160 * 1024;     // >= the operands' extent under either stride reading
+constexpr uint32_t kSmemBytes = 160 * 1024;     // the carve-up takes 102 KB; more than half an SM's: one CTA per SM
 static_assert(kMisc + kMiscBytes <= kSmemBytes, "shared-memory carve-up");
 static_assert(1536 + 16 * kRedStride * 4 <= kMiscBytes, "reduction slots");
 
